@@ -33,10 +33,31 @@ struct Grid {
   }
 };
 
-// Interior box of one multigrid level.
+// Division of n < 2^31 by a fixed d in one wide multiplication and a shift
+// (m = floor(2^(31+s) / d) + 1 with 2^(s-1) < d <= 2^s: the quotient of
+// Granlund and Montgomery, PLDI 1994); a hardware-less 32-bit division is
+// some twenty instructions.
+struct FastDiv {
+  uint32_t m = 0;
+  int s = 0;
+  void set(int d) {
+    s = 0;
+    while ((1ll << s) < d) s++;
+    m = (uint32_t)((1ull << (31 + s)) / (uint32_t)d + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (uint32_t)(((uint64_t)n * m) >> (31 + s)); }
+};
+
+// Interior box of one multigrid level (set_size fills the divisors too).
 struct Box {
   int nx, ny, nz;
   int px, py, pz;
+  FastDiv dx, dy;
+  void set_size(int x, int y, int z) {
+    nx = x; ny = y; nz = z;
+    dx.set(x);
+    dy.set(y);
+  }
   __host__ __device__ size_t n() const { return (size_t)nx * ny * nz; }
   __host__ __device__ size_t at(int i, int j, int k) const {
     return ((size_t)k * ny + j) * nx + i;
@@ -44,10 +65,10 @@ struct Box {
 };
 
 // (i, j, k) of box-layout cell c, in 32-bit arithmetic (a box holds fewer
-// than 2^32 cells; 64-bit integer division costs a software routine).
+// than 2^28 cells).
 __device__ __forceinline__ void box_ijk(const Box &b, size_t c, int &i, int &j, int &k) {
   const uint32_t u = (uint32_t)c, nx = (uint32_t)b.nx, ny = (uint32_t)b.ny;
-  const uint32_t row = u / nx, kk = row / ny;
+  const uint32_t row = b.dx.div(u), kk = b.dy.div(row);
   i = (int)(u - row * nx);
   j = (int)(row - kk * ny);
   k = (int)kk;

@@ -21,6 +21,15 @@ struct MetricPtrs {
   double *gface;
 };
 
+// The factors of Projection's correction, v dt st / coeff, and which of them
+// differ from 1 (ops bits 0..2), decided on the host: a comparison per face
+// would go to the FP64 pipe.  Bit 3: coeff lies in 2^-100..2^100, so the
+// division may go through rcoeff = RN(1 / coeff).
+struct ProjScale {
+  double dt, st, coeff, rcoeff;
+  int ops;
+};
+
 // setup.cu (compiled without FMA contraction)
 __global__ void k_metrics_cell(Grid g, const double *coor, MetricPtrs m);
 __global__ void k_face_coef(Grid g, MetricPtrs m, double *gface);
@@ -75,13 +84,18 @@ __global__ void k_box_to_da_phi(Grid g, Box b, const double *nvert, const double
                                 const double *shift);
 __global__ void k_da_to_box(Grid g, Box b, const double *da, double *x);
 __global__ void k_box_to_da(Grid g, Box b, const double *x, double *da);
-__global__ void k_update_pressure(Grid g, const double *nvert, const double *phi, double *p);
-__global__ void k_periodic_copy2(Grid g, double *p, double *phi);
-__global__ void k_projection(Grid g, Box b, const double *nvert, const double *phi, const double *pc, double dt,
-                             double st, double coeff, double *ucont, MetricPtrs m, LevelSet ls);
+__global__ void k_near_body(Grid g, Box b, const double *nvert, uint8_t *near);
+__global__ void k_near_body_rows(Grid g, Box b, const double *nvert, uint8_t *near, const int *rows, const int *nrows);
+__global__ void k_update_pressure(Grid g, const double *nvert, const uint8_t *near, const double *phi, double *p,
+                                  double *phi_out);
+__global__ void k_periodic_copy2(Grid g, double *p, double *phi, double *phi2);
+__global__ void k_projection(Grid g, Box b, const double *nvert, const uint8_t *near, const double *phi,
+                             const double *pc, ProjScale ps, double *ucont, MetricPtrs m);
+__global__ void k_projection_ls(Grid g, Box b, const double *nvert, const uint8_t *near, const double *phi,
+                                const double *pc, ProjScale ps, double *ucont, MetricPtrs m, LevelSet ls);
 __global__ void k_periodic_faces(Grid g, double *ucont);
-__global__ void k_divergence(Grid g, Box b, const double *nvert, const double *ucont, const double *aj,
-                             double *partial);
+__global__ void k_divergence(Grid g, Box b, const double *nvert, const uint8_t *near, const double *ucont,
+                             const double *aj, double *partial);
 __global__ void k_reduce_max(const double *partial, int nb, double *out);
 __global__ void k_coarse_nodes(Grid gf, Grid gc, int cx, int cy, int cz, const double *cf, double *cc);
 __global__ void k_nvert_restrict(Grid gh, Grid gc, int cx, int cy, int cz, const double *nh, double *nc);

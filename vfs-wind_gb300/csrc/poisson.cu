@@ -452,6 +452,7 @@ struct vfs_poisson {
   double *A0 = nullptr, *scale = nullptr, *pc = nullptr, *aj_box = nullptr;
   float *scale32 = nullptr;  // the row scale in FP32 (the FP32 V-cycle's right-hand side)
   uint8_t *rowtype0 = nullptr, *fluid = nullptr;
+  uint8_t *near = nullptr;  // cells with a non-zero nvert within one point (k_near_body)
   int *gid_box = nullptr, *gid_da = nullptr, *blk = nullptr, *total = nullptr;
   int ndof = 0;
   double *b = nullptr, *x = nullptr, *r = nullptr;
@@ -646,6 +647,11 @@ int sync(vfs_poisson *h) {
 dim3 da_grid(const Grid &g, int bx = 128) { return dim3((g.mx + bx - 1) / bx, g.my, g.mz); }
 dim3 box_grid(const Box &b, int bx = 128) { return dim3((b.nx + bx - 1) / bx, b.ny, b.nz); }
 unsigned lin_grid(size_t n, int bx = 256) { return (unsigned)((n + bx - 1) / bx); }
+// grid of the passes over the periodic ghost layers (shell_point); 0: no periodic axis
+unsigned shell_grid(const Grid &g) {
+  return lin_grid(2 * ((g.px ? (size_t)g.my * g.mz : 0) + (g.py ? (size_t)g.mx * g.mz : 0) +
+                       (g.pz ? (size_t)g.mx * g.my : 0)));
+}
 // grid of the guess's reduction kernels: 128 columns x kGuessRows j-rows
 dim3 guess_grid(const Box &b) { return dim3((b.nx + 127) / 128, (b.ny + kGuessRows - 1) / kGuessRows, b.nz); }
 
@@ -1077,9 +1083,7 @@ int build_hierarchy(vfs_poisson *h, int coarsest_max) {
     f.cx = c[0]; f.cy = c[1]; f.cz = c[2];
     Level q;
     q.b = f.b;
-    q.b.nx = c[0] ? f.b.nx / 2 : f.b.nx;
-    q.b.ny = c[1] ? f.b.ny / 2 : f.b.ny;
-    q.b.nz = c[2] ? f.b.nz / 2 : f.b.nz;
+    q.b.set_size(c[0] ? f.b.nx / 2 : f.b.nx, c[1] ? f.b.ny / 2 : f.b.ny, c[2] ? f.b.nz / 2 : f.b.nz);
     q.g = f.g;
     q.g.mx = q.b.nx + 2; q.g.my = q.b.ny + 2; q.g.mz = q.b.nz + 2;
     TRY(dalloc(h, &q.coor, q.g.n() * 3));
@@ -2096,7 +2100,8 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
   vfs_poisson *h = new vfs_poisson();
   h->desc = *gd;
   h->g = Grid{gd->mx, gd->my, gd->mz, px, py, pz};
-  h->box = Box{nx, ny, nz, px, py, pz};
+  h->box.px = px; h->box.py = py; h->box.pz = pz;
+  h->box.set_size(nx, ny, nz);
   cudaGetDevice(&h->device);
   auto bail = [&](int rc) { vfs_poisson_destroy(h); return rc; };
   // a blocking stream: work the caller queued on the legacy default stream
@@ -2130,7 +2135,8 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
       (rc = alloc_metrics(h, h->g, h->met)) || (rc = dalloc(h, &h->A0, n * NSLOT)) ||
       (rc = dalloc(h, &h->scale, n)) || (rc = dalloc(h, &h->scale32, n)) || (rc = dalloc(h, &h->pc, 12 * n)) ||
       (rc = dalloc(h, &h->aj_box, n)) ||
-      (rc = dalloc(h, &h->rowtype0, n)) || (rc = dalloc(h, &h->fluid, n)) || (rc = dalloc(h, &h->gid_box, n)) ||
+      (rc = dalloc(h, &h->rowtype0, n)) || (rc = dalloc(h, &h->fluid, n)) ||
+      (rc = dalloc(h, &h->near, n)) || (rc = dalloc(h, &h->gid_box, n)) ||
       (rc = dalloc(h, &h->gid_da, N)) || (rc = dalloc(h, &h->b, n)) || (rc = dalloc(h, &h->x, n)) ||
       (rc = dalloc(h, &h->r, n)) || (rc = dalloc(h, &h->red, 512)) || (rc = dalloc(h, &h->total, 1)))
     return bail(rc);
@@ -2242,6 +2248,9 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
     fls.rho = h->ls_rho; fls.level = h->ls_level; fls.on = 1;
     fls.bc3 = h->ls_bc3; fls.bc4 = h->ls_bc4; fls.bc5 = h->ls_bc5;
   }
+  if (!incremental)
+    LAUNCH(h, k_near_body, dim3((h->box.nx + 125) / 126, h->box.ny, h->box.nz), 128, h->g, h->box,
+           (const double *)h->nvert, h->near);
   if (incremental) {
     LAUNCH(h, k_mask_changed, kRedBlocks, 256, N, (const double *)h->nvert, (const double *)h->nvert_prev, h->chg_a);
     LAUNCH(h, k_dilate_axis, da_grid(h->g), 128, h->g, 0, 2, (const uint8_t *)h->chg_a, h->chg_b);
@@ -2252,6 +2261,8 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
     LAUNCH(h, k_list_rows, kRedBlocks, 256, h->g, h->box, (const uint8_t *)h->chg_b, h->rows, h->nrows, h->colflag);
     LAUNCH(h, k_assemble_fine_rows, kRedBlocks, 256, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
            h->L[0].A64, h->L[0].rowtype, fls, (const int *)h->rows, (const int *)h->nrows);
+    LAUNCH(h, k_near_body_rows, kRedBlocks, 256, h->g, h->box, (const double *)h->nvert, h->near,
+           (const int *)h->rows, (const int *)h->nrows);
     h->inc_rows = true;
   } else if (refills) {  // both fine operators from one evaluation of each row
     LAUNCH(h, k_assemble_fine, box_grid(h->box), 128, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
@@ -3051,12 +3062,18 @@ int vfs_poisson_update_pressure(vfs_poisson *h, double *p, double *phi) {
   if (!h || !p) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before update_pressure");
   const size_t N = h->g.n();
-  TRY(upload(h, h->p_da, p, N));
-  if (phi) TRY(upload(h, h->phi_da, phi, N));
-  LAUNCH(h, k_update_pressure, da_grid(h->g), 128, h->g, h->nvert, h->phi_da, h->p_da);
-  LAUNCH(h, k_periodic_copy2, da_grid(h->g), 128, h->g, h->p_da, h->phi_da);
-  TRY(download(h, p, h->p_da, N));
-  if (phi) TRY(download(h, phi, h->phi_da, N));
+  // device arrays are updated where they lie; the handle's phi (which
+  // Projection reads) receives its copy in the same pass
+  const bool pdev = is_device_ptr(p), fdev = phi && is_device_ptr(phi);
+  double *pd = pdev ? p : h->p_da;
+  if (!pdev) TRY(upload(h, pd, p, N));
+  if (phi && !fdev) TRY(upload(h, h->phi_da, phi, N));
+  LAUNCH(h, k_update_pressure, lin_grid(N), 256, h->g, h->nvert, h->near, fdev ? phi : h->phi_da, pd,
+         fdev ? h->phi_da : nullptr);
+  if (const unsigned nb = shell_grid(h->g))
+    LAUNCH(h, k_periodic_copy2, nb, 256, h->g, pd, h->phi_da, fdev ? phi : nullptr);
+  if (!pdev) TRY(download(h, p, pd, N));
+  if (phi && !fdev) TRY(download(h, phi, h->phi_da, N));
   return sync(h);
 }
 
@@ -3064,17 +3081,25 @@ int vfs_poisson_projection(vfs_poisson *h, double *ucont, double dt, double st, 
   if (!h || !ucont) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before projection");
   if (!(coeff != 0.)) return fail(VFS_EINVAL, "coeff must be non-zero");
-  const size_t N = h->g.n();
-  TRY(upload(h, h->ucont, ucont, 3 * N));
-  LevelSet pls;
+  const size_t N = h->g.n(), n = h->box.n();
+  const bool dev = is_device_ptr(ucont);
+  double *u = dev ? ucont : h->ucont;
+  if (!dev) TRY(upload(h, u, ucont, 3 * N));
+  ProjScale ps;
+  ps.dt = dt; ps.st = st; ps.coeff = coeff;
+  ps.rcoeff = 1.0 / coeff;
+  const double ac = std::fabs(coeff);
+  ps.ops = (dt != 1.0 ? 1 : 0) | (st != 1.0 ? 2 : 0) | (coeff != 1.0 ? 4 : 0) | (ac > 0x1p-100 && ac < 0x1p100 ? 8 : 0);
   if (h->ls_on) {
+    LevelSet pls;
     pls.rho = h->ls_rho; pls.level = h->ls_level; pls.on = 1;
     pls.bc3 = h->ls_bc3; pls.bc4 = h->ls_bc4; pls.bc5 = h->ls_bc5;
+    LAUNCH(h, k_projection_ls, lin_grid(n), 256, h->g, h->box, h->nvert, h->near, h->phi_da, h->pc, ps, u, h->met, pls);
+  } else {
+    LAUNCH(h, k_projection, lin_grid(n), 256, h->g, h->box, h->nvert, h->near, h->phi_da, h->pc, ps, u, h->met);
   }
-  LAUNCH(h, k_projection, box_grid(h->box), 128, h->g, h->box, h->nvert, h->phi_da, h->pc, dt, st, coeff, h->ucont,
-         h->met, pls);
-  LAUNCH(h, k_periodic_faces, da_grid(h->g), 128, h->g, h->ucont);
-  TRY(download(h, ucont, h->ucont, 3 * N));
+  if (const unsigned nb = shell_grid(h->g)) LAUNCH(h, k_periodic_faces, nb, 256, h->g, u);
+  if (!dev) TRY(download(h, ucont, u, 3 * N));
   return sync(h);
 }
 
@@ -3082,12 +3107,9 @@ int vfs_poisson_divergence(vfs_poisson *h, const double *ucont, double *maxdiv) 
   if (!h || !ucont || !maxdiv) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before divergence");
   const size_t N = h->g.n();
-  const double *u = ucont;
-  if (!is_device_ptr(ucont)) {
-    TRY(upload(h, h->stage, ucont, 3 * N));
-    u = h->stage;
-  }
-  LAUNCH(h, k_divergence, kRedBlocks, 256, h->g, h->box, h->nvert, u, h->met.aj, h->partial);
+  const double *u = nullptr;
+  TRY(device_view(h, ucont, h->stage, 3 * N, &u));
+  LAUNCH(h, k_divergence, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, u, h->met.aj, h->partial);
   LAUNCH(h, k_reduce_max, 1, 1024, h->partial, kRedBlocks, h->red);
   CUDA_TRY(cudaMemcpyAsync(h->hbuf, h->red, 8, cudaMemcpyDeviceToHost, h->stream));
   TRY(sync(h));
