@@ -50,9 +50,11 @@ struct FastDiv {
 
 // Interior box of one multigrid level (set_size fills the divisors too).
 struct Box {
-  int nx, ny, nz;
-  int px, py, pz;
+  int nx = 0, ny = 0, nz = 0;
+  int px = 0, py = 0, pz = 0;
   FastDiv dx, dy;
+  Box() = default;
+  Box(int x, int y, int z, int perx, int pery, int perz) : px(perx), py(pery), pz(perz) { set_size(x, y, z); }
   void set_size(int x, int y, int z) {
     nx = x; ny = y; nz = z;
     dx.set(x);

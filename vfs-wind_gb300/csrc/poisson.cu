@@ -2100,8 +2100,7 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
   vfs_poisson *h = new vfs_poisson();
   h->desc = *gd;
   h->g = Grid{gd->mx, gd->my, gd->mz, px, py, pz};
-  h->box.px = px; h->box.py = py; h->box.pz = pz;
-  h->box.set_size(nx, ny, nz);
+  h->box = Box{nx, ny, nz, px, py, pz};
   cudaGetDevice(&h->device);
   auto bail = [&](int rc) { vfs_poisson_destroy(h); return rc; };
   // a blocking stream: work the caller queued on the legacy default stream
