@@ -69,3 +69,43 @@ def test_pressure_projection_divergence(cuda_lib, dims, periodic, kind):
             assert s.divergence(u) == O.divergence(d, case.nvert, u_o, met["aj"])
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("kind", ["none", "plain", "odd"])
+@pytest.mark.parametrize("dims,periodic", BOXES, ids=["x".join(map(str, b[0])) for b in BOXES])
+def test_volume_flux_and_rhs(cuda_lib, dims, periodic, kind):
+    """The sums are reduced in another order than the oracle's: corrected
+    fluxes and right-hand side to 1e-12 of the largest value, flux and area
+    to 1e-10 (the tolerances of the other VolumeFlux and right-hand-side
+    tests)."""
+    import torch
+    import vfs_poisson as V
+    case, rng = build(dims, periodic, kind, seed=5)
+    d = O.dims_of(case)
+    met = O.form_metrics(d, case.coor)
+    lhs = O.poisson_lhs(d, case.nvert, met)
+    u0 = case.ucont.copy()
+    u0[rng.random(u0.shape) < 0.2] *= 1e-9  # faces VolumeFlux zeroes
+    s = V.PoissonSolver(*case.dims, periodic=periodic)
+    try:
+        s.set_grid(case.coor)
+        s.set_nvert(case.nvert)
+
+        def close(u, f, a, u_o, f_o, a_o):
+            assert np.abs(u.cpu().numpy() - u_o).max() <= 1e-12
+            assert abs(a - a_o) <= 1e-10 * max(abs(a_o), 1e-300)
+            assert abs(f - f_o) <= 1e-10 * max(np.abs(u0).sum(), 1.0)
+        for flg in range(4):
+            u = torch.from_numpy(u0.copy()).cuda()
+            f, a = s.volume_flux(u, flg=flg, flux_intp_sum=0.01)
+            close(u, f, a, *O.volume_flux(d, case.nvert, met, u0, flg=flg, flux_intp_sum=0.01))
+        for immersed in (0, 2, 3, 4):
+            u = torch.from_numpy(u0.copy()).cuda()
+            f, a = s.volume_flux0(u, immersed)
+            close(u, f, a, *O.volume_flux0(d, case.nvert, met, u0, immersed))
+        b_o = O.to_da(d, lhs["gid"], O.rhs(d, case.nvert, lhs["gid"], case.ucont, met["aj"], 0.5, 1.0, 1.5))
+        for u in (case.ucont, torch.from_numpy(case.ucont).cuda()):
+            s.rhs(u, 0.5, 1.0, 1.5)
+            assert np.abs(s.rhs_array() - b_o).max() <= 1e-12 * np.abs(b_o).max()
+    finally:
+        s.close()

@@ -13,10 +13,34 @@
 
 namespace vfs {
 
+// Division of n < 2^31 by a fixed d in one wide multiplication and a shift
+// (m = floor(2^(31+s) / d) + 1 with 2^(s-1) < d <= 2^s: the quotient of
+// Granlund and Montgomery, PLDI 1994); a hardware-less 32-bit division is
+// some twenty instructions.
+struct FastDiv {
+  uint32_t m = 0;
+  int s = 0;
+  void set(int d) {
+    s = 0;
+    while ((1ll << s) < d) s++;
+    m = (uint32_t)((1ull << (31 + s)) / (uint32_t)d + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (uint32_t)(((uint64_t)n * m) >> (31 + s)); }
+};
+
 // DA-layout grid with merged periodic flags (i_periodic || ii_periodic, ...).
+// (set_size fills the divisors too).
 struct Grid {
-  int mx, my, mz;
-  int px, py, pz;
+  int mx = 0, my = 0, mz = 0;
+  int px = 0, py = 0, pz = 0;
+  FastDiv dx, dy;
+  Grid() = default;
+  Grid(int x, int y, int z, int perx, int pery, int perz) : px(perx), py(pery), pz(perz) { set_size(x, y, z); }
+  void set_size(int x, int y, int z) {
+    mx = x; my = y; mz = z;
+    dx.set(x);
+    dy.set(y);
+  }
   __host__ __device__ size_t n() const { return (size_t)mx * my * mz; }
   __host__ __device__ size_t at(int i, int j, int k) const {
     return ((size_t)k * my + j) * mx + i;
@@ -31,21 +55,6 @@ struct Grid {
     if (pz) { if (k == 0) { c = mz - 2; fk = 1; } else if (k == mz - 1) { c = 1; fk = 1; } }
     return fi | fj | fk;
   }
-};
-
-// Division of n < 2^31 by a fixed d in one wide multiplication and a shift
-// (m = floor(2^(31+s) / d) + 1 with 2^(s-1) < d <= 2^s: the quotient of
-// Granlund and Montgomery, PLDI 1994); a hardware-less 32-bit division is
-// some twenty instructions.
-struct FastDiv {
-  uint32_t m = 0;
-  int s = 0;
-  void set(int d) {
-    s = 0;
-    while ((1ll << s) < d) s++;
-    m = (uint32_t)((1ull << (31 + s)) / (uint32_t)d + 1);
-  }
-  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (uint32_t)(((uint64_t)n * m) >> (31 + s)); }
 };
 
 // Interior box of one multigrid level (set_size fills the divisors too).
@@ -73,6 +82,15 @@ __device__ __forceinline__ void box_ijk(const Box &b, size_t c, int &i, int &j, 
   const uint32_t row = b.dx.div(u), kk = b.dy.div(row);
   i = (int)(u - row * nx);
   j = (int)(row - kk * ny);
+  k = (int)kk;
+}
+
+// (i, j, k) of DA point t (fewer than 2^28 points).
+__device__ __forceinline__ void da_ijk(const Grid &g, size_t t, int &i, int &j, int &k) {
+  const uint32_t u = (uint32_t)t;
+  const uint32_t row = g.dx.div(u), kk = g.dy.div(row);
+  i = (int)(u - row * (uint32_t)g.mx);
+  j = (int)(row - kk * (uint32_t)g.my);
   k = (int)kk;
 }
 

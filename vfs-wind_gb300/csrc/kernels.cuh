@@ -44,11 +44,15 @@ __global__ void k_rhs2(Grid g, Box b, const double *nvert, const uint8_t *rowtyp
                        const double *aj, double dt, double st, double coeff, int poisson, double *rhs, double *partial);
 __global__ void k_rhs2_shift(Grid g, Box b, const double *nvert, const double *aj, const double *sums, int poisson,
                              double *rhs);
-__global__ void k_vflux_sum(Grid g, const double *nvert, MetricPtrs m, double *ucont, int flg, int pass,
-                            double *partial);
-__global__ void k_vflux_apply(Grid g, const double *nvert, MetricPtrs m, double *ucont, int flg, double corr);
-__global__ void k_vflux0_sum(Grid g, const double *nvert, MetricPtrs m, double *ucont, double *partial);
-__global__ void k_vflux0_apply(Grid g, const double *nvert, MetricPtrs m, double *ucont, double corr, int zero);
+__global__ void k_vflux_sum(Grid g, Box b, const double *nvert, const uint8_t *near, MetricPtrs m, double *ucont,
+                            int flg, double *partial);
+__global__ void k_vflux_corr(const double *partial, int nb, int flg, double flux_intp_sum, double *corr);
+__global__ void k_vflux_apply(Grid g, Box b, const double *nvert, const uint8_t *near, MetricPtrs m, double *ucont,
+                              int flg, const double *corr, double *partial);
+__global__ void k_vflux0_sum(Grid g, Box b, const double *nvert, const uint8_t *near, MetricPtrs m, double *ucont,
+                             double *partial);
+__global__ void k_vflux0_apply(Grid g, Box b, const double *nvert, const uint8_t *near, MetricPtrs m, double *ucont,
+                               const double *corr, int zero, double *partial);
 __global__ void k_periodic_cmpnts(Grid g, const double *src, double *dst);
 __global__ void k_contra2cart(Grid g, const double *nvert, MetricPtrs m, const double *lu, double *ucat);
 __global__ void k_zero_solid(Grid g, const double *nvert, double *ucat);
@@ -65,23 +69,23 @@ __global__ void k_mask_changed(size_t N, const double *a, const double *b, uint8
 __global__ void k_dilate_axis(Grid g, int axis, int R, const uint8_t *src, uint8_t *dst);
 __global__ void k_list_rows(Grid g, Box b, const uint8_t *flag, int *rows, int *nrows, uint8_t *colflag);
 __global__ void k_projection_coef(Grid g, Box b, MetricPtrs m, double *pc);
-__global__ void k_level_masks(Grid g, Box b, const double *nvert, uint8_t *blank, double *w64, float *w32,
-                              double *aj_box, const double *aj_da);
-__global__ void k_rhs(Grid g, Box b, const double *nvert, const double *ucont, const double *aj, double dt,
-                      double st, double coeff, double *rhs, double *partial);
+__global__ void k_level_masks(Grid g, Box b, const double *nvert, uint8_t *blank, double *w64, float *w32);
+__global__ void k_rhs(Grid g, Box b, const uint8_t *fluid, const double *ucont, double dt, double st, double coeff,
+                      double *rhs, double *partial);
 __global__ void k_reduce_rows(const double *partial, int nb, int nrow, double *out);
-__global__ void k_rhs_nullspace(Grid g, Box b, const double *nvert, const double *aj, const double *sums,
-                                double *rhs);
+__global__ void k_rhs_nullspace(Box b, const uint8_t *fluid, const double *aj_box, const double *sum,
+                                const double *fsum, double *rhs);
 __global__ void k_fully_blocked(Grid g, const double *nvert, int *ksk, int *unblocked);
 __global__ void k_nullspace_sums(Grid g, const double *nvert, const int *ksk, int multi, const double *x,
                                  double *partial);
 __global__ void k_nullspace_apply(Grid g, const double *nvert, const int *ksk, int multi, double shift0,
                                   double shift1, double *x);
-__global__ void k_mean_partial(Box b, const uint8_t *fluid, const double *x, double *partial);
-__global__ void k_fluid_mask(Grid g, Box b, const double *nvert, uint8_t *fluid);
-__global__ void k_mean_shift(double *sums);
-__global__ void k_box_to_da_phi(Grid g, Box b, const double *nvert, const double *x, double *phi,
-                                const double *shift);
+__global__ void k_mean_partial(size_t n, const uint8_t *fluid, const double *x, double *partial);
+__global__ void k_fluid_mask(Grid g, Box b, const double *nvert, const double *aj, uint8_t *fluid, double *aj_box,
+                             double *partial);
+__global__ void k_mean_shift(const double *partial, int nb, const double *fsum, double *shift);
+__global__ void k_box_to_da_phi(Grid g, Box b, const uint8_t *rowtype, const uint8_t *fluid, const double *x,
+                                double *phi, const double *shift);
 __global__ void k_da_to_box(Grid g, Box b, const double *da, double *x);
 __global__ void k_box_to_da(Grid g, Box b, const double *x, double *da);
 __global__ void k_near_body(Grid g, Box b, const double *nvert, uint8_t *near);

@@ -461,6 +461,7 @@ struct vfs_poisson {
   std::vector<double *> V, Z;
   double **dV = nullptr, **dZ = nullptr;
   // dsv[2q] = ||V_q||^2 and dsv[2q+1] = 1 / ||V_q||; dsv32[q] the latter in FP32
+  double *fsum = nullptr;  // over the fluid cells of the mask: sum of aj, count
   double *partial = nullptr, *red = nullptr, *coef = nullptr, *dsv = nullptr;
   float *dsv32 = nullptr;
   size_t partial_len = 0;
@@ -959,8 +960,7 @@ int build_level_operator(vfs_poisson *h, Level &l, bool assembled = false) {
            (const int *)h->rows, (const int *)h->nrows);
   else if (!assembled)
     LAUNCH(h, k_assemble, box_grid(l.b), 128, l.g, l.b, l.nvert, l.met, 1, 0, 1, l.A64, l.rowtype, level_set(h, l));
-  LAUNCH(h, k_level_masks, lin_grid(n), 256, l.g, l.b, l.nvert, l.blank, l.w64, l.w32, (double *)nullptr,
-         (const double *)nullptr);
+  LAUNCH(h, k_level_masks, lin_grid(n), 256, l.g, l.b, l.nvert, l.blank, l.w64, l.w32);
   // a level of an incremental refill: only the listed rows' copies and the
   // j-columns that hold one are formed again
   const uint8_t *cols = h->inc_rows ? h->colflag : nullptr;
@@ -1085,7 +1085,7 @@ int build_hierarchy(vfs_poisson *h, int coarsest_max) {
     q.b = f.b;
     q.b.set_size(c[0] ? f.b.nx / 2 : f.b.nx, c[1] ? f.b.ny / 2 : f.b.ny, c[2] ? f.b.nz / 2 : f.b.nz);
     q.g = f.g;
-    q.g.mx = q.b.nx + 2; q.g.my = q.b.ny + 2; q.g.mz = q.b.nz + 2;
+    q.g.set_size(q.b.nx + 2, q.b.ny + 2, q.b.nz + 2);
     TRY(dalloc(h, &q.coor, q.g.n() * 3));
     TRY(dalloc(h, &q.nvert, q.g.n()));
     double *tmp;
@@ -2135,7 +2135,7 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
       (rc = dalloc(h, &h->scale, n)) || (rc = dalloc(h, &h->scale32, n)) || (rc = dalloc(h, &h->pc, 12 * n)) ||
       (rc = dalloc(h, &h->aj_box, n)) ||
       (rc = dalloc(h, &h->rowtype0, n)) || (rc = dalloc(h, &h->fluid, n)) ||
-      (rc = dalloc(h, &h->near, n)) || (rc = dalloc(h, &h->gid_box, n)) ||
+      (rc = dalloc(h, &h->near, n)) || (rc = dalloc(h, &h->fsum, 2)) || (rc = dalloc(h, &h->gid_box, n)) ||
       (rc = dalloc(h, &h->gid_da, N)) || (rc = dalloc(h, &h->b, n)) || (rc = dalloc(h, &h->x, n)) ||
       (rc = dalloc(h, &h->r, n)) || (rc = dalloc(h, &h->red, 512)) || (rc = dalloc(h, &h->total, 1)))
     return bail(rc);
@@ -2240,7 +2240,10 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
   LAUNCH(h, k_scan_blocks, 1, 1024, h->blk, nblk, h->total);
   LAUNCH(h, k_number_dofs, nblk, 1024, h->g, h->box, h->nvert, h->blk, h->gid_box);
   LAUNCH(h, k_gid_da, da_grid(h->g), 128, h->g, h->box, h->gid_box, h->gid_da);
-  LAUNCH(h, k_fluid_mask, lin_grid(n), 256, h->g, h->box, h->nvert, h->fluid);
+  // the fluid mask, aj at the box cells and the mask's sums (aj and count
+  // over the fluid), which every right-hand side and mean removal uses
+  LAUNCH(h, k_fluid_mask, kRedBlocks, 256, h->g, h->box, h->nvert, h->met.aj, h->fluid, h->aj_box, h->partial);
+  LAUNCH(h, k_reduce_rows, 2, 1024, h->partial, kRedBlocks, 2, h->fsum);
   // PoissonLHSNew: unscaled operator with the reference's insertion filter
   LevelSet fls;
   if (h->ls_on) {
@@ -2268,9 +2271,6 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
            h->L[0].A64, h->L[0].rowtype, fls);
   } else
     LAUNCH(h, k_assemble, box_grid(h->box), 128, h->g, h->box, h->nvert, h->met, 0, 1, 0, h->A0, h->rowtype0, fls);
-  // aj at the box cells for the row scale (each level forms its own masks)
-  LAUNCH(h, k_level_masks, lin_grid(n), 256, h->g, h->box, h->nvert, (uint8_t *)nullptr, (double *)nullptr,
-         (float *)nullptr, h->aj_box, (const double *)h->met.aj);
   LAUNCH(h, k_row_scale, lin_grid(n), 256, n, h->rowtype0, h->aj_box, h->scale);
   LAUNCH(h, k_cast_planes_f32, kRedBlocks, 256, h->scale, h->scale32, n);
   int tot = 0;
@@ -2298,14 +2298,14 @@ int vfs_poisson_rhs(vfs_poisson *h, const double *ucont, double dt, double st, d
   if (!h || !ucont) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before rhs");
   if (!(dt != 0.) || !(coeff != 0.)) return fail(VFS_EINVAL, "dt and coeff must be non-zero");
-  const size_t N = h->g.n();
-  TRY(upload(h, h->ucont, ucont, 3 * N));
-  LAUNCH(h, k_rhs, kRedBlocks, 256, h->g, h->box, h->nvert, h->ucont, h->met.aj, dt, st, coeff, h->b, h->partial);
+  const double *u = nullptr;
+  TRY(device_view(h, ucont, h->ucont, 3 * h->g.n(), &u));
+  LAUNCH(h, k_rhs, kRedBlocks, 256, h->g, h->box, h->fluid, u, dt, st, coeff, h->b, h->partial);
   // Remove_Nullspace_Scale, skipped for bctype[3] == -10 and for a level
   // set with the Dirichlet top bctype[5] == 4 (poisson_hypre.c:120, :375)
   if (h->desc.bctype3 != -10 && !(h->ls_on && h->ls_bc5 == 4)) {
-    LAUNCH(h, k_reduce_rows, 2, 1024, h->partial, kRedBlocks, 2, h->red);
-    LAUNCH(h, k_rhs_nullspace, kRedBlocks, 256, h->g, h->box, h->nvert, h->met.aj, h->red, h->b);
+    LAUNCH(h, k_reduce_rows, 1, 1024, h->partial, kRedBlocks, 1, h->red);
+    LAUNCH(h, k_rhs_nullspace, kRedBlocks, 256, h->box, h->fluid, h->aj_box, h->red, h->fsum, h->b);
   }
   TRY(sync(h));
   h->have_rhs = true;
@@ -2368,22 +2368,17 @@ int vfs_poisson_volume_flux(vfs_poisson *h, double *ucont, int flg, double flux_
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before volume_flux");
   if (flg < 0 || flg > 3) return fail(VFS_EINVAL, "flg must be 0..3");
   const size_t N = h->g.n();
-  TRY(upload(h, h->ucont, ucont, 3 * N));
-  double sums[3];
-  LAUNCH(h, k_vflux_sum, kRedBlocks, 256, h->g, h->nvert, h->met, h->ucont, flg, 0, h->partial);
-  TRY(reduce_read(h, kRedBlocks, 3, sums));
-  double corr = 0.;
-  if (sums[2] > 1.e-15) {
-    if (flg > 1) corr = (sums[0] + flux_intp_sum) / sums[1];
-    else if (flg) corr = (sums[0] + flux_intp_sum) / sums[2];
-    else corr = sums[0] / sums[2];
-  }
-  LAUNCH(h, k_vflux_apply, kRedBlocks, 256, h->g, h->nvert, h->met, h->ucont, flg, corr);
-  LAUNCH(h, k_vflux_sum, kRedBlocks, 256, h->g, h->nvert, h->met, h->ucont, flg, 2, h->partial);
-  TRY(reduce_read(h, kRedBlocks, 3, sums));
+  const bool dev = is_device_ptr(ucont);
+  double *u = dev ? ucont : h->ucont;
+  if (!dev) TRY(upload(h, u, ucont, 3 * N));
+  LAUNCH(h, k_vflux_sum, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, h->met, u, flg, h->partial);
+  LAUNCH(h, k_vflux_corr, 1, 1024, h->partial, kRedBlocks, flg, flux_intp_sum, h->red);
+  LAUNCH(h, k_vflux_apply, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, h->met, u, flg, h->red, h->partial);
+  double sums[2];
+  TRY(reduce_read(h, kRedBlocks, 2, sums));
   if (ibm_flux) *ibm_flux = sums[0];
-  if (ibm_area) *ibm_area = sums[2];
-  TRY(download(h, ucont, h->ucont, 3 * N));
+  if (ibm_area) *ibm_area = sums[1];
+  if (!dev) TRY(download(h, ucont, u, 3 * N));
   return sync(h);
 }
 
@@ -2392,20 +2387,20 @@ int vfs_poisson_volume_flux0(vfs_poisson *h, double *ucont, int immersed, double
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before volume_flux0");
   if (immersed == 1) return fail(VFS_EINVAL, "immersed 1 takes the other VolumeFlux (vfs_poisson_volume_flux)");
   const size_t N = h->g.n();
-  TRY(upload(h, h->ucont, ucont, 3 * N));
-  double sums[2];
-  LAUNCH(h, k_vflux0_sum, kRedBlocks, 256, h->g, h->nvert, h->met, h->ucont, h->partial);
-  TRY(reduce_read(h, kRedBlocks, 2, sums));
+  const bool dev = is_device_ptr(ucont);
+  double *u = dev ? ucont : h->ucont;
+  if (!dev) TRY(upload(h, u, ucont, 3 * N));
+  LAUNCH(h, k_vflux0_sum, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, h->met, u, h->partial);
   if (immersed != 2) {
-    const double corr = sums[1] > 1.e-15 ? sums[0] / sums[1] : 0.;
-    LAUNCH(h, k_vflux0_apply, kRedBlocks, 256, h->g, h->nvert, h->met, h->ucont, corr,
-           (immersed == 0 || immersed == 3) ? 1 : 0);
+    LAUNCH(h, k_vflux_corr, 1, 1024, h->partial, kRedBlocks, 4, 0., h->red);
+    LAUNCH(h, k_vflux0_apply, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, h->met, u, h->red,
+           (immersed == 0 || immersed == 3) ? 1 : 0, h->partial);
   }
-  LAUNCH(h, k_vflux0_sum, kRedBlocks, 256, h->g, h->nvert, h->met, h->ucont, h->partial);
+  double sums[2];
   TRY(reduce_read(h, kRedBlocks, 2, sums));
   if (flux) *flux = sums[0];
   if (area) *area = sums[1];
-  TRY(download(h, ucont, h->ucont, 3 * N));
+  if (!dev) TRY(download(h, ucont, u, 3 * N));
   return sync(h);
 }
 
@@ -2535,12 +2530,11 @@ int vfs_poisson_solve(vfs_poisson *h, double *phi, const vfs_solve_opts *opts, v
   // Remove_Nullspace of phi (:604-608), its shift applied by the DA output
   const bool shift = h->desc.bctype3 != -10 && !(h->ls_on && h->ls_bc5 == 4);
   if (shift) {
-    LAUNCH(h, k_mean_partial, kRedBlocks, 256, h->box, h->fluid, h->x, h->partial);
-    LAUNCH(h, k_reduce_rows, 2, 1024, h->partial, kRedBlocks, 2, h->red);
-    LAUNCH(h, k_mean_shift, 1, 32, h->red);
+    LAUNCH(h, k_mean_partial, kRedBlocks, 256, n, h->fluid, h->x, h->partial);
+    LAUNCH(h, k_mean_shift, 1, 1024, h->partial, kRedBlocks, h->fsum, h->red);
   }
-  LAUNCH(h, k_box_to_da_phi, da_grid(h->g), 128, h->g, h->box, h->nvert, h->x, h->phi_da,
-         shift ? (const double *)h->red + 2 : nullptr);
+  LAUNCH(h, k_box_to_da_phi, lin_grid(h->g.n()), 256, h->g, h->box, h->rowtype0, h->fluid, h->x, h->phi_da,
+         shift ? (const double *)h->red : nullptr);
   // phi to a host array on a side stream, while the solution enters the
   // history on the handle's stream (it reads x, b and the residual, not
   // phi); the handle's stream waits for the copy before the call returns
@@ -3171,7 +3165,7 @@ int vfs_poisson_get_metric(vfs_poisson *h, int which, double *out) {
 int vfs_poisson_get_rhs(vfs_poisson *h, double *b) {
   if (!h || !b) return fail(VFS_EINVAL, "null argument");
   if (!h->have_rhs) return fail(VFS_ESTATE, "rhs must come first");
-  LAUNCH(h, k_box_to_da, da_grid(h->g), 128, h->g, h->box, h->b, h->stage);
+  LAUNCH(h, k_box_to_da, lin_grid(h->g.n()), 256, h->g, h->box, h->b, h->stage);
   TRY(download(h, b, h->stage, h->g.n()));
   return sync(h);
 }
@@ -3184,7 +3178,7 @@ int vfs_poisson_apply(vfs_poisson *h, const double *x, double *y) {
   double *tmp = h->L[0].v64[3];
   LAUNCH(h, k_da_to_box, lin_grid(n), 256, h->g, h->box, h->stage, h->r);
   LAUNCH(h, k_apply64, box_grid(h->box), 128, h->box, h->A0, h->r, tmp);
-  LAUNCH(h, k_box_to_da, da_grid(h->g), 128, h->g, h->box, tmp, h->stage);
+  LAUNCH(h, k_box_to_da, lin_grid(h->g.n()), 256, h->g, h->box, tmp, h->stage);
   TRY(download(h, y, h->stage, h->g.n()));
   return sync(h);
 }
@@ -3218,7 +3212,7 @@ int vfs_poisson_mg_restrict(vfs_poisson *h, int fine, const double *xf, double *
   TRY(upload(h, h->stage, xf, l.g.n()));
   LAUNCH(h, k_da_to_box, lin_grid(l.b.n()), 256, l.g, l.b, h->stage, l.v64[2]);
   LAUNCH(h, k_restrict_f64, box_grid(q.b), 128, l.b, q.b, l.cx, l.cy, l.cz, l.v64[2], l.w64, q.blank, q.v64[1]);
-  LAUNCH(h, k_box_to_da, da_grid(q.g), 128, q.g, q.b, q.v64[1], h->stage);
+  LAUNCH(h, k_box_to_da, lin_grid(q.g.n()), 256, q.g, q.b, q.v64[1], h->stage);
   TRY(download(h, fc, h->stage, q.g.n()));
   return sync(h);
 }
@@ -3231,7 +3225,7 @@ int vfs_poisson_mg_interpolate(vfs_poisson *h, int fine, const double *xc, doubl
   LAUNCH(h, k_da_to_box, lin_grid(q.b.n()), 256, q.g, q.b, h->stage, q.v64[0]);
   LAUNCH(h, k_prolong_f64, box_grid(l.b), 128, l.b, q.b, l.cx, l.cy, l.cz, (const double *)q.v64[0], q.blank,
          l.blank, l.v64[2], 0);
-  LAUNCH(h, k_box_to_da, da_grid(l.g), 128, l.g, l.b, l.v64[2], h->stage);
+  LAUNCH(h, k_box_to_da, lin_grid(l.g.n()), 256, l.g, l.b, l.v64[2], h->stage);
   TRY(download(h, ff, h->stage, l.g.n()));
   return sync(h);
 }
@@ -3247,7 +3241,7 @@ int vfs_poisson_mg_vcycle(vfs_poisson *h, int precision, const double *r, double
   TRY(upload(h, h->stage, r, h->g.n()));
   LAUNCH(h, k_da_to_box, lin_grid(n), 256, h->g, h->box, h->stage, h->r);
   TRY(precondition(h, h->r, 1.0, nullptr, nullptr, h->r, o));
-  LAUNCH(h, k_box_to_da, da_grid(h->g), 128, h->g, h->box, h->r, h->stage);
+  LAUNCH(h, k_box_to_da, lin_grid(h->g.n()), 256, h->g, h->box, h->r, h->stage);
   TRY(download(h, z, h->stage, h->g.n()));
   return sync(h);
 }

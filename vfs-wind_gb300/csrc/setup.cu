@@ -638,57 +638,53 @@ __global__ void k_projection_coef(Grid g, Box b, MetricPtrs m, double *pc) {
 // Box-layout masks of a level: row-active flag from the assembly, blanking
 // (nvert > 0.1) and the restriction weight max(0, 1 - nvert)
 // (MyRestriction, poisson.c:433-441), in both precisions.
-__global__ void k_level_masks(Grid g, Box b, const double *nvert, uint8_t *blank, double *w64, float *w32,
-                              double *aj_box, const double *aj_da) {
+__global__ void k_level_masks(Grid g, Box b, const double *nvert, uint8_t *blank, double *w64, float *w32) {
   size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= b.n()) return;
   int i, j, k;
   box_ijk(b, c, i, j, k);
   double nv = nvert[g.at(i + 1, j + 1, k + 1)];
   double w = 1 - nv > 0. ? 1 - nv : 0.;
-  if (blank) blank[c] = nv > 0.1 ? 1 : 0;  // (null outputs are skipped)
-  if (w64) w64[c] = w;
-  if (w32) w32[c] = (float)w;
-  if (aj_box) aj_box[c] = aj_da[g.at(i + 1, j + 1, k + 1)];
+  blank[c] = nv > 0.1 ? 1 : 0;
+  w64[c] = w;
+  w32[c] = (float)w;
 }
 
 // --------------------------------------------------------------------------
 // Right-hand side: PoissonRHS2_hypre (Source/poisson_hypre.c:265-407) and
 // Remove_Nullspace_Scale (:118-200)
 // --------------------------------------------------------------------------
-__global__ void k_rhs(Grid g, Box b, const double *__restrict__ nvert, const double *__restrict__ ucont,
-                      const double *__restrict__ aj, double dt, double st, double coeff, double *rhs,
-                      double *partial) {
-  double sb = 0, sa = 0;
+// The fluid test is the mask's byte plane and the sum of aj over the fluid,
+// which the mask alone decides, is formed with it (k_fluid_mask): 7 FP64
+// instructions per cell (the pipe that bounds this kernel) and 33 bytes,
+// against 10 and 48.  256x192x256: 0.18 ms (0.26 ms before; at 40 registers
+// the fixed grid did not fit the SMs in one wave).
+__global__ void __launch_bounds__(256, 8) k_rhs(Grid g, Box b, const uint8_t *__restrict__ fluid,
+                                                const double *__restrict__ ucont, double dt, double st, double coeff,
+                                                double *__restrict__ rhs, double *partial) {
+  double sb = 0;
   const size_t n = b.n();
   const double f = -1.0 / dt * st * coeff;  // the reference's factor, formed once
+  const int sj = 3 * g.mx, sk = 3 * g.mx * g.my;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    int i, j, k;
-    box_ijk(b, c, i, j, k);
-    i++; j++; k++;
-    size_t t = g.at(i, j, k);
     double val = 0.;
-    if (nvert[t] < 0.1) {
-#define U(a, bb, cc, q) ucont[g.at(a, bb, cc) * 3 + (q)]
-      val -= U(i, j, k, 0);
-      if (i == 1 && g.px) val += U(g.mx - 2, j, k, 0);
-      else val += U(i - 1, j, k, 0);
-      val -= U(i, j, k, 1);
-      if (j == 1 && g.py) val += U(i, g.my - 2, k, 1);
-      else val += U(i, j - 1, k, 1);
-      val -= U(i, j, k, 2);
-      if (k == 1 && g.pz) val += U(i, j, g.mz - 2, 2);
-      else val += U(i, j, k - 1, 2);
-#undef U
+    if (fluid[c]) {
+      int i, j, k;
+      box_ijk(b, c, i, j, k);
+      const double *__restrict__ u = ucont + g.at(i + 1, j + 1, k + 1) * 3;
+      // (0 - U_i) + U_{i-1} as one subtraction: the same value
+      val = u[i == 0 && g.px ? 3 * (b.nx - 1) : -3] - u[0];
+      val -= u[1];
+      val += u[1 + (j == 0 && g.py ? (b.ny - 1) * sj : -sj)];
+      val -= u[2];
+      val += u[2 + (k == 0 && g.pz ? (ptrdiff_t)(b.nz - 1) * sk : -(ptrdiff_t)sk)];
       val *= f;
       sb += val;
-      sa += aj[t];
     }
     rhs[c] = val;
   }
-  double tb = block_sum(sb);
-  double ta = block_sum(sa);
-  if (threadIdx.x == 0) { partial[blockIdx.x] = tb; partial[gridDim.x + blockIdx.x] = ta; }
+  const double tb = block_sum(sb);
+  if (threadIdx.x == 0) partial[blockIdx.x] = tb;
 }
 
 // PoissonRHS2 (Source/poisson.c:1780-1906), the -poisson 0 / -1 variant:
@@ -773,23 +769,17 @@ __device__ __forceinline__ double markstein(double a, double d, double y) {
   r = fma(-q, d, a);
   return fma(r, y, q);
 }
-__device__ __forceinline__ double div_rn(double a, double d, double y) {
-  return isfinite(y) ? markstein(a, d, y) : a / d;
-}
 
-__global__ void k_rhs_nullspace(Grid g, Box b, const double *__restrict__ nvert, const double *__restrict__ aj,
-                                const double *sums, double *rhs) {
-  const double sum = sums[0], sum_aj = sums[1], y = 1.0 / sum_aj;
+__global__ void __launch_bounds__(256, 8) k_rhs_nullspace(Box b, const uint8_t *__restrict__ fluid,
+                                                          const double *__restrict__ aj_box, const double *sums,
+                                                          const double *fsum, double *__restrict__ rhs) {
+  const double sum = sums[0], sum_aj = fsum[0], y = 1.0 / sum_aj;
+  const bool fast = isfinite(y);
   const size_t n = b.n();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    int i, j, k;
-    box_ijk(b, c, i, j, k);
-    i++; j++; k++;
-    size_t t = g.at(i, j, k);
-    if (nvert[t] < 0.1) {
-      const double val = div_rn(-sum * aj[t], sum_aj, y);
-      rhs[c] += val;
-    }
+    if (!fluid[c]) continue;
+    const double a = -sum * aj_box[c];
+    rhs[c] += fast ? markstein(a, sum_aj, y) : a / sum_aj;
   }
 }
 
@@ -847,49 +837,77 @@ __global__ void k_nullspace_apply(Grid g, const double *__restrict__ nvert, cons
 
 // Remove_Nullspace (Source/poisson_hypre.c:202-263) on a box vector: sum and
 // count over nvert < 0.1
-__global__ void k_mean_partial(Box b, const uint8_t *fluid, const double *x, double *partial) {
-  double s = 0, cnt = 0;
-  const size_t n = b.n();
+__global__ void __launch_bounds__(256, 8) k_mean_partial(size_t n, const uint8_t *__restrict__ fluid,
+                                                         const double *__restrict__ x, double *partial) {
+  double s = 0;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
-    if (fluid[c]) { s += x[c]; cnt += 1.0; }
-  double ts = block_sum(s);
-  double tc = block_sum(cnt);
-  if (threadIdx.x == 0) { partial[blockIdx.x] = ts; partial[gridDim.x + blockIdx.x] = tc; }
+    if (fluid[c]) s += x[c];
+  const double ts = block_sum(s);
+  if (threadIdx.x == 0) partial[blockIdx.x] = ts;
 }
-__global__ void k_fluid_mask(Grid g, Box b, const double *nvert, uint8_t *fluid) {
-  size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= b.n()) return;
-  int i, j, k;
-  box_ijk(b, c, i, j, k);
-  i++; j++; k++;
-  fluid[c] = nvert[g.at(i, j, k)] < 0.1 ? 1 : 0;
+// The fluid mask of a new nvert (nvert < 0.1), aj at the box cells, and the
+// block partials of what the mask alone decides: the sum of aj over the
+// fluid cells (row 0, Remove_Nullspace_Scale's sum_aj) and their count (row
+// 1, Remove_Nullspace's).
+__global__ void __launch_bounds__(256, 8) k_fluid_mask(Grid g, Box b, const double *__restrict__ nvert,
+                                                       const double *__restrict__ aj, uint8_t *__restrict__ fluid,
+                                                       double *__restrict__ aj_box, double *partial) {
+  double sa = 0;
+  int cnt = 0;
+  const size_t n = b.n();
+  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
+    int i, j, k;
+    box_ijk(b, c, i, j, k);
+    const size_t t = g.at(i + 1, j + 1, k + 1);
+    const bool f = nvert[t] < 0.1;
+    const double a = aj[t];
+    fluid[c] = f ? 1 : 0;
+    aj_box[c] = a;
+    if (f) sa += a;
+    cnt += f ? 1 : 0;
+  }
+  const double ta = block_sum(sa);
+  const int tc = block_sum(cnt);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = ta;
+    partial[gridDim.x + blockIdx.x] = (double)tc;
+  }
 }
 
-// Remove_Nullspace's shift from the fluid sum and count (sums[0], sums[1]):
-// sums[2] = -sum / count, as k_shift_fluid forms it
-__global__ void k_mean_shift(double *sums) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) sums[2] = -sums[0] / sums[1];
+// Remove_Nullspace's shift, -sum / count, from the block partials of the
+// fluid sum (in k_reduce_rows' order) and the mask's count; one block
+__global__ void k_mean_shift(const double *partial, int nb, const double *fsum, double *shift) {
+  double s = 0;
+  for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[q];
+  s = block_sum(s);
+  if (threadIdx.x == 0) *shift = -s / fsum[1];
 }
 
 // Convert_Phi2_Phi (Source/poisson.c:98-186): box phi -> DA phi, zero on
 // non-dof cells and non-periodic ghosts, partner values on periodic ghosts.
 // With `shift` (device, one value), Remove_Nullspace's x += shift on the
 // fluid cells (nvert < 0.1) is applied on the way (x itself is left as is).
-__global__ void k_box_to_da_phi(Grid g, Box b, const double *nvert, const double *x, double *phi,
-                                const double *shift) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-  if (i >= g.mx) return;
-  int a, bb, c, fi, fj, fk;
+// One thread per point in linear order (a row of 258 points would leave the
+// third block of a row-wise launch nearly empty), the dof and fluid tests from
+// byte planes: 18 bytes per point.
+__global__ void __launch_bounds__(256) k_box_to_da_phi(Grid g, Box b, const uint8_t *__restrict__ rowtype,
+                                                       const uint8_t *__restrict__ fluid,
+                                                       const double *__restrict__ x, double *__restrict__ phi,
+                                                       const double *shift) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= g.n()) return;
+  int i, j, k, a, bb, c, fi, fj, fk;
+  da_ijk(g, t, i, j, k);
   g.remap(i, j, k, a, bb, c, fi, fj, fk);
   double v = 0.;
   if (a >= 1 && a < g.mx - 1 && bb >= 1 && bb < g.my - 1 && c >= 1 && c < g.mz - 1) {
-    const double nv = nvert[g.at(a, bb, c)];
-    if (!((int)nv > kThr)) {
-      v = x[b.at(a - 1, bb - 1, c - 1)];
-      if (shift && nv < 0.1) v += shift[0];
+    const size_t q = b.at(a - 1, bb - 1, c - 1);
+    if (rowtype[q]) {
+      v = x[q];
+      if (shift && fluid[q]) v += shift[0];
     }
   }
-  phi[g.at(i, j, k)] = v;
+  phi[t] = v;
 }
 // DA -> box copy of the interior (warm start / inspection input)
 __global__ void k_da_to_box(Grid g, Box b, const double *da, double *x) {
@@ -900,13 +918,16 @@ __global__ void k_da_to_box(Grid g, Box b, const double *da, double *x) {
   i++; j++; k++;
   x[c] = da[g.at(i, j, k)];
 }
-__global__ void k_box_to_da(Grid g, Box b, const double *x, double *da) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-  if (i >= g.mx) return;
+__global__ void __launch_bounds__(256) k_box_to_da(Grid g, Box b, const double *__restrict__ x,
+                                                   double *__restrict__ da) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= g.n()) return;
+  int i, j, k;
+  da_ijk(g, t, i, j, k);
   double v = 0.;
   if (i >= 1 && i < g.mx - 1 && j >= 1 && j < g.my - 1 && k >= 1 && k < g.mz - 1)
     v = x[b.at(i - 1, j - 1, k - 1)];
-  da[g.at(i, j, k)] = v;
+  da[t] = v;
 }
 
 // Periodic ghost points, one thread per point of the two boundary layers of
@@ -950,8 +971,8 @@ __global__ void __launch_bounds__(256) k_update_pressure(Grid g, const double *_
                                                          double *__restrict__ phi_out) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.n()) return;
-  const uint32_t row = (uint32_t)t / (uint32_t)g.mx;
-  const int i = (int)((uint32_t)t - row * g.mx), j = (int)(row % (uint32_t)g.my), k = (int)(row / (uint32_t)g.my);
+  int i, j, k;
+  da_ijk(g, t, i, j, k);
   const double f = phi[t];
   if (phi_out) phi_out[t] = f;
   if (i < 1 || i >= g.mx - 1 || j < 1 || j >= g.my - 1 || k < 1 || k >= g.mz - 1) return;
@@ -1396,29 +1417,32 @@ __device__ inline int vflux_faces(Grid g, const double *nvert, MetricPtrs m, dou
   return nf;
 }
 
-// pass 0: zero |U| <= 1e-8 and sum flux, |U| (or |U| / area for flg 3)
-// and area; pass 2: sum flux and area after the correction
-__global__ void k_vflux_sum(Grid g, const double *__restrict__ nvert, MetricPtrs m, double *ucont, int flg, int pass,
-                            double *partial) {
+// Both passes look only at the cells of the near plane (elsewhere no face
+// qualifies): one byte per cell instead of five nvert values and a 64-bit
+// index division.  256x192x256: 0.22 ms for the two passes (0.89 ms as three
+// passes over every cell).
+//
+// First pass: zero |U| <= 1e-8 and sum flux, |U| (or |U| / area for flg 3)
+// and area
+__global__ void __launch_bounds__(256) k_vflux_sum(Grid g, Box b, const double *__restrict__ nvert,
+                                                   const uint8_t *__restrict__ near, MetricPtrs m, double *ucont,
+                                                   int flg, double *partial) {
   double sf = 0, sab = 0, sa = 0;
-  const size_t n = (size_t)(g.mx - 2) * (g.my - 2) * (g.mz - 2);
+  const size_t n = b.n();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    const int i = c % (g.mx - 2) + 1, j = (c / (g.mx - 2)) % (g.my - 2) + 1, k = c / ((size_t)(g.mx - 2) * (g.my - 2)) + 1;
+    if (!near[c]) continue;
+    int i, j, k;
+    box_ijk(b, c, i, j, k);
     VfluxFace f[6];
-    const int nf = vflux_faces(g, nvert, m, ucont, i, j, k, f);
+    const int nf = vflux_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, f);
     for (int q = 0; q < nf; q++) {
       const double u = *f[q].u;
-      if (pass == 0) {
-        if (fabs(u) > 1.e-8) {
-          sf += f[q].s == 0 ? u : -u;
-          sab += flg == 3 ? fabs(u) / f[q].a : fabs(u);
-          sa += f[q].a;
-        } else {
-          *f[q].u = 0.;
-        }
-      } else {
+      if (fabs(u) > 1.e-8) {
         sf += f[q].s == 0 ? u : -u;
+        sab += flg == 3 ? fabs(u) / f[q].a : fabs(u);
         sa += f[q].a;
+      } else {
+        *f[q].u = 0.;
       }
     }
   }
@@ -1429,23 +1453,60 @@ __global__ void k_vflux_sum(Grid g, const double *__restrict__ nvert, MetricPtrs
     partial[2 * gridDim.x + blockIdx.x] = t2;
   }
 }
+// The correction from the first pass's partials, rows summed in
+// k_reduce_rows' order (one block; flg 4: the overload for immersed != 1,
+// whose rows are flux and area).
+__global__ void k_vflux_corr(const double *partial, int nb, int flg, double flux_intp_sum, double *corr) {
+  double sums[3] = {0., 0., 0.};
+  for (int r = 0; r < (flg == 4 ? 2 : 3); r++) {
+    double s = 0;
+    for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[(size_t)r * nb + q];
+    sums[r] = block_sum(s);
+  }
+  if (threadIdx.x) return;
+  double v = 0.;
+  if (flg == 4) {
+    if (sums[1] > 1.e-15) v = sums[0] / sums[1];
+  } else if (sums[2] > 1.e-15) {
+    if (flg > 1) v = (sums[0] + flux_intp_sum) / sums[1];
+    else if (flg) v = (sums[0] + flux_intp_sum) / sums[2];
+    else v = sums[0] / sums[2];
+  }
+  *corr = v;
+}
 
-__global__ void k_vflux_apply(Grid g, const double *__restrict__ nvert, MetricPtrs m, double *ucont, int flg,
-                              double corr) {
-  const size_t n = (size_t)(g.mx - 2) * (g.my - 2) * (g.mz - 2);
+// Second pass: the correction, and the flux and area after it (each face
+// belongs to one cell, so its new value is final)
+__global__ void __launch_bounds__(256) k_vflux_apply(Grid g, Box b, const double *__restrict__ nvert,
+                                                     const uint8_t *__restrict__ near, MetricPtrs m, double *ucont,
+                                                     int flg, const double *corr, double *partial) {
+  const double cr = *corr;
+  double sf = 0, sa = 0;
+  const size_t n = b.n();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    const int i = c % (g.mx - 2) + 1, j = (c / (g.mx - 2)) % (g.my - 2) + 1, k = c / ((size_t)(g.mx - 2) * (g.my - 2)) + 1;
+    if (!near[c]) continue;
+    int i, j, k;
+    box_ijk(b, c, i, j, k);
     VfluxFace f[6];
-    const int nf = vflux_faces(g, nvert, m, ucont, i, j, k, f);
+    const int nf = vflux_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, f);
     for (int q = 0; q < nf; q++) {
-      const double u = *f[q].u;
-      if (!(fabs(u) > 1.e-8)) continue;
-      double dlt;
-      if (flg == 3) dlt = corr * fabs(u) / f[q].a;
-      else if (flg == 2) dlt = corr * fabs(u);
-      else dlt = f[q].a * corr;
-      *f[q].u = f[q].s == 0 ? u - dlt : u + dlt;
+      double u = *f[q].u;
+      if (fabs(u) > 1.e-8) {
+        double dlt;
+        if (flg == 3) dlt = cr * fabs(u) / f[q].a;
+        else if (flg == 2) dlt = cr * fabs(u);
+        else dlt = f[q].a * cr;
+        u = f[q].s == 0 ? u - dlt : u + dlt;
+        *f[q].u = u;
+      }
+      sf += f[q].s == 0 ? u : -u;
+      sa += f[q].a;
     }
+  }
+  const double t0 = block_sum(sf), t1 = block_sum(sa);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = t0;
+    partial[gridDim.x + blockIdx.x] = t1;
   }
 }
 
@@ -1476,14 +1537,17 @@ __device__ inline int vflux0_faces(Grid g, const double *nvert, MetricPtrs m, do
 
 // block partials of the flux (+U on the fluid side, -U on the blanked side)
 // and of the area
-__global__ void k_vflux0_sum(Grid g, const double *__restrict__ nvert, MetricPtrs m, double *ucont,
-                             double *partial) {
+__global__ void __launch_bounds__(256) k_vflux0_sum(Grid g, Box b, const double *__restrict__ nvert,
+                                                    const uint8_t *__restrict__ near, MetricPtrs m, double *ucont,
+                                                    double *partial) {
   double sf = 0, sa = 0;
-  const size_t n = (size_t)(g.mx - 2) * (g.my - 2) * (g.mz - 2);
+  const size_t n = b.n();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    const int i = c % (g.mx - 2) + 1, j = (c / (g.mx - 2)) % (g.my - 2) + 1, k = c / ((size_t)(g.mx - 2) * (g.my - 2)) + 1;
+    if (!near[c]) continue;
+    int i, j, k;
+    box_ijk(b, c, i, j, k);
     VfluxFace f[6];
-    const int nf = vflux0_faces(g, nvert, m, ucont, i, j, k, f);
+    const int nf = vflux0_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, f);
     for (int q = 0; q < nf; q++) {
       const double u = *f[q].u;
       sf += f[q].s == 0 ? u : -u;
@@ -1498,19 +1562,32 @@ __global__ void k_vflux0_sum(Grid g, const double *__restrict__ nvert, MetricPtr
 }
 
 // the correction: off the fluid side, onto the blanked side; then the face
-// is zeroed when `zero` (immersed 0 or 3)
-__global__ void k_vflux0_apply(Grid g, const double *__restrict__ nvert, MetricPtrs m, double *ucont, double corr,
-                               int zero) {
-  const size_t n = (size_t)(g.mx - 2) * (g.my - 2) * (g.mz - 2);
+// is zeroed when `zero` (immersed 0 or 3); the flux and area after it
+__global__ void __launch_bounds__(256) k_vflux0_apply(Grid g, Box b, const double *__restrict__ nvert,
+                                                      const uint8_t *__restrict__ near, MetricPtrs m, double *ucont,
+                                                      const double *corr, int zero, double *partial) {
+  const double cr = *corr;
+  double sf = 0, sa = 0;
+  const size_t n = b.n();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    const int i = c % (g.mx - 2) + 1, j = (c / (g.mx - 2)) % (g.my - 2) + 1, k = c / ((size_t)(g.mx - 2) * (g.my - 2)) + 1;
+    if (!near[c]) continue;
+    int i, j, k;
+    box_ijk(b, c, i, j, k);
     VfluxFace f[6];
-    const int nf = vflux0_faces(g, nvert, m, ucont, i, j, k, f);
+    const int nf = vflux0_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, f);
     for (int q = 0; q < nf; q++) {
-      const double u = *f[q].u;
-      const double dlt = f[q].a * corr;
-      *f[q].u = zero ? 0. : (f[q].s == 0 ? u - dlt : u + dlt);
+      double u = *f[q].u;
+      const double dlt = f[q].a * cr;
+      u = zero ? 0. : (f[q].s == 0 ? u - dlt : u + dlt);
+      *f[q].u = u;
+      sf += f[q].s == 0 ? u : -u;
+      sa += f[q].a;
     }
+  }
+  const double t0 = block_sum(sf), t1 = block_sum(sa);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = t0;
+    partial[gridDim.x + blockIdx.x] = t1;
   }
 }
 
