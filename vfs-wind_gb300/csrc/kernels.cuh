@@ -149,6 +149,37 @@ LINE_FUSED_DECL(k_line_fused16)
 LINE_FUSED_DECL(k_line_fused16_oz)
 LINE_FUSED_DECL(k_line_fused16_z)
 #undef LINE_FUSED_DECL
+// The V-cycle's tail (vtail.cu): all levels from the first small one down to
+// the coarsest and back, in one cluster of CTAs.  Level l's k-planes are dealt
+// to the CTAs q at a time; x, t, b and r live in their shared memory (byte
+// offsets ox, ot, ob, orr; rows of rs words, columns at their split
+// positions), the operator too (oA) when it fits (res).
+constexpr int kTailLevels = 10, kTailThreads = 512, kTailDofs = 384;
+// FP32 works on units of 8 rows x 4 columns, one a warp at a time
+constexpr int kTailUnits = 4 * (kTailThreads / 32);
+struct TailLevel {
+  Box b;
+  FastDiv dnh, dcw, dq, dP, dnq, dr4;  // by (nx + 1) / 2, cw, q, P, nq and the copies of an operator row
+  int cx, cy, cz;                      // coarsening to the next level
+  int q, res, rs;
+  int P, cw, nq;  // chunks of a j-line (at most 32), columns a warp takes (32 / P), column quads of a colour
+  const void *A, *D, *Asp, *inv, *cp, *w;  // FP32: A the packed couplings, D the diagonal; FP64: A the 19 planes
+  const uint8_t *blank;
+  uint32_t ox, ot, ob, orr, oA, obl;  // obl: blank flags (the first level: the CTA's planes; the others: all)
+};
+struct TailArgs {
+  int nl, nu1, nu2;
+  double omega;
+  const void *b;  // right-hand side of the first level
+  void *x;        // its correction
+  int nd, nc;     // dofs and cells of the coarsest level
+  const int *dmap, *didx;
+  const double *dinv;
+  uint32_t osb, odi;  // shared memory of the coarsest gather and of its index lists
+  TailLevel lv[kTailLevels];
+};
+__global__ void k_vtail_f32(const __grid_constant__ TailArgs a);
+__global__ void k_vtail_f64(const __grid_constant__ TailArgs a);
 __global__ void k_apply64(Box b, const double *A, const double *x, double *y);
 __global__ void k_residual64(Box b, const double *A, const double *x, const double *rhs, double *r, double *partial);
 __global__ void k_residual64r(Box b, const double *A, const double *x, const double *rhs, double *r);

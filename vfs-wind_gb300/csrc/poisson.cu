@@ -488,6 +488,10 @@ struct vfs_poisson {
   // dependent launch; VFS_PDL=0 at create turns it off); pdl_prev: the last
   // operation issued on the stream was such a kernel
   bool pdl = true, pdl_prev = false;
+  // the V-cycle's tail in one cluster (vtail.cu): CTAs of the cluster (0: the
+  // device cannot hold one) and the dynamic shared memory of one, per precision
+  int tail_ctas[2] = {0, 0};
+  size_t tail_smem[2] = {0, 0};
   // incremental refill of the finest level on a new mask (VFS_INCREMENTAL=0
   // at create turns it off): the mask the hierarchy was last filled with
   // (nvert_prev after the swap), the changed DA points, the rows to refill
@@ -1306,10 +1310,156 @@ void smooth(vfs_poisson *h, Level &l, int li, int smoother, bool zero_guess, T o
   prof_end(h, li);
 }
 
+// What the V-cycle's tail can hold on this device: the largest cluster that
+// fits with all the shared memory of its SMs.
+void tail_limits(vfs_poisson *h) {
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+  for (int p = 0; p < 2; p++) {
+    auto kern = p ? k_vtail_f64 : k_vtail_f32;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.sharedSizeBytes >= (size_t)optin) continue;
+    const size_t dyn = ((size_t)optin - fa.sharedSizeBytes) & ~(size_t)15;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      continue;
+    for (int nc : {16, 8}) {
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim = {(unsigned)nc, 1, 1};
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = nc;
+      cfg.blockDim = kTailThreads;
+      cfg.dynamicSmemBytes = dyn;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0) {
+        h->tail_ctas[p] = nc;
+        h->tail_smem[p] = dyn;
+        break;
+      }
+    }
+  }
+  cudaGetLastError();
+}
+
+// The tail kernel's arguments for the levels li .. coarsest; false when they
+// do not suit it.  Cells per CTA bound a phase's time: a colour of 256 cells a
+// CTA takes 2.6 us there and 4.2 us as a launch, one of 2048 cells 5 and 4.6
+// us, one of 3072 cells 9 and 5 us (FP64: 720 cells 7.5 and 9.5 us).  Solves
+// with limits of 0, 512, 2048, 4096 cells: 24x16x24 1525, 1321, 1220, 1210 us;
+// 64^3 2165, 1924, 1908, 1902; 128x96x128 6022, 5649, 5651, 5838; FP64
+// 72x40x56 6833, 6141, 6084, 6137.  A coarsest inverse of more than kTailDofs
+// rows is better spread over the whole chip.
+constexpr size_t kTailCells[2] = {2048, 2048};
+template <typename T>
+bool tail_plan(vfs_poisson *h, int li, int nu1, int smoother, TailArgs *a, size_t *smem) {
+  constexpr int p = std::is_same<T, double>::value;
+  const int nl = (int)h->L.size() - li, nc = h->tail_ctas[p];
+  const Level &last = h->L.back();
+  if (smoother != 4 || !nc || nl < 2 || nl > kTailLevels || (h->prof && li == 0) || last.nd > kTailDofs) return false;
+  size_t used = 0;
+  auto bytes = [&](size_t n) {
+    const size_t o = used;
+    used += (n + 15) & ~(size_t)15;
+    return (uint32_t)o;
+  };
+  auto take = [&](size_t words) { return bytes(words * sizeof(T)); };
+  a->nl = nl;
+  a->nd = last.nd;
+  a->nc = (int)last.b.n();
+  a->osb = bytes(last.nd * sizeof(double));
+  a->odi = bytes((last.nd + last.b.n()) * sizeof(int));
+  for (int m = 0; m < nl; m++) {
+    Level &l = h->L[li + m];
+    TailLevel &t = a->lv[m];
+    const Box &b = l.b;
+    // FP32 rows of 4 (2 r + 1) words: 8 rows of 4 columns lie in 32 banks
+    t.rs = p ? b.nx : ((b.nx + 3) / 4 | 1) * 4;
+    t.b = b;
+    t.dnh.set((b.nx + 1) / 2);
+    t.cx = l.cx; t.cy = l.cy; t.cz = l.cz;
+    t.q = (b.nz + nc - 1) / nc;
+    t.dq.set(t.q);
+    t.res = 0;
+    t.P = (b.ny + kLineChunk - 1) / kLineChunk;
+    t.nq = ((b.nx + 1) / 2 + 3) / 4;
+    if (t.P > 32 || (size_t)t.q * b.nx * b.ny > kTailCells[p] || (!p && t.q * t.nq * t.P > kTailUnits)) return false;
+    t.cw = 32 / t.P;
+    t.dcw.set(t.cw);
+    t.dP.set(t.P);
+    t.dnq.set(t.nq);
+    t.dr4.set(b.nx * sizeof(T) % 16 ? b.nx : (int)(b.nx * sizeof(T) / 16));
+    t.blank = l.blank;
+    const size_t slab = (size_t)t.rs * b.ny;
+    t.obl = bytes(m ? b.n() : (size_t)t.q * b.nx * b.ny);
+    t.ox = take((t.q + 2) * slab);
+    t.ob = take(t.q * slab);
+    t.ot = t.orr = t.oA = 0;
+    t.A = t.D = t.Asp = t.inv = t.cp = t.w = nullptr;
+    if (m == nl - 1) continue;
+    t.ot = take((t.q + 2) * slab);
+    // the weighted residual: FP32 forms it straight where x is not (the buffer
+    // that holds no x after nu1 sweeps)
+    t.orr = p ? take(t.q * slab) : (nu1 & 1 ? t.ox : t.ot) + (uint32_t)(slab * sizeof(T));
+    t.A = p ? (const void *)l.A64 : (const void *)l.C16;
+    t.D = l.D32;
+    t.Asp = Prec<T>::A(l) + (size_t)SP * b.n();
+    t.inv = Prec<T>::inv(l);
+    t.cp = Prec<T>::cp(l);
+    t.w = Prec<T>::w(l);
+  }
+  if (used > h->tail_smem[p]) return false;
+  // the operators in shared memory, the coarse ones (read as often, and
+  // small) first
+  for (int m = nl - 2; m >= 0; m--) {
+    TailLevel &t = a->lv[m];
+    const size_t words = (size_t)t.q * t.rs * t.b.ny * (p ? 21 : 14);
+    if (used + words * sizeof(T) + 16 > h->tail_smem[p]) break;
+    t.oA = take(words);
+    t.res = 1;
+  }
+  a->b = Prec<T>::v(h->L[li])[1];
+  a->x = Prec<T>::v(h->L[li])[0];
+  a->dmap = last.dmap;
+  a->didx = last.didx;
+  a->dinv = last.dinv;
+  *smem = used;
+  return true;
+}
+void launch_tail(vfs_poisson *h, bool fp64, const TailArgs &a, size_t smem) {
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {(unsigned)h->tail_ctas[fp64], 1, 1};
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = h->tail_ctas[fp64];
+  cfg.blockDim = kTailThreads;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = h->pdl && h->pdl_prev ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, fp64 ? k_vtail_f64 : k_vtail_f32, a);
+  h->pdl_prev = true;
+  h->launches++;
+}
+
 template <typename T>
 void vcycle(vfs_poisson *h, int li, int nu1, int nu2, T omega, int smoother) {
   Level &l = h->L[li];
   T **v = Prec<T>::v(l);
+  TailArgs ta;
+  size_t tsm;
+  if (tail_plan<T>(h, li, nu1, smoother, &ta, &tsm)) {
+    ta.nu1 = nu1;
+    ta.nu2 = nu2;
+    ta.omega = omega;
+    launch_tail(h, std::is_same<T, double>::value, ta, tsm);
+    Prec<T>::xfinal(l) = v[0];
+    return;
+  }
   T *x = v[0], *bb = v[1], *r = v[2], *t = v[3];
   if (li == (int)h->L.size() - 1) {
     launch_v(h, Prec<T>::coarsest, (int)((l.b.n() + 7) / 8), 256, 0, l.nd, l.dmap, l.didx, l.dinv, bb, x,
@@ -2127,6 +2277,7 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
     const char *inc = getenv("VFS_INCREMENTAL");
     h->inc_enable = !(inc && inc[0] == '0');
   }
+  tail_limits(h);
   const size_t N = h->g.n(), n = h->box.n();
   int rc;
   if ((rc = dalloc(h, &h->coor, 3 * N)) || (rc = dalloc(h, &h->nvert, N)) || (rc = dalloc(h, &h->ucont, 3 * N)) ||

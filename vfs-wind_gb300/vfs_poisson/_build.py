@@ -24,6 +24,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE
 UNITS = {
     "setup.cu": ["-fmad=false"],
     "solve.cu": [],
+    "vtail.cu": [],
     "poisson.cu": [],
     "noalloc.cu": ["-fmad=false"],
     "ibm.cu": ["-fmad=false", "-Xcompiler", "-ffp-contract=off"],
