@@ -897,8 +897,8 @@ namespace vfs {
 // noslip velocity and interpolated pressure at every IB node of one body
 // (ibm.c:3405-3560, wallfunction.c:140-156); lucat / lp are the inputs as
 // read (the reference's local copies), ucat / p are written at the nodes.
-__global__ void k_ibm_apply(Grid g, const vfs_ibm_node *nodes, int n_nodes, const int *tri, const double *u_surf,
-                            const double *nvert, const double *lucat, const double *lp, double *ucat, double *p) {
+__global__ void k_ibm_gather(Grid g, const vfs_ibm_node *nodes, int n_nodes, const int *tri, const double *u_surf,
+                             const double *nvert, const double *lucat, const double *lp, double *val) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= n_nodes) return;
   const vfs_ibm_node nd = nodes[n];
@@ -914,17 +914,25 @@ __global__ void k_ibm_apply(Grid g, const vfs_ibm_node *nodes, int n_nodes, cons
       ua[q] = u_surf[3 * v1 + q] * nd.cs[0] + u_surf[3 * v2 + q] * nd.cs[1] + u_surf[3 * v3 + q] * nd.cs[2];
   }
   if (nvert[t1] + nvert[t2] + nvert[t3] > 0.1 || nvert[t] > 2.9) {
-    for (int q = 0; q < 3; q++) ucat[t * 3 + q] = 0.;
+    for (int q = 0; q < 3; q++) val[(size_t)n * 4 + q] = 0.;
   } else {
     for (int q = 0; q < 3; q++) {
       const double uc = (lucat[t1 * 3 + q] * sk1 + lucat[t2 * 3 + q] * sk2 + lucat[t3 * 3 + q] * sk3);
       const double uq = uc - ua[q];
       double v = sb / sc * uq;
       v += ua[q];
-      ucat[t * 3 + q] = v;
+      val[(size_t)n * 4 + q] = v;
     }
   }
-  p[t] = (lp[t1] * sk1 + lp[t2] * sk2 + lp[t3] * sk3);
+  val[(size_t)n * 4 + 3] = (lp[t1] * sk1 + lp[t2] * sk2 + lp[t3] * sk3);
+}
+__global__ void k_ibm_scatter(Grid g, const vfs_ibm_node *nodes, int n_nodes, const double *val, double *ucat,
+                              double *p) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= n_nodes) return;
+  const size_t t = g.at(nodes[n].i, nodes[n].j, nodes[n].k);
+  for (int q = 0; q < 3; q++) ucat[t * 3 + q] = val[(size_t)n * 4 + q];
+  p[t] = val[(size_t)n * 4 + 3];
 }
 
 __device__ inline double face_flux(const double *lu, size_t a, size_t b, const double *m) {
@@ -935,33 +943,41 @@ __device__ inline double face_flux(const double *lu, size_t a, size_t b, const d
 }
 
 // the face fluxes around the IB nodes (ibm.c:3577-3630): every interior
-// cell writes only its own three faces, so cells are independent
-__global__ void k_ibm_faces(Grid g, const double *nvert, const double *lu, const double *icsi, const double *jeta,
-                            const double *kzet, double f, int b0, int b1, int b2, int b3, int b4, int b5,
-                            double *ucont) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, k = blockIdx.z + 1;
-  if (i >= g.mx - 1) return;
+// cell writes only its own three faces, so cells are independent.  A cell
+// without a blanked point near has no such face: one byte of the 24 it would
+// read of nvert, and no FP64.  u: ucat, whose periodic ghosts are read in
+// their partners.
+__global__ void k_ibm_faces(Grid g, Box b, const double *__restrict__ nvert, const uint8_t *__restrict__ near,
+                            const double *__restrict__ lu, const double *icsi, const double *jeta, const double *kzet,
+                            double f, int b0, int b1, int b2, int b3, int b4, int b5, double *ucont) {
+  const size_t bc = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (bc >= b.n() || !near[bc]) return;
+  int i, j, k;
+  box_ijk(b, bc, i, j, k);
+  i++, j++, k++;
   const size_t t = g.at(i, j, k), te = g.at(i + 1, j, k), tn = g.at(i, j + 1, k), tt = g.at(i, j, k + 1);
+  const size_t ue = i == g.mx - 2 && g.px ? g.at(1, j, k) : te, un = j == g.my - 2 && g.py ? g.at(i, 1, k) : tn,
+               ut = k == g.mz - 2 && g.pz ? g.at(i, j, 1) : tt;
   const bool wi0 = b0 == -1 || b0 == -2, wi1 = b1 == -1 || b1 == -2, wj0 = b2 == -1 || b2 == -2,
              wj1 = b3 == -1 || b3 == -2, wk0 = b4 == -1 || b4 == -2, wk1 = b5 == -1 || b5 == -2;
   if ((int)(nvert[t] + 0.5) == 1) {
-    ucont[t * 3] = face_flux(lu, t, te, &icsi[t * 3]) * f;
-    ucont[t * 3 + 1] = face_flux(lu, tn, t, &jeta[t * 3]) * f;
-    ucont[t * 3 + 2] = face_flux(lu, tt, t, &kzet[t * 3]) * f;
+    ucont[t * 3] = face_flux(lu, t, ue, &icsi[t * 3]) * f;
+    ucont[t * 3 + 1] = face_flux(lu, un, t, &jeta[t * 3]) * f;
+    ucont[t * 3 + 2] = face_flux(lu, ut, t, &kzet[t * 3]) * f;
     if (wi0 && i == 1) ucont[t * 3] = 0;
     if (wj0 && j == 1) ucont[t * 3 + 1] = 0;
     if (wk0 && k == 1) ucont[t * 3 + 2] = 0;
   }
   if ((int)(nvert[te] + 0.5) == 1) {
-    ucont[t * 3] = face_flux(lu, t, te, &icsi[t * 3]) * f;
+    ucont[t * 3] = face_flux(lu, t, ue, &icsi[t * 3]) * f;
     if (wi1 && i == g.mx - 3) ucont[t * 3] = 0;
   }
   if ((int)(nvert[tn] + 0.5) == 1) {
-    ucont[t * 3 + 1] = face_flux(lu, tn, t, &jeta[t * 3]) * f;
+    ucont[t * 3 + 1] = face_flux(lu, un, t, &jeta[t * 3]) * f;
     if (wj1 && j == g.my - 3) ucont[t * 3 + 1] = 0;
   }
   if ((int)(nvert[tt] + 0.5) == 1) {
-    ucont[t * 3 + 2] = face_flux(lu, tt, t, &kzet[t * 3]) * f;
+    ucont[t * 3 + 2] = face_flux(lu, ut, t, &kzet[t * 3]) * f;
     if (wk1 && k == g.mz - 3) ucont[t * 3 + 2] = 0;
   }
 }
@@ -969,14 +985,17 @@ __global__ void k_ibm_faces(Grid g, const double *nvert, const double *lu, const
 // IB_BC's interior loop (momentum.c:2114-2178): the IB faces from ucat
 // ((int)nvert == 1), the immersed == 3 zeroing and the -1/-2 walls in i and
 // j (the i == 1 / j == 1 rows write the face below them, which no other cell
-// of this loop writes)
-__global__ void k_ib_bc_faces(Grid g, const double *nvert, const double *lu, const double *icsi,
-                              const double *jeta, const double *kzet, int immersed, int b0, int b1, int b2, int b3,
-                              double *ucont) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, k = blockIdx.z + 1;
-  if (i >= g.mx - 1) return;
+// of this loop writes); the mask is looked at next to a body only
+__global__ void k_ib_bc_faces(Grid g, Box b, const double *__restrict__ nvert, const uint8_t *__restrict__ near,
+                              const double *lu, const double *icsi, const double *jeta, const double *kzet,
+                              int immersed, int b0, int b1, int b2, int b3, double *ucont) {
+  const size_t bc = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (bc >= b.n()) return;
+  int i, j, k;
+  box_ijk(b, bc, i, j, k);
+  i++, j++, k++;
   const size_t t = g.at(i, j, k), te = g.at(i + 1, j, k), tn = g.at(i, j + 1, k), tt = g.at(i, j, k + 1);
-  if (immersed) {
+  if (immersed && near[bc]) {
     const double f = immersed == 3 ? 0. : 1.;
     if ((int)nvert[t] == 1) {
       ucont[t * 3] = face_flux(lu, t, te, &icsi[t * 3]) * f;
@@ -1008,37 +1027,40 @@ __global__ void k_ib_bc_faces(Grid g, const double *nvert, const double *lu, con
 // (10) walls and the periodic faces.  The reference runs it in place in
 // k, j, i order; a periodic copy there reads its partner before a slip rule
 // of the same row could zero it, so every value follows from the values
-// before the loop (uold).
-__global__ void k_ib_bc_edges(Grid g, const double *uold, int b0, int b1, int b2, int b3, int b4, int b5,
-                              double *ucont) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-  if (i >= g.mx) return;
-  const size_t t = g.at(i, j, k);
-  double vx = uold[t * 3], vy = uold[t * 3 + 1], vz = uold[t * 3 + 2];
-  if (i == 0) {
-    if (g.px) vx = uold[g.at(g.mx - 2, j, k) * 3];
-    if (b0 == 10) vx = 0;
-  } else if (i == g.mx - 1) {
-    if (g.px) vx = uold[g.at(1, j, k) * 3];
+// before the loop.  Component q changes at the ends of the lines along axis
+// q only, and no other line reads it: one thread a line takes both partners
+// before it writes, in place (the whole array was copied and rewritten
+// before: 192x128x192 71 -> 3 us).
+__global__ void k_ib_bc_edges(Grid g, int b0, int b1, int b2, int b3, int b4, int b5, double *ucont) {
+  const uint32_t nx = (uint32_t)g.my * g.mz, ny = (uint32_t)g.mx * g.mz, nz = (uint32_t)g.mx * g.my;
+  uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  int q, m, per, lo, hi;
+  size_t base, step;
+  if (u < nx) {
+    q = 0; m = g.mx; per = g.px; lo = b0; hi = b1;
+    base = (size_t)u * g.mx;
+    step = 1;
+  } else if ((u -= nx) < ny) {
+    q = 1; m = g.my; per = g.py; lo = b2; hi = b3;
+    const uint32_t k = u / (uint32_t)g.mx;
+    base = g.at((int)(u - k * g.mx), 0, (int)k);
+    step = g.mx;
+  } else if ((u -= ny) < nz) {
+    q = 2; m = g.mz; per = g.pz; lo = b4; hi = b5;
+    base = u;
+    step = (size_t)g.mx * g.my;
+  } else {
+    return;
   }
-  if (i == g.mx - 2 && b1 == 10) vx = 0;
-  if (j == 0) {
-    if (g.py) vy = uold[g.at(i, g.my - 2, k) * 3 + 1];
-    if (b2 == 10) vy = 0;
-  } else if (j == g.my - 1) {
-    if (g.py) vy = uold[g.at(i, 1, k) * 3 + 1];
+  double *line = ucont + base * 3 + q;
+  step *= 3;
+  const double first = line[step], last = line[(m - 2) * step];
+  if (per) {
+    line[0] = last;
+    line[(m - 1) * step] = first;
   }
-  if (j == g.my - 2 && b3 == 10) vy = 0;
-  if (k == 0) {
-    if (g.pz) vz = uold[g.at(i, j, g.mz - 2) * 3 + 2];
-    if (b4 == 10) vz = 0;
-  } else if (k == g.mz - 1) {
-    if (g.pz) vz = uold[g.at(i, j, 1) * 3 + 2];
-  }
-  if (k == g.mz - 2 && b5 == 10) vz = 0;
-  ucont[t * 3] = vx;
-  ucont[t * 3 + 1] = vy;
-  ucont[t * 3 + 2] = vz;
+  if (lo == 10) line[0] = 0;
+  if (hi == 10) line[(m - 2) * step] = 0;
 }
 
 }  // namespace vfs

@@ -53,9 +53,11 @@ __global__ void k_vflux0_sum(Grid g, Box b, const double *nvert, const uint8_t *
                              double *partial);
 __global__ void k_vflux0_apply(Grid g, Box b, const double *nvert, const uint8_t *near, MetricPtrs m, double *ucont,
                                const double *corr, int zero, double *partial);
-__global__ void k_periodic_cmpnts(Grid g, const double *src, double *dst);
-__global__ void k_contra2cart(Grid g, const double *nvert, MetricPtrs m, const double *lu, double *ucat);
-__global__ void k_zero_solid(Grid g, const double *nvert, double *ucat);
+__global__ void k_periodic_cmpnts(Grid g, double *u);
+__global__ void k_contra2cart_coef(Grid g, Box b, MetricPtrs m, double *cc);
+__global__ void k_contra2cart(Grid g, Box b, const double *nvert, const uint8_t *near, const double *cc,
+                              const double *u, double *ucat, int zero);
+__global__ void k_zero_rim(Grid g, const double *nvert, double *ucat);
 __global__ void k_cellfield_restrict(Grid gh, Grid gc, int cx, int cy, int cz, const double *fh, double *fc);
 __global__ void k_assemble(Grid g, Box b, const double *nvert, MetricPtrs m, int scale, int filter, int split, double *A,
                            uint8_t *rowtype, LevelSet ls);
@@ -278,15 +280,16 @@ struct IbmContext {
   IbmScratch *scratch;
 };
 // ibm.cu: the IB interpolation and IB_BC kernels (launched by poisson.cu)
-__global__ void k_ibm_apply(Grid g, const vfs_ibm_node *nodes, int n_nodes, const int *tri, const double *u_surf,
-                            const double *nvert, const double *lucat, const double *lp, double *ucat, double *p);
-__global__ void k_ibm_faces(Grid g, const double *nvert, const double *lu, const double *icsi, const double *jeta,
-                            const double *kzet, double f, int b0, int b1, int b2, int b3, int b4, int b5,
-                            double *ucont);
-__global__ void k_ib_bc_faces(Grid g, const double *nvert, const double *lu, const double *icsi,
-                              const double *jeta, const double *kzet, int immersed, int b0, int b1, int b2, int b3,
-                              double *ucont);
-__global__ void k_ib_bc_edges(Grid g, const double *uold, int b0, int b1, int b2, int b3, int b4, int b5,
-                              double *ucont);
+__global__ void k_ibm_gather(Grid g, const vfs_ibm_node *nodes, int n_nodes, const int *tri, const double *u_surf,
+                             const double *nvert, const double *ucat, const double *p, double *val);
+__global__ void k_ibm_scatter(Grid g, const vfs_ibm_node *nodes, int n_nodes, const double *val, double *ucat,
+                              double *p);
+__global__ void k_ibm_faces(Grid g, Box b, const double *nvert, const uint8_t *near, const double *u,
+                            const double *icsi, const double *jeta, const double *kzet, double f, int b0, int b1,
+                            int b2, int b3, int b4, int b5, double *ucont);
+__global__ void k_ib_bc_faces(Grid g, Box b, const double *nvert, const uint8_t *near, const double *lu,
+                              const double *icsi, const double *jeta, const double *kzet, int immersed, int b0, int b1,
+                              int b2, int b3, double *ucont);
+__global__ void k_ib_bc_edges(Grid g, int b0, int b1, int b2, int b3, int b4, int b5, double *ucont);
 
 }  // namespace vfs

@@ -472,14 +472,18 @@ struct vfs_poisson {
   float *gfeat = nullptr, *gtgt = nullptr, *gfc = nullptr, *gout = nullptr, *gof[2] = {nullptr, nullptr};
   int gsmooth = 2;  // binomial passes over the prolonged correction
   std::vector<IbmBody> ibm_bodies;  // IB node records per body (ibm.cu)
-  double *ibm_work = nullptr;        // 5 N words + the surface velocities (allocated on first use)
+  double *ibm_work = nullptr;        // new values of a body's nodes + the surface velocities (grown on demand)
   IbmScratch ibm_scratch;            // the surface search's buffers
   size_t ibm_work_len = 0;
   // residual of the iterate installed by the learned guess, handed to the
   // next solve (warm_start 2) so that it does not form it again
   double *rprev = nullptr, *rlearn = nullptr, *r0 = nullptr;
   float *prev32 = nullptr;
-  double *ucat = nullptr;  // Contra2Cart output staging (3 per DA point)
+  double *ucat = nullptr;  // Contra2Cart output staging (3 per DA point, host arrays only)
+  // what Contra2Cart takes from the grid (k_contra2cart_coef: 11 planes over
+  // the box), formed by its first call after the grid was set
+  double *c2c = nullptr;
+  bool c2c_valid = false;
   // level-set variant of the operator and projection (vfs_poisson_set_levelset)
   double *ls_rho = nullptr, *ls_level = nullptr;
   int ls_on = 0, ls_bc3 = 0, ls_bc4 = 0, ls_bc5 = 0;
@@ -638,6 +642,17 @@ int device_view(vfs_poisson *h, const double *src, double *stage, size_t count, 
   *out = stage;
   return upload(h, stage, src, count);
 }
+// an array that is read and written: device memory where it lies, host memory
+// through *stage (allocated on first use; the caller downloads it)
+int device_inout(vfs_poisson *h, double *a, double **stage, size_t count, double **out) {
+  if (is_device_ptr(a)) {
+    *out = a;
+    return VFS_OK;
+  }
+  if (!*stage) TRY(dalloc(h, stage, count));
+  *out = *stage;
+  return upload(h, *stage, a, count);
+}
 int download(vfs_poisson *h, double *dst, const double *src, size_t count) {
   CUDA_TRY(cudaMemcpyAsync(dst, src, count * sizeof(double),
                            is_device_ptr(dst) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, h->stream));
@@ -717,6 +732,23 @@ int face_coef(vfs_poisson *h, const Grid &g, MetricPtrs &m) {
   MetricPtrs src = m;
   src.gface = nullptr;
   LAUNCH(h, k_face_coef, da_grid(g), 128, g, src, m.gface);
+  return VFS_OK;
+}
+// Contra2Cart on device arrays: u read (periodic ghosts in their partners), v
+// updated in place with its periodic ghosts
+int contra2cart(vfs_poisson *h, const double *u, double *v, int zero_solid) {
+  const Grid &g = h->g;
+  const size_t n = h->box.n();
+  if (!h->c2c_valid) {
+    if (!h->c2c) TRY(dalloc(h, &h->c2c, 11 * n));
+    LAUNCH(h, k_contra2cart_coef, lin_grid(n), 256, g, h->box, h->met, h->c2c);
+    h->c2c_valid = true;
+  }
+  LAUNCH(h, k_contra2cart, lin_grid(n), 256, g, h->box, h->nvert, h->near, h->c2c, u, v, zero_solid);
+  if (const unsigned nb = shell_grid(g)) LAUNCH(h, k_periodic_cmpnts, nb, 256, g, v);
+  if (zero_solid)
+    LAUNCH(h, k_zero_rim, lin_grid(4 * ((size_t)g.my * g.mz + (size_t)g.mx * g.mz + (size_t)g.mx * g.my)), 256, g,
+           h->nvert, v);
   return VFS_OK;
 }
 void free_metrics(vfs_poisson *h, MetricPtrs &m) {
@@ -2341,6 +2373,7 @@ void vfs_poisson_destroy(vfs_poisson *h) {
 int vfs_poisson_set_grid(vfs_poisson *h, const double *coor, const double *const *fm) {
   if (!h || !coor) return fail(VFS_EINVAL, "null argument");
   h->hier_cmax = -1;  // new coordinates: the next mask builds the hierarchy afresh
+  h->c2c_valid = false;
   h->ibm_scratch.bbox_valid = false;  // and the next search bounds the new centres
   h->nvert_prev_valid = false;        // and the next mask fills every row
   const size_t N = h->g.n();
@@ -2559,15 +2592,12 @@ int vfs_poisson_contra2cart(vfs_poisson *h, const double *ucont, double *ucat, i
   if (!h || !ucont || !ucat) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before contra2cart");
   const size_t N = h->g.n();
-  if (!h->ucat) TRY(dalloc(h, &h->ucat, 3 * N));
-  TRY(upload(h, h->ucont, ucont, 3 * N));
-  TRY(upload(h, h->ucat, ucat, 3 * N));
-  LAUNCH(h, k_periodic_cmpnts, da_grid(h->g), 128, h->g, h->ucont, h->stage);
-  LAUNCH(h, k_contra2cart, dim3((h->g.mx - 2 + 127) / 128, h->g.my - 2, h->g.mz - 2), 128, h->g, h->nvert, h->met,
-         h->stage, h->ucat);
-  LAUNCH(h, k_periodic_cmpnts, da_grid(h->g), 128, h->g, h->ucat, h->stage);
-  if (zero_solid) LAUNCH(h, k_zero_solid, kRedBlocks, 256, h->g, h->nvert, h->stage);
-  TRY(download(h, ucat, h->stage, 3 * N));
+  const double *u = nullptr;
+  double *v = nullptr;
+  TRY(device_view(h, ucont, h->ucont, 3 * N, &u));
+  TRY(device_inout(h, ucat, &h->ucat, 3 * N, &v));
+  TRY(contra2cart(h, u, v, zero_solid));
+  if (v != ucat) TRY(download(h, ucat, v, 3 * N));
   return sync(h);
 }
 
@@ -2578,11 +2608,9 @@ int vfs_poisson_ibm_interpolate(vfs_poisson *h, int ibi, const double *u_surf, i
   if (ibi < 0 || ibi >= (int)h->ibm_bodies.size() || !h->ibm_bodies[ibi].nodes)
     return fail(VFS_ESTATE, "vfs_poisson_ibm_search_nodes must run for this body first");
   const IbmBody &B = h->ibm_bodies[ibi];
-  const size_t N = h->g.n();
-  if (!h->ucat) TRY(dalloc(h, &h->ucat, 3 * N));
-  // device work space: ucat (h->ucat) and ucont (h->ucont); the copies of
-  // the inputs as read, p and the surface velocities in ibm_work
-  const size_t need = 5 * N + (size_t)B.n_v * 3;
+  const size_t N = h->g.n(), n = h->box.n();
+  // work space: the nodes' new values and the surface velocities
+  const size_t need = 4 * (size_t)B.n_nodes + (size_t)B.n_v * 3;
   if (h->ibm_work_len < need) {
     if (h->ibm_work) dfree(h, h->ibm_work);
     h->ibm_work = nullptr;
@@ -2590,70 +2618,57 @@ int vfs_poisson_ibm_interpolate(vfs_poisson *h, int ibi, const double *u_surf, i
     TRY(dalloc(h, &h->ibm_work, need));
     h->ibm_work_len = need;
   }
-  double *lucat = h->ibm_work, *lpr = h->ibm_work + 3 * N, *pd = h->ibm_work + 4 * N, *us = nullptr;
-  TRY(upload(h, h->ucat, ucat, 3 * N));
-  TRY(upload(h, pd, p, N));
-  TRY(upload(h, h->ucont, ucont, 3 * N));
-  CUDA_TRY(cudaMemcpyAsync(lucat, h->ucat, 3 * N * 8, cudaMemcpyDeviceToDevice, h->stream));
-  CUDA_TRY(cudaMemcpyAsync(lpr, pd, N * 8, cudaMemcpyDeviceToDevice, h->stream));
+  double *ud = nullptr, *pd = nullptr, *cd = nullptr, *us = nullptr;
+  TRY(device_inout(h, ucat, &h->ucat, 3 * N, &ud));
+  TRY(device_inout(h, p, &h->p_da, N, &pd));
+  TRY(device_inout(h, ucont, &h->ucont, 3 * N, &cd));
   if (u_surf) {
     if (is_device_ptr(u_surf)) {
       us = const_cast<double *>(u_surf);
     } else {
-      us = h->ibm_work + 5 * N;
+      us = h->ibm_work + 4 * (size_t)B.n_nodes;
       CUDA_TRY(cudaMemcpyAsync(us, u_surf, (size_t)B.n_v * 3 * 8, cudaMemcpyHostToDevice, h->stream));
     }
   }
-  if (B.n_nodes > 0)
-    LAUNCH(h, k_ibm_apply, (B.n_nodes + 127) / 128, 128, h->g, B.nodes, B.n_nodes, B.tri, us, h->nvert, lucat, lpr,
-           h->ucat, pd);
-  // the new ucat with periodic ghosts (the local copy the flux loop reads)
-  LAUNCH(h, k_periodic_cmpnts, da_grid(h->g), 128, h->g, h->ucat, h->stage);
+  // every node's new values from the arrays as they were, then the writes
+  if (B.n_nodes > 0) {
+    LAUNCH(h, k_ibm_gather, (B.n_nodes + 127) / 128, 128, h->g, B.nodes, B.n_nodes, B.tri, us, h->nvert, ud, pd,
+           h->ibm_work);
+    LAUNCH(h, k_ibm_scatter, (B.n_nodes + 127) / 128, 128, h->g, B.nodes, B.n_nodes, h->ibm_work, ud, pd);
+  }
   int b[6] = {0, 0, 0, 0, 0, 0};
   if (bctype)
     for (int q = 0; q < 6; q++) b[q] = bctype[q];
-  LAUNCH(h, k_ibm_faces, dim3((h->g.mx - 2 + 127) / 128, h->g.my - 2, h->g.mz - 2), 128, h->g, h->nvert, h->stage,
-         h->met.icsi, h->met.jeta, h->met.kzet, immersed == 3 ? 0. : 1., b[0], b[1], b[2], b[3], b[4], b[5],
-         h->ucont);
+  LAUNCH(h, k_ibm_faces, lin_grid(n), 256, h->g, h->box, h->nvert, h->near, ud, h->met.icsi, h->met.jeta,
+         h->met.kzet, immersed == 3 ? 0. : 1., b[0], b[1], b[2], b[3], b[4], b[5], cd);
   // Contra2Cart with the solid zeroing
-  LAUNCH(h, k_periodic_cmpnts, da_grid(h->g), 128, h->g, h->ucont, h->stage);
-  LAUNCH(h, k_contra2cart, dim3((h->g.mx - 2 + 127) / 128, h->g.my - 2, h->g.mz - 2), 128, h->g, h->nvert, h->met,
-         h->stage, h->ucat);
-  LAUNCH(h, k_periodic_cmpnts, da_grid(h->g), 128, h->g, h->ucat, h->stage);
-  LAUNCH(h, k_zero_solid, kRedBlocks, 256, h->g, h->nvert, h->stage);
-  TRY(download(h, ucat, h->stage, 3 * N));
-  TRY(download(h, p, pd, N));
-  TRY(download(h, ucont, h->ucont, 3 * N));
+  TRY(contra2cart(h, cd, ud, 1));
+  if (ud != ucat) TRY(download(h, ucat, ud, 3 * N));
+  if (pd != p) TRY(download(h, p, pd, N));
+  if (cd != ucont) TRY(download(h, ucont, cd, 3 * N));
   return sync(h);
 }
 
 int vfs_poisson_ib_bc(vfs_poisson *h, int immersed, const int *bctype, double *ucat, double *ucont) {
   if (!h || !ucat || !ucont) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before IB_BC");
-  const size_t N = h->g.n();
-  if (!h->ucat) TRY(dalloc(h, &h->ucat, 3 * N));
-  TRY(upload(h, h->ucat, ucat, 3 * N));
-  TRY(upload(h, h->ucont, ucont, 3 * N));
+  const Grid &g = h->g;
+  const size_t N = g.n();
+  double *ud = nullptr, *cd = nullptr;
+  TRY(device_inout(h, ucat, &h->ucat, 3 * N, &ud));
+  TRY(device_inout(h, ucont, &h->ucont, 3 * N, &cd));
   int b[6] = {0, 0, 0, 0, 0, 0};
   if (bctype)
     for (int q = 0; q < 6; q++) b[q] = bctype[q];
   // periodic ghosts of ucat from their partners (written back: the
   // reference writes them into lUcat)
-  LAUNCH(h, k_periodic_cmpnts, da_grid(h->g), 128, h->g, h->ucat, h->stage);
-  LAUNCH(h, k_ib_bc_faces, dim3((h->g.mx - 2 + 127) / 128, h->g.my - 2, h->g.mz - 2), 128, h->g, h->nvert,
-         h->stage, h->met.icsi, h->met.jeta, h->met.kzet, immersed, b[0], b[1], b[2], b[3], h->ucont);
-  if (h->ibm_work_len < 3 * N) {
-    if (h->ibm_work) dfree(h, h->ibm_work);
-    h->ibm_work = nullptr;
-    h->ibm_work_len = 0;
-    TRY(dalloc(h, &h->ibm_work, 3 * N));
-    h->ibm_work_len = 3 * N;
-  }
-  double *uold = h->ibm_work;
-  CUDA_TRY(cudaMemcpyAsync(uold, h->ucont, 3 * N * 8, cudaMemcpyDeviceToDevice, h->stream));
-  LAUNCH(h, k_ib_bc_edges, da_grid(h->g), 128, h->g, uold, b[0], b[1], b[2], b[3], b[4], b[5], h->ucont);
-  TRY(download(h, ucat, h->stage, 3 * N));
-  TRY(download(h, ucont, h->ucont, 3 * N));
+  if (const unsigned nb = shell_grid(g)) LAUNCH(h, k_periodic_cmpnts, nb, 256, g, ud);
+  LAUNCH(h, k_ib_bc_faces, lin_grid(h->box.n()), 256, g, h->box, h->nvert, h->near, ud, h->met.icsi, h->met.jeta,
+         h->met.kzet, immersed, b[0], b[1], b[2], b[3], cd);
+  LAUNCH(h, k_ib_bc_edges, lin_grid((size_t)g.my * g.mz + (size_t)g.mx * g.mz + (size_t)g.mx * g.my), 256, g, b[0],
+         b[1], b[2], b[3], b[4], b[5], cd);
+  if (ud != ucat) TRY(download(h, ucat, ud, 3 * N));
+  if (cd != ucont) TRY(download(h, ucont, cd, 3 * N));
   return sync(h);
 }
 
