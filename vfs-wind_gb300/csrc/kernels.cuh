@@ -36,10 +36,10 @@ __global__ void k_face_coef(Grid g, MetricPtrs m, double *gface);
 __global__ void k_metrics_mirror(Grid g, MetricPtrs m, int dir);
 __global__ void k_metrics_periodic(Grid g, MetricPtrs m, int faces);
 __global__ void k_metrics_face(Grid g, MetricPtrs m, int dir);
-__global__ void k_count_dofs(Grid g, Box b, const double *nvert, int *block_count);
+__global__ void k_count_dofs(size_t n, const uint8_t *rowtype, int *block_count);
 __global__ void k_scan_blocks(int *block_count, int nblocks, int *total);
-__global__ void k_number_dofs(Grid g, Box b, const double *nvert, const int *block_off, int *gid_box);
-__global__ void k_gid_da(Grid g, Box b, const int *gid_box, int *gid_da);
+__global__ void k_number_dofs(Grid g, Box b, const uint8_t *rowtype, const int *block_off, int *gid_da);
+__global__ void k_gid_ghosts(Grid g, int *gid_da);
 __global__ void k_rhs2(Grid g, Box b, const double *nvert, const uint8_t *rowtype, const double *ucont,
                        const double *aj, double dt, double st, double coeff, int poisson, double *rhs, double *partial);
 __global__ void k_rhs2_shift(Grid g, Box b, const double *nvert, const double *aj, const double *sums, int poisson,
@@ -67,9 +67,12 @@ __global__ void k_assemble_rows(Grid g, Box b, const double *nvert, MetricPtrs m
                                 double *A, uint8_t *rowtype, LevelSet ls, const int *rows, const int *nrows);
 __global__ void k_assemble_fine_rows(Grid g, Box b, const double *nvert, MetricPtrs m, double *A0, uint8_t *rowtype0,
                                      double *A1, uint8_t *rowtype1, LevelSet ls, const int *rows, const int *nrows);
-__global__ void k_mask_changed(size_t N, const double *a, const double *b, uint8_t *chg);
-__global__ void k_dilate_axis(Grid g, int axis, int R, const uint8_t *src, uint8_t *dst);
-__global__ void k_list_rows(Grid g, Box b, const uint8_t *flag, int *rows, int *nrows, uint8_t *colflag);
+__global__ void k_changed_bits(Grid g, int wpr, const double *src, double *nvert, const double *prev, uint32_t *bits);
+__global__ void k_list_rows(Grid g, Box b, int wpr, const uint32_t *bits, int *rows, int *nrows, uint8_t *colflag);
+__global__ void k_level_masks_rows(Grid g, Box b, const double *nvert, uint8_t *blank, double *w64, float *w32,
+                                   const int *rows, const int *nrows);
+__global__ void k_fluid_rows(Grid g, Box b, const double *nvert, uint8_t *fluid, const int *rows, const int *nrows);
+__global__ void k_fluid_sums(size_t n, const uint8_t *fluid, const double *aj_box, double *partial);
 __global__ void k_projection_coef(Grid g, Box b, MetricPtrs m, double *pc);
 __global__ void k_level_masks(Grid g, Box b, const double *nvert, uint8_t *blank, double *w64, float *w32);
 __global__ void k_rhs(Grid g, Box b, const uint8_t *fluid, const double *ucont, double dt, double st, double coeff,
@@ -120,7 +123,6 @@ __global__ void k_prolong_f64(Box bf, Box bc, int cx, int cy, int cz, const doub
 // solve.cu (hot loop kernels)
 #define TYPED_DECL(T, S)                                                                                 \
   __global__ void k_residual_##S(Box b, const T *A, const T *x, const T *rhs, T *r, int color);          \
-  __global__ void k_line_lu_##S(Box b, const double *A64, T *inv, T *cp, const uint8_t *colflag);        \
   __global__ void k_line_sweep_##S(Box b, const T *A, const T *inv, const T *cp, const T *x, const T *rhs, \
                                    T *xo, T omega, int zero_guess);                                      \
   __global__ void k_line_tri_##S(Box b, const T *r, const T *Asp, const T *inv, const T *cp, T *x, T omega,  \
@@ -132,6 +134,8 @@ TYPED_DECL(float, f32)
 TYPED_DECL(double, f64)
 #undef TYPED_DECL
 
+__global__ void k_line_lu(Box b, const double *A64, double *inv64, double *cp64, float *inv32, float *cp32,
+                          const uint8_t *colflag);
 __global__ void k_pack16(size_t n, const double *A, __half2 *C, float *D);
 __global__ void k_pack16_rows(Box b, const double *A, __half2 *C, float *D, float *A32, const int *rows,
                               const int *nrows);

@@ -48,10 +48,21 @@ constexpr int kMaxLevels = 24;
 constexpr int kRedBlocks = 1216;  // 8 x 152 SMs, fixed for deterministic reductions
 
 // device helper kernels that only the host orchestration needs
-__global__ void k_row_scale(size_t n, const uint8_t *rowtype, const double *aj_box, double *scale) {
+__device__ __forceinline__ void row_scale(const uint8_t *rowtype, const double *aj_box, double *scale, float *scale32,
+                                          size_t c) {
+  const double v = rowtype[c] == 1 ? aj_box[c] : (rowtype[c] == 2 ? 1.0 : 0.0);
+  scale[c] = v;
+  scale32[c] = (float)v;
+}
+__global__ void k_row_scale(size_t n, const uint8_t *rowtype, const double *aj_box, double *scale, float *scale32) {
   size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  scale[c] = rowtype[c] == 1 ? aj_box[c] : (rowtype[c] == 2 ? 1.0 : 0.0);
+  if (c < n) row_scale(rowtype, aj_box, scale, scale32, c);
+}
+__global__ void k_row_scale_rows(const uint8_t *rowtype, const double *aj_box, double *scale, float *scale32,
+                                 const int *__restrict__ rows, const int *__restrict__ nrows) {
+  const int nr = *nrows;
+  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nr; w += gridDim.x * blockDim.x)
+    row_scale(rowtype, aj_box, scale, scale32, rows[w]);
 }
 // one operator plane from the parity-split row layout to the natural one
 __global__ void k_unsplit_plane(Box b, const float *src, float *dst) {
@@ -453,7 +464,7 @@ struct vfs_poisson {
   float *scale32 = nullptr;  // the row scale in FP32 (the FP32 V-cycle's right-hand side)
   uint8_t *rowtype0 = nullptr, *fluid = nullptr;
   uint8_t *near = nullptr;  // cells with a non-zero nvert within one point (k_near_body)
-  int *gid_box = nullptr, *gid_da = nullptr, *blk = nullptr, *total = nullptr;
+  int *gid_da = nullptr, *blk = nullptr, *total = nullptr;
   int ndof = 0;
   double *b = nullptr, *x = nullptr, *r = nullptr;
   // Krylov basis
@@ -503,7 +514,8 @@ struct vfs_poisson {
   // inc_rows: the level-0 refill in progress uses that list
   bool inc_enable = true, nvert_prev_valid = false, inc_rows = false;
   double *nvert_prev = nullptr;
-  uint8_t *chg_a = nullptr, *chg_b = nullptr, *colflag = nullptr;
+  uint32_t *chg = nullptr;  // changed points, bits in words of 32 along i
+  uint8_t *colflag = nullptr;
   int *rows = nullptr, *nrows = nullptr;
   // history of the last hist_cnt (at most hist_cap) converged solutions for
   // the initial guess, held as the newest one X_n (the FGMRES iterate before
@@ -996,12 +1008,16 @@ int build_level_operator(vfs_poisson *h, Level &l, bool assembled = false) {
            (const int *)h->rows, (const int *)h->nrows);
   else if (!assembled)
     LAUNCH(h, k_assemble, box_grid(l.b), 128, l.g, l.b, l.nvert, l.met, 1, 0, 1, l.A64, l.rowtype, level_set(h, l));
-  LAUNCH(h, k_level_masks, lin_grid(n), 256, l.g, l.b, l.nvert, l.blank, l.w64, l.w32);
+  if (h->inc_rows)
+    LAUNCH(h, k_level_masks_rows, kRedBlocks, 256, l.g, l.b, (const double *)l.nvert, l.blank, l.w64, l.w32,
+           (const int *)h->rows, (const int *)h->nrows);
+  else
+    LAUNCH(h, k_level_masks, lin_grid(n), 256, l.g, l.b, l.nvert, l.blank, l.w64, l.w32);
   // a level of an incremental refill: only the listed rows' copies and the
   // j-columns that hold one are formed again
   const uint8_t *cols = h->inc_rows ? h->colflag : nullptr;
-  LAUNCH(h, k_line_lu_f64, dim3((l.b.nx + 127) / 128, l.b.nz), 128, l.b, l.A64, l.inv64, l.cp64, cols);
-  LAUNCH(h, k_line_lu_f32, dim3((l.b.nx + 127) / 128, l.b.nz), 128, l.b, l.A64, l.inv32, l.cp32, cols);
+  LAUNCH(h, k_line_lu, dim3((l.b.nx + 127) / 128, l.b.nz), 128, l.b, (const double *)l.A64, l.inv64, l.cp64, l.inv32,
+         l.cp32, cols);
   if (cols) {
     LAUNCH(h, k_pack16_rows, kRedBlocks, 256, l.b, (const double *)l.A64, l.C16, l.D32, l.A32, (const int *)h->rows,
            (const int *)h->nrows);
@@ -1009,6 +1025,18 @@ int build_level_operator(vfs_poisson *h, Level &l, bool assembled = false) {
     LAUNCH(h, k_cast_planes_f32, kRedBlocks, 256, l.A64, l.A32, n * NSLOT);
     LAUNCH(h, k_pack16, kRedBlocks, 256, n, l.A64, l.C16, l.D32);
   }
+  return VFS_OK;
+}
+
+// The rows to refill after a new mask (src, copied to nvert on the way where
+// they differ) in place of the mask prev, with their j-columns.
+int list_rows(vfs_poisson *h, const Grid &g, const Box &b, const double *src, double *nvert, const double *prev) {
+  const int wpr = (g.mx + 31) / 32;
+  LAUNCH(h, k_changed_bits, kRedBlocks, 256, g, wpr, src, nvert, prev, h->chg);
+  CUDA_TRY(cudaMemsetAsync(h->nrows, 0, sizeof(int), h->stream));
+  CUDA_TRY(cudaMemsetAsync(h->colflag, 0, (size_t)b.nx * b.nz, h->stream));
+  LAUNCH(h, k_list_rows, lin_grid((size_t)b.ny * b.nz * wpr), 256, g, b, wpr, (const uint32_t *)h->chg, h->rows,
+         h->nrows, h->colflag);
   return VFS_OK;
 }
 
@@ -1046,14 +1074,7 @@ int refresh_hierarchy(vfs_poisson *h) {
       // the rows of this level within two points of a changed restricted
       // mask value (the list buffers of the finest level, consumed by its
       // launches above, are reused in stream order)
-      LAUNCH(h, k_mask_changed, kRedBlocks, 256, l.g.n(), (const double *)l.nvert, (const double *)l.nvert_prev,
-             h->chg_a);
-      LAUNCH(h, k_dilate_axis, da_grid(l.g), 128, l.g, 0, 2, (const uint8_t *)h->chg_a, h->chg_b);
-      LAUNCH(h, k_dilate_axis, da_grid(l.g), 128, l.g, 1, 2, (const uint8_t *)h->chg_b, h->chg_a);
-      LAUNCH(h, k_dilate_axis, da_grid(l.g), 128, l.g, 2, 2, (const uint8_t *)h->chg_a, h->chg_b);
-      CUDA_TRY(cudaMemsetAsync(h->nrows, 0, sizeof(int), h->stream));
-      CUDA_TRY(cudaMemsetAsync(h->colflag, 0, (size_t)l.b.nx * l.b.nz, h->stream));
-      LAUNCH(h, k_list_rows, kRedBlocks, 256, l.g, l.b, (const uint8_t *)h->chg_b, h->rows, h->nrows, h->colflag);
+      TRY(list_rows(h, l.g, l.b, l.nvert, l.nvert, l.nvert_prev));
     }
     TRY(build_level_operator(h, l, li == 0));
   }
@@ -2318,7 +2339,7 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
       (rc = dalloc(h, &h->scale, n)) || (rc = dalloc(h, &h->scale32, n)) || (rc = dalloc(h, &h->pc, 12 * n)) ||
       (rc = dalloc(h, &h->aj_box, n)) ||
       (rc = dalloc(h, &h->rowtype0, n)) || (rc = dalloc(h, &h->fluid, n)) ||
-      (rc = dalloc(h, &h->near, n)) || (rc = dalloc(h, &h->fsum, 2)) || (rc = dalloc(h, &h->gid_box, n)) ||
+      (rc = dalloc(h, &h->near, n)) || (rc = dalloc(h, &h->fsum, 2)) ||
       (rc = dalloc(h, &h->gid_da, N)) || (rc = dalloc(h, &h->b, n)) || (rc = dalloc(h, &h->x, n)) ||
       (rc = dalloc(h, &h->r, n)) || (rc = dalloc(h, &h->red, 512)) || (rc = dalloc(h, &h->total, 1)))
     return bail(rc);
@@ -2332,6 +2353,7 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
   if ((rc = dalloc(h, &h->partial, h->partial_len))) return bail(rc);
   if (cudaMallocHost(&h->hbuf, 1024 * 8) != cudaSuccess) { cudaGetLastError(); return bail(fail(VFS_ENOMEM, "pinned alloc")); }
   cudaMemsetAsync(h->phi_da, 0, N * 8, h->stream);
+  cudaMemsetAsync(h->gid_da, 0xff, N * 4, h->stream);  // -1 on the boundary layer for good
   cudaMemsetAsync(h->x, 0, n * 8, h->stream);
   if ((rc = sync(h))) return bail(rc);
   *out = h;
@@ -2410,53 +2432,53 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
   h->inc_rows = false;
   if (h->inc_enable && !h->nvert_prev) {
     TRY(dalloc(h, &h->nvert_prev, N));
-    TRY(dalloc(h, &h->chg_a, N));
-    TRY(dalloc(h, &h->chg_b, N));
+    TRY(dalloc(h, &h->chg, (size_t)((h->g.mx + 31) / 32) * h->g.my * h->g.mz));
     TRY(dalloc(h, &h->colflag, (size_t)h->box.nx * h->box.nz));
     TRY(dalloc(h, &h->rows, n));
     TRY(dalloc(h, &h->nrows, 1));
   }
   if (incremental) std::swap(h->nvert, h->nvert_prev);
-  TRY(upload(h, h->nvert, nvert, N));
-  // setup_lidx2: dof numbering in k-j-i order
-  const int nblk = (int)((n + 1023) / 1024);
-  LAUNCH(h, k_count_dofs, nblk, 1024, h->g, h->box, h->nvert, h->blk);
-  LAUNCH(h, k_scan_blocks, 1, 1024, h->blk, nblk, h->total);
-  LAUNCH(h, k_number_dofs, nblk, 1024, h->g, h->box, h->nvert, h->blk, h->gid_box);
-  LAUNCH(h, k_gid_da, da_grid(h->g), 128, h->g, h->box, h->gid_box, h->gid_da);
-  // the fluid mask, aj at the box cells and the mask's sums (aj and count
-  // over the fluid), which every right-hand side and mean removal uses
-  LAUNCH(h, k_fluid_mask, kRedBlocks, 256, h->g, h->box, h->nvert, h->met.aj, h->fluid, h->aj_box, h->partial);
-  LAUNCH(h, k_reduce_rows, 2, 1024, h->partial, kRedBlocks, 2, h->fsum);
-  // PoissonLHSNew: unscaled operator with the reference's insertion filter
+  const int *rows = h->rows, *nrows = h->nrows;
   LevelSet fls;
   if (h->ls_on) {
     fls.rho = h->ls_rho; fls.level = h->ls_level; fls.on = 1;
     fls.bc3 = h->ls_bc3; fls.bc4 = h->ls_bc4; fls.bc5 = h->ls_bc5;
   }
-  if (!incremental)
+  // the operator (PoissonLHSNew, unscaled with the reference's insertion
+  // filter; beside it the hierarchy's), the fluid mask with its sums (aj and
+  // count over the fluid, which every right-hand side and mean removal uses),
+  // aj at the box cells, the cells near a body and the row scale
+  if (incremental) {
+    const bool dev = is_device_ptr(nvert);
+    if (!dev) TRY(upload(h, h->nvert, nvert, N));
+    TRY(list_rows(h, h->g, h->box, dev ? nvert : h->nvert, h->nvert, h->nvert_prev));
+    LAUNCH(h, k_assemble_fine_rows, kRedBlocks, 256, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
+           h->L[0].A64, h->L[0].rowtype, fls, rows, nrows);
+    LAUNCH(h, k_near_body_rows, kRedBlocks, 256, h->g, h->box, (const double *)h->nvert, h->near, rows, nrows);
+    LAUNCH(h, k_fluid_rows, kRedBlocks, 256, h->g, h->box, (const double *)h->nvert, h->fluid, rows, nrows);
+    LAUNCH(h, k_fluid_sums, kRedBlocks, 256, n, (const uint8_t *)h->fluid, (const double *)h->aj_box, h->partial);
+    LAUNCH(h, k_row_scale_rows, kRedBlocks, 256, (const uint8_t *)h->rowtype0, (const double *)h->aj_box, h->scale,
+           h->scale32, rows, nrows);
+    h->inc_rows = true;
+  } else {
+    TRY(upload(h, h->nvert, nvert, N));
+    LAUNCH(h, k_fluid_mask, kRedBlocks, 256, h->g, h->box, h->nvert, h->met.aj, h->fluid, h->aj_box, h->partial);
     LAUNCH(h, k_near_body, dim3((h->box.nx + 125) / 126, h->box.ny, h->box.nz), 128, h->g, h->box,
            (const double *)h->nvert, h->near);
-  if (incremental) {
-    LAUNCH(h, k_mask_changed, kRedBlocks, 256, N, (const double *)h->nvert, (const double *)h->nvert_prev, h->chg_a);
-    LAUNCH(h, k_dilate_axis, da_grid(h->g), 128, h->g, 0, 2, (const uint8_t *)h->chg_a, h->chg_b);
-    LAUNCH(h, k_dilate_axis, da_grid(h->g), 128, h->g, 1, 2, (const uint8_t *)h->chg_b, h->chg_a);
-    LAUNCH(h, k_dilate_axis, da_grid(h->g), 128, h->g, 2, 2, (const uint8_t *)h->chg_a, h->chg_b);
-    CUDA_TRY(cudaMemsetAsync(h->nrows, 0, sizeof(int), h->stream));
-    CUDA_TRY(cudaMemsetAsync(h->colflag, 0, (size_t)h->box.nx * h->box.nz, h->stream));
-    LAUNCH(h, k_list_rows, kRedBlocks, 256, h->g, h->box, (const uint8_t *)h->chg_b, h->rows, h->nrows, h->colflag);
-    LAUNCH(h, k_assemble_fine_rows, kRedBlocks, 256, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
-           h->L[0].A64, h->L[0].rowtype, fls, (const int *)h->rows, (const int *)h->nrows);
-    LAUNCH(h, k_near_body_rows, kRedBlocks, 256, h->g, h->box, (const double *)h->nvert, h->near,
-           (const int *)h->rows, (const int *)h->nrows);
-    h->inc_rows = true;
-  } else if (refills) {  // both fine operators from one evaluation of each row
-    LAUNCH(h, k_assemble_fine, box_grid(h->box), 128, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
-           h->L[0].A64, h->L[0].rowtype, fls);
-  } else
-    LAUNCH(h, k_assemble, box_grid(h->box), 128, h->g, h->box, h->nvert, h->met, 0, 1, 0, h->A0, h->rowtype0, fls);
-  LAUNCH(h, k_row_scale, lin_grid(n), 256, n, h->rowtype0, h->aj_box, h->scale);
-  LAUNCH(h, k_cast_planes_f32, kRedBlocks, 256, h->scale, h->scale32, n);
+    if (refills)  // both fine operators from one evaluation of each row
+      LAUNCH(h, k_assemble_fine, box_grid(h->box), 128, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
+             h->L[0].A64, h->L[0].rowtype, fls);
+    else
+      LAUNCH(h, k_assemble, box_grid(h->box), 128, h->g, h->box, h->nvert, h->met, 0, 1, 0, h->A0, h->rowtype0, fls);
+    LAUNCH(h, k_row_scale, lin_grid(n), 256, n, h->rowtype0, h->aj_box, h->scale, h->scale32);
+  }
+  LAUNCH(h, k_reduce_rows, 2, 1024, h->partial, kRedBlocks, 2, h->fsum);
+  // setup_lidx2: dof numbering in k-j-i order
+  const int nblk = (int)((n + 1023) / 1024);
+  LAUNCH(h, k_count_dofs, nblk, 1024, n, (const uint8_t *)h->rowtype0, h->blk);
+  LAUNCH(h, k_scan_blocks, 1, 1024, h->blk, nblk, h->total);
+  LAUNCH(h, k_number_dofs, nblk, 1024, h->g, h->box, (const uint8_t *)h->rowtype0, (const int *)h->blk, h->gid_da);
+  if (const unsigned nb = shell_grid(h->g)) LAUNCH(h, k_gid_ghosts, nb, 256, h->g, h->gid_da);
   int tot = 0;
   CUDA_TRY(cudaMemcpyAsync(&tot, h->total, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   TRY(sync(h));

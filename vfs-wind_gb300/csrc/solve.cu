@@ -190,30 +190,45 @@ __global__ void __launch_bounds__(256) k_residual64(Box b, const double *__restr
 }
 
 // LU factors of the tridiagonal j-line part (S, CP, N slots) of a level
-// operator, computed in FP64 and stored in T.  Rows without a dof get an
-// identity line entry.  The j-periodic wrap couplings stay off the line.
-template <typename T>
-__device__ __forceinline__ void line_lu_body(Box b, const double *__restrict__ A, T *inv, T *cp,
-                                             const uint8_t *__restrict__ colflag) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+// operator, computed in FP64 and stored in both precisions (one recurrence
+// for the two).  Rows without a dof get an identity line entry.  The
+// j-periodic wrap couplings stay off the line.  A column is a chain of ny
+// divisions; the loads of 8 rows go ahead of it (with each row's loads in the
+// chain, and once per precision, 192-row columns took 0.39 ms; now 0.10, the
+// divisions themselves).
+__global__ void __launch_bounds__(128) k_line_lu(Box b, const double *__restrict__ A, double *__restrict__ inv64,
+                                                 double *__restrict__ cp64, float *__restrict__ inv32,
+                                                 float *__restrict__ cp32, const uint8_t *__restrict__ colflag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
   if (i >= b.nx) return;
   if (colflag && !colflag[(size_t)k * b.nx + i]) return;  // (a column left as it was)
   const size_t n = b.n();
   double cprev = 0.;
-  const int p = split_pos(i, b.nx);
-  for (int j = 0; j < b.ny; j++) {
-    size_t c = b.at(p, j, k);  // split position of cell i
-    double d = A[CP * n + c], a = 0., cc = 0.;
-    if (d != 0.) {
-      a = j > 0 ? A[SP * n + c] : 0.;
-      cc = j < b.ny - 1 ? A[NP * n + c] : 0.;
-    } else {
-      d = 1.;
+  const size_t col = b.at(split_pos(i, b.nx), 0, k);  // split position of cell i
+  for (int j0 = 0; j0 < b.ny; j0 += 8) {
+    double d[8], a[8], c[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const size_t at = col + (size_t)min(j0 + e, b.ny - 1) * b.nx;
+      d[e] = A[CP * n + at];
+      a[e] = A[SP * n + at];
+      c[e] = A[NP * n + at];
     }
-    double iv = 1.0 / (d - a * cprev);
-    inv[c] = (T)iv;
-    cp[c] = (T)(cc * iv);
-    cprev = cc * iv;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const int j = j0 + e;
+      if (j < b.ny) {
+        const bool row = d[e] != 0.;
+        const double dd = row ? d[e] : 1., aa = row && j > 0 ? a[e] : 0., cc = row && j < b.ny - 1 ? c[e] : 0.;
+        const double iv = 1.0 / (dd - aa * cprev);
+        const size_t at = col + (size_t)j * b.nx;
+        cprev = cc * iv;
+        inv64[at] = iv;
+        cp64[at] = cprev;
+        inv32[at] = (float)iv;
+        cp32[at] = (float)cprev;
+      }
+    }
   }
 }
 
@@ -1170,9 +1185,6 @@ void launch_hist_push(cudaStream_t st, int blocks, size_t n, const double *x, co
   __global__ void __launch_bounds__(256) k_residual_##S(Box b, const T *A, const T *x, const T *rhs, T *r,  \
                                                         int color) {                                       \
     residual_body<T>(b, A, x, rhs, r, color);                                                              \
-  }                                                                                                        \
-  __global__ void k_line_lu_##S(Box b, const double *A64, T *inv, T *cp, const uint8_t *colflag) {            \
-    line_lu_body<T>(b, A64, inv, cp, colflag);                                                            \
   }                                                                                                        \
   __global__ void __launch_bounds__(768, 1) k_line_sweep_##S(Box b, const T *A, const T *inv, const T *cp,      \
                                                            const T *x, const T *rhs, T *xo, T omega, int zg) { \
