@@ -59,22 +59,49 @@ unsigned glibc_rand_first(unsigned seed) {
 
 struct HashBox {
   double xmin, ymin, zmin, xmax, ymax, zmax, dcx, dcy, dcz;
+  // for the FP32 tests: the hash cells' sizes and reciprocals, the rays' end
+  // height over zmin and the sum of the box's extents
+  float fcx, fcy, fcz, rcx, rcy, rcz, fz, L;
 };
+
+// x > 0 without an FP64 comparison
+__device__ __forceinline__ bool positive(double x) {
+  const long long v = __double_as_longlong(x);
+  return v > 0 && v <= 0x7ff0000000000000ll;
+}
+// floor(t / d) from FP32 where its error (below 40 * 2^-22) cannot matter
+__device__ __forceinline__ int hash_cell(double t, double d, float r) {
+  const float q = (float)t * r, k = floorf(q), f = q - k;
+  return f > 1e-4f && f < 0.9999f ? (int)k : (int)floor(t / d);
+}
 
 // One cell centre: 4 if a ray from it crosses the surface an odd number of
 // times, 0 if even, -1 if every ray met a singular (double) intersection or
 // too many intersections.
-__device__ int point_cell(const double p[3], int ip, int jp, int kp, const HashBox &H, const int *col_start,
-                          const int *col_tri, const int *col_kmax, const double *tv, const double *nf,
-                          const double *s_tab) {
+//
+// Nearly all triangles of a column are missed by far, and an FP64 test of
+// some 45 instructions holds a quarter of the SM for 64 cycles each: a test in
+// FP32 on coordinates relative to the box drops the triangles that the FP64
+// test is certain to drop.  With unit roundoff u = 2^-24, coordinates of at
+// most L and one-norms D, E1, E2 and T of the ray, the edges and the vertex
+// offset, inputs are off by at most 3 u L, and the triple products by at most
+// 24 u times the product of their norms (with L added to T): the margins are
+// 64 u.  A triangle whose det might be 0 within its margin is kept.  tf: v0,
+// e1, e2, |e1|, |e2| per triangle.  A tower over 840 k cells: 674 -> 380 us, a
+// rod over 48 k cells: 75 -> 58 us, the longest column's chain of loads.
+__device__ int point_cell(const double p[3], const double rel[3], int ip, int jp, int kp, const HashBox &H,
+                          const int *col_start, const int *col_tri, const int *col_kmax, const double *tv,
+                          const double *nf, const double *s_tab, const float4 *tf) {
   const int col = jp * kHash + ip;
   const int e0 = col_start[col], e1 = col_start[col + 1];
+  const float px = (float)rel[0], py = (float)rel[1], pz = (float)rel[2];
   for (int tries = 1; tries <= kMaxTries; tries++) {
-    const double xpc = H.dcx * (ip + 0.5) + H.xmin, ypc = H.dcy * (jp + 0.5) + H.ymin;
     const double s = s_tab[tries];
-    double dir[3] = {xpc + s * H.dcx - p[0], ypc + s * H.dcy - p[1], H.zmax + 0.2 - p[2]};
-    const double nrm = sqrt(dir[0] * dir[0] + dir[1] * dir[1] + dir[2] * dir[2]);
-    dir[0] /= nrm; dir[1] /= nrm; dir[2] /= nrm;
+    const float fs = (float)s;
+    const float dx = H.fcx * ((float)ip + 0.5f + fs) - px, dy = H.fcy * ((float)jp + 0.5f + fs) - py, dz = H.fz - pz;
+    const float mD = 4e-6f * (fabsf(dx) + fabsf(dy) + fabsf(dz));
+    bool aimed = false;
+    double dir[3] = {0., 0., 0.};
     double dt[kMaxHits];
     int dn[kMaxHits];
     int nintp = 0;
@@ -82,6 +109,32 @@ __device__ int point_cell(const double p[3], int ip, int jp, int kp, const HashB
     for (int q = e0; q < e1 && !singular; q++) {
       if (col_kmax[q] - 1 < kp) break;  // list sorted by top hash cell, descending
       const int e = col_tri[q];
+      {
+        const float4 A = tf[3 * e], B = tf[3 * e + 1], C = tf[3 * e + 2];
+        const float ax = A.w, ay = B.x, az = B.y, bx = B.z, by = B.w, bz = C.x, n1 = C.y, n2 = C.z;
+        const float qx = dy * bz - dz * by, qy = dz * bx - dx * bz, qz = dx * by - dy * bx;
+        const float det = ax * qx + ay * qy + az * qz, ad = fabsf(det), md = mD * n1 * n2;
+        if (ad > md) {
+          const float sg = det < 0.f ? -1.f : 1.f;
+          const float tx = px - A.x, ty = py - A.y, tz = pz - A.z;
+          const float T = fabsf(tx) + fabsf(ty) + fabsf(tz) + H.L;
+          const float un = (tx * qx + ty * qy + tz * qz) * sg, mu = mD * n2 * T;
+          if (un < -mu || un > ad + mu + md) continue;
+          const float rx = ty * az - tz * ay, ry = tz * ax - tx * az, rz = tx * ay - ty * ax;
+          const float wn = (dx * rx + dy * ry + dz * rz) * sg, mw = mD * n1 * T;
+          if (wn < -mw || un + wn > ad + mu + mw + md) continue;
+          if ((bx * rx + by * ry + bz * rz) * sg < -4e-6f * n1 * n2 * T) continue;
+        }
+      }
+      if (!aimed) {
+        aimed = true;
+        const double xpc = H.dcx * (ip + 0.5) + H.xmin, ypc = H.dcy * (jp + 0.5) + H.ymin;
+        dir[0] = xpc + s * H.dcx - p[0];
+        dir[1] = ypc + s * H.dcy - p[1];
+        dir[2] = H.zmax + 0.2 - p[2];
+        const double nrm = sqrt(dir[0] * dir[0] + dir[1] * dir[1] + dir[2] * dir[2]);
+        dir[0] /= nrm; dir[1] /= nrm; dir[2] /= nrm;
+      }
       const double *v = &tv[(size_t)e * 9];
       // intsect_triangle, compgeom.c:25-60
       const double EPS = 0.00000001;
@@ -117,45 +170,111 @@ __device__ int point_cell(const double p[3], int ip, int jp, int kp, const HashB
   return -1;
 }
 
-// Classification of one body (ibm_search_advanced, ibm.c:92-325) as a
-// copying pass over every DA point: boundary points take src unchanged,
-// interior points whose centre lies in the body's hash box the larger of
-// their value and the ray-parity test (4 inside), body 0 first clearing
-// every value below 5 (src may be dst: each point reads and writes only
-// itself).
-__global__ void k_ibm_classify_from(Grid g, const double *__restrict__ cent, int ibi, HashBox H,
-                                    const int *__restrict__ col_start, const int *__restrict__ col_tri,
-                                    const int *__restrict__ col_kmax, const double *__restrict__ tv,
-                                    const double *__restrict__ nf, const double *__restrict__ s_tab, const double *src,
-                                    double *dst, uint8_t *is4, int *failed, int3 lo, int3 hi) {
-  const int i = lo.x + blockIdx.x * blockDim.x + threadIdx.x, j = lo.y + blockIdx.y, k = lo.z + blockIdx.z;
-  if (i >= hi.x) return;
+// The device copy of one body's surface.
+struct Surface {
+  HashBox H;
+  const int *col_start, *col_tri, *col_kmax;
+  const double *tv, *nf, *s_tab;
+  const float4 *tf;
+};
+
+// Classification of one body (ibm_search_advanced, ibm.c:92-325) at DA point
+// t of value nv: boundary points as they are, interior points whose centre
+// lies in the body's hash box the larger of their value and the ray-parity
+// test (4 inside); first: body 0 clears every value below 5 before.
+__device__ __forceinline__ double classify_point(const Grid &g, const double *__restrict__ cent, bool first,
+                                                 const Surface &S, int i, int j, int k, size_t t, double nv,
+                                                 int *failed) {
+  if (i < 1 || i >= g.mx - 1 || j < 1 || j >= g.my - 1 || k < 1 || k >= g.mz - 1) return nv;
+  const HashBox &H = S.H;
+  if (first && nv < 5.) nv = 0;
+  const double p[3] = {cent[t * 3], cent[t * 3 + 1], cent[t * 3 + 2]};
+  // (a difference has its exact sign)
+  const double rel[3] = {p[0] - H.xmin, p[1] - H.ymin, p[2] - H.zmin};
+  if (positive(rel[0]) && positive(H.xmax - p[0]) && positive(rel[1]) && positive(H.ymax - p[1]) &&
+      positive(rel[2]) && positive(H.zmax - p[2])) {
+    const int ic = hash_cell(rel[0], H.dcx, H.rcx), jc = hash_cell(rel[1], H.dcy, H.rcy),
+              kc = hash_cell(rel[2], H.dcz, H.rcz);
+    int val = point_cell(p, rel, ic, jc, kc, H, S.col_start, S.col_tri, S.col_kmax, S.tv, S.nf, S.s_tab, S.tf);
+    if (val < 0) {
+      atomicAdd(failed, 1);
+      val = 0;
+    }
+    nv = nv > val ? nv : (double)val;
+    if (nv < 0) nv = 0;
+  }
+  return nv;
+}
+// the dilation's test of a point as a neighbour, once per point instead of in
+// each of its 27 neighbours
+__device__ __forceinline__ uint8_t is_four(double nv) {
+  if ((__double_as_longlong(nv) << 1) == 0) return 0;
+  return (int)((nv < 0 ? 0. : nv) + 0.5) == 4;
+}
+// over every DA point (the search with IB node records; is4 null there)
+__global__ void k_ibm_classify_from(Grid g, const double *__restrict__ cent, int first, Surface S, const double *src,
+                                    double *dst, uint8_t *is4, int *failed) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  if (i >= g.mx) return;
   const size_t t = g.at(i, j, k);
-  double nv = src[t];
-  if (i >= 1 && i < g.mx - 1 && j >= 1 && j < g.my - 1 && k >= 1 && k < g.mz - 1) {
-    if (ibi == 0 && nv < 5.) nv = 0;
-    const double p[3] = {cent[t * 3], cent[t * 3 + 1], cent[t * 3 + 2]};
-    if (p[0] > H.xmin && p[0] < H.xmax && p[1] > H.ymin && p[1] < H.ymax && p[2] > H.zmin && p[2] < H.zmax) {
-      const int ic = (int)floor((p[0] - H.xmin) / H.dcx);
-      const int jc = (int)floor((p[1] - H.ymin) / H.dcy);
-      const int kc = (int)floor((p[2] - H.zmin) / H.dcz);
-      int val = point_cell(p, ic, jc, kc, H, col_start, col_tri, col_kmax, tv, nf, s_tab);
-      if (val < 0) {
-        atomicAdd(failed, 1);
-        val = 0;
-      }
-      nv = nv > val ? nv : (double)val;
-      if (nv < 0) nv = 0;
+  const double nv = classify_point(g, cent, first, S, i, j, k, t, src[t], failed);
+  dst[t] = nv;
+  if (is4) is4[t] = is_four(nv);
+}
+// Body 0 clears every interior value below 5, in place (negative boundary
+// values become 0, as the dilation leaves them); state[1]: a boundary point
+// counts as a 4 for the dilation.
+__global__ void k_ibm_clear(Grid g, double *nvert, int *state) {
+  const size_t N = g.n();
+  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < N; t += (size_t)gridDim.x * blockDim.x) {
+    const double v = nvert[t];
+    if (__double_as_longlong(v) == 0) continue;
+    int i, j, k;
+    da_ijk(g, t, i, j, k);
+    if (i >= 1 && i < g.mx - 1 && j >= 1 && j < g.my - 1 && k >= 1 && k < g.mz - 1) {
+      if (v < 5.) nvert[t] = 0;
+    } else {
+      if (v < 0) nvert[t] = 0;
+      if (is_four(v)) state[1] = 1;
     }
   }
-  dst[t] = nv;
-  // the dilation's test of this point as a neighbour, (int)(max(v, 0) + 0.5)
-  // == 4, once here instead of in each of its 27 neighbours (integer loads
-  // there; FP64 arithmetic is the scarce pipe)
-  if (is4) is4[t] = (int)((nv < 0 ? 0. : nv) + 0.5) == 4;
+}
+// A body changes only the cells whose centre lies in its hash box and, by the
+// dilation, their neighbours (the earlier bodies' marks are finished: no 2 or
+// 4 is left): both passes run on the index box of those cells (box: lower
+// ends, upper ends; k_ibm_box_cells), grown by m points.  Body 0, too, once
+// the mask is cleared: 28 M points 2.06 -> 0.50 ms.
+struct Region {
+  int lo[3], n[3];
+  __device__ Region(const Grid &g, const int *box, int m) {
+    const int hi[3] = {g.mx, g.my, g.mz};
+    for (int q = 0; q < 3; q++) {
+      lo[q] = max(box[q] - m, 0);
+      n[q] = box[0] > box[3] ? 0 : min(box[3 + q] + m + 1, hi[q]) - lo[q];
+    }
+  }
+};
+// (the last factor keeps a warp on consecutive points of the box)
+#define REGION_LOOP(R, i, j, k)                                                                              \
+  for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < (uint32_t)R.n[0] * R.n[1] * R.n[2];           \
+       w += gridDim.x * blockDim.x)                                                                          \
+    if (const uint32_t row = w / (uint32_t)R.n[0], kk = row / (uint32_t)R.n[1]; true)                       \
+      if (const int i = R.lo[0] + (int)(w - row * R.n[0]), j = R.lo[1] + (int)(row - kk * R.n[1]),           \
+          k = R.lo[2] + (int)kk;                                                                             \
+          true)
+__global__ void __launch_bounds__(128) k_ibm_classify(Grid g, const double *__restrict__ cent, Surface S,
+                                                      const int *__restrict__ box, const double *__restrict__ src,
+                                                      double *__restrict__ dst, uint8_t *is4, int *failed) {
+  const Region R(g, box, 2);
+  REGION_LOOP(R, i, j, k) {
+    const size_t t = g.at(i, j, k);
+    const double nv = classify_point(g, cent, false, S, i, j, k, t, src[t], failed);
+    dst[t] = nv;
+    is4[t] = is_four(nv);
+  }
 }
 
-// The search of a body after the first needs the index box of the interior
+// The search of a body needs the index box of the interior
 // cells whose centre lies strictly inside its hash box.  The centres are
 // bounded per block of 8x8x8 interior cells once per grid (k_cent_blocks);
 // a block whose bounds miss the hash box holds no such cell, so only the
@@ -192,7 +311,7 @@ __global__ void __launch_bounds__(512) k_cent_blocks(Grid g, const double *__res
 // One thread tests one block's bounds and lists the block when they meet
 // the hash box (box[6]: the count); then every thread block of a fixed grid
 // takes listed blocks in turn and tests their cells, two per thread (box[0..5]:
-// atomic min/max of i, j, k), so that a large box's blocks spread over the
+// min/max of i, j, k), so that a large box's blocks spread over the
 // whole GPU.
 __global__ void __launch_bounds__(256) k_ibm_box_hits(const double *__restrict__ bbox, int nblocks, HashBox H,
                                                       int *box, int *hits) {
@@ -205,6 +324,7 @@ __global__ void __launch_bounds__(256) k_ibm_box_hits(const double *__restrict__
 __global__ void __launch_bounds__(256) k_ibm_box_cells(Grid g, const double *__restrict__ cent, int nbx, int nby,
                                                        HashBox H, const int *__restrict__ hits, int *box) {
   const int nh = *(volatile int *)&box[6];
+  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
   for (int w = blockIdx.x; w < nh; w += gridDim.x) {
     const int bb = hits[w];
     const int bi = bb % nbx, bj = (bb / nbx) % nby, bk = bb / (nbx * nby);
@@ -214,10 +334,18 @@ __global__ void __launch_bounds__(256) k_ibm_box_cells(Grid g, const double *__r
       if (i >= g.mx - 1 || j >= g.my - 1 || k >= g.mz - 1) continue;
       const size_t t = g.at(i, j, k);
       const double p0 = cent[t * 3], p1 = cent[t * 3 + 1], p2 = cent[t * 3 + 2];
-      if (p0 > H.xmin && p0 < H.xmax && p1 > H.ymin && p1 < H.ymax && p2 > H.zmin && p2 < H.zmax) {
-        atomicMin(&box[0], i); atomicMin(&box[1], j); atomicMin(&box[2], k);
-        atomicMax(&box[3], i); atomicMax(&box[4], j); atomicMax(&box[5], k);
+      if (positive(p0 - H.xmin) && positive(H.xmax - p0) && positive(p1 - H.ymin) && positive(H.ymax - p1) &&
+          positive(p2 - H.zmin) && positive(H.zmax - p2)) {
+        lo[0] = min(lo[0], i); lo[1] = min(lo[1], j); lo[2] = min(lo[2], k);
+        hi[0] = max(hi[0], i); hi[1] = max(hi[1], j); hi[2] = max(hi[2], k);
       }
+    }
+  }
+  for (int q = 0; q < 3; q++) {  // six atomics a warp, not a cell
+    const int l = __reduce_min_sync(0xffffffffu, lo[q]), u = __reduce_max_sync(0xffffffffu, hi[q]);
+    if ((threadIdx.x & 31) == 0 && l <= u) {
+      atomicMin(&box[q], l);
+      atomicMax(&box[3 + q], u);
     }
   }
 }
@@ -268,14 +396,11 @@ __global__ void k_ibm_finish(Grid g, int b0, int b1, int b2, int b3, int b4, int
   nvert[t] = ibm_finish_value(g, b0, b1, b2, b3, b4, b5, i, j, k, nvert[t]);
 }
 // the dilation and the finishing pass in one (the search without IB node
-// records, where nothing reads the dilated marks in between): every DA
-// point of dst gets the dilation of src, the interior points then their
-// finished value
-__global__ void k_ibm_dilate_finish(Grid g, int b0, int b1, int b2, int b3, int b4, int b5,
-                                    const double *__restrict__ src, const uint8_t *__restrict__ is4,
-                                    double *__restrict__ dst, int3 lo, int3 hi) {
-  int i = lo.x + blockIdx.x * blockDim.x + threadIdx.x, j = lo.y + blockIdx.y, k = lo.z + blockIdx.z;
-  if (i >= hi.x) return;
+// records, where nothing reads the dilated marks in between): the DA points
+// get the dilation of src, the interior ones then their finished value
+__device__ __forceinline__ void dilate_finish_point(const Grid &g, const int (&b)[6], const double *__restrict__ src,
+                                                    const uint8_t *__restrict__ is4, double *__restrict__ dst, int i,
+                                                    int j, int k) {
   const size_t t = g.at(i, j, k);
   double v = src[t];
   if (v < 0) v = 0;
@@ -290,8 +415,22 @@ __global__ void k_ibm_dilate_finish(Grid g, int b0, int b1, int b2, int b3, int 
     if (near) v = v > 2 ? v : 2;
   }
   if (i >= 1 && i < g.mx - 1 && j >= 1 && j < g.my - 1 && k >= 1 && k < g.mz - 1)
-    v = ibm_finish_value(g, b0, b1, b2, b3, b4, b5, i, j, k, v);
+    v = ibm_finish_value(g, b[0], b[1], b[2], b[3], b[4], b[5], i, j, k, v);
   dst[t] = v;
+}
+struct Walls {
+  int b[6];
+};
+__global__ void k_ibm_dilate_finish_all(Grid g, Walls W, const double *__restrict__ src,
+                                        const uint8_t *__restrict__ is4, double *__restrict__ dst) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  if (i < g.mx) dilate_finish_point(g, W.b, src, is4, dst, i, j, k);
+}
+__global__ void __launch_bounds__(128) k_ibm_dilate_finish(Grid g, Walls W, const int *__restrict__ box,
+                                                           const double *__restrict__ src,
+                                                           const uint8_t *__restrict__ is4, double *__restrict__ dst) {
+  const Region R(g, box, 1);
+  REGION_LOOP(R, i, j, k) dilate_finish_point(g, W.b, src, is4, dst, i, j, k);
 }
 
 // ---- IB interpolation records (ibm.c:373-508) ----
@@ -604,8 +743,15 @@ int ibm_search_impl(vfs_poisson *h, int ibi, int n_v, const double *xyz, int n_e
   H.dcx = (H.xmax - H.xmin) / (kHash - 1.);
   H.dcy = (H.ymax - H.ymin) / (kHash - 1.);
   H.dcz = (H.zmax - H.zmin) / (kHash - 1.);
-  std::vector<std::vector<std::pair<int, int>>> cols(kHash * kHash);  // (kv_max, triangle)
-  std::vector<double> tv((size_t)n_elmt * 9), nf((size_t)n_elmt * 3);
+  H.fcx = (float)H.dcx; H.fcy = (float)H.dcy; H.fcz = (float)H.dcz;
+  H.rcx = (float)(1. / H.dcx); H.rcy = (float)(1. / H.dcy); H.rcz = (float)(1. / H.dcz);
+  H.fz = (float)(H.zmax + 0.2 - H.zmin);
+  H.L = (float)((H.xmax - H.xmin) + (H.ymax - H.ymin) + (H.zmax + 0.2 - H.zmin));
+  // everything the kernels read of the body in one buffer and one copy:
+  // column starts, column entries (triangle and its top hash cell, sorted by
+  // the latter, descending), vertices, normals, ray offsets, FP32 triangles
+  std::vector<int> range((size_t)n_elmt * 5);  // hash columns of a triangle, its top cell
+  std::vector<int> start(kHash * kHash + 1, 0);
   for (int e = 0; e < n_elmt; e++) {
     const int a = tri[3 * e], b = tri[3 * e + 1], c = tri[3 * e + 2];
     const double xv_min = std::min(std::min(x[a], x[b]), x[c]), xv_max = std::max(std::max(x[a], x[b]), x[c]);
@@ -617,8 +763,49 @@ int ibm_search_impl(vfs_poisson *h, int ibi, int n_v, const double *xyz, int n_e
     iv_min = std::max(iv_min, 0); iv_max = std::min(iv_max, kHash);
     jv_min = std::max(jv_min, 0); jv_max = jv_max > kHash ? kHash : jv_max;
     kv_max = std::min(kv_max, kHash);
+    const int r[5] = {iv_min, iv_max, jv_min, jv_max, kv_max};
+    std::copy(r, r + 5, &range[(size_t)e * 5]);
     for (int jj = jv_min; jj < jv_max; jj++)
-      for (int ii = iv_min; ii < iv_max; ii++) cols[jj * kHash + ii].push_back({kv_max, e});
+      for (int ii = iv_min; ii < iv_max; ii++) start[jj * kHash + ii + 1]++;
+  }
+  for (int q = 0; q < kHash * kHash; q++) start[q + 1] += start[q];
+  const size_t entries = (size_t)start[kHash * kHash];
+  size_t total = 0;
+  auto place = [&](size_t bytes) {
+    const size_t o = total;
+    total += (std::max<size_t>(bytes, 1) + 15) & ~(size_t)15;
+    return o;
+  };
+  const size_t o_start = place(start.size() * 4), o_tri = place(entries * 4), o_kmax = place(entries * 4),
+               o_tv = place((size_t)n_elmt * 72), o_nf = place((size_t)n_elmt * 24), o_s = place((kMaxTries + 1) * 8),
+               o_tf = place((size_t)n_elmt * 48);
+  std::vector<double> pack((total + 7) / 8);
+  unsigned char *pk = (unsigned char *)pack.data();
+  int *col_tri = (int *)(pk + o_tri), *col_kmax = (int *)(pk + o_kmax);
+  double *tv = (double *)(pk + o_tv), *nf = (double *)(pk + o_nf), *s_tab = (double *)(pk + o_s);
+  float *tf = (float *)(pk + o_tf);
+  std::copy(start.begin(), start.end(), (int *)(pk + o_start));
+  // triangles by descending top cell, equal ones in their order (a stable
+  // counting sort), dealt to their columns in that order
+  {
+    int first[kHash + 2] = {0};
+    auto key = [&](int e) { return kHash - std::max(range[(size_t)e * 5 + 4], 0); };
+    for (int e = 0; e < n_elmt; e++) first[key(e) + 1]++;
+    for (int q = 0; q <= kHash; q++) first[q + 1] += first[q];
+    std::vector<int> order(n_elmt), at(start.begin(), start.end());
+    for (int e = 0; e < n_elmt; e++) order[first[key(e)]++] = e;
+    for (int e : order) {
+      const int *r = &range[(size_t)e * 5];
+      for (int jj = r[2]; jj < r[3]; jj++)
+        for (int ii = r[0]; ii < r[1]; ii++) {
+          const int w = at[jj * kHash + ii]++;
+          col_tri[w] = e;
+          col_kmax[w] = r[4];
+        }
+    }
+  }
+  for (int e = 0; e < n_elmt; e++) {
+    const int a = tri[3 * e], b = tri[3 * e + 1], c = tri[3 * e + 2];
     const double vv[9] = {x[a], y[a], z[a], x[b], y[b], z[b], x[c], y[c], z[c]};
     std::copy(vv, vv + 9, &tv[(size_t)e * 9]);
     // face normal as the UCD reader computes it (Source/ibm_io.c:997-1011)
@@ -627,167 +814,118 @@ int ibm_search_impl(vfs_poisson *h, int ibi, int n_v, const double *xyz, int n_e
     const double fx = dy12 * dz13 - dz12 * dy13, fy = -dx12 * dz13 + dz12 * dx13, fz = dx12 * dy13 - dy12 * dx13;
     const double dr = std::sqrt(fx * fx + fy * fy + fz * fz);
     nf[(size_t)e * 3] = fx / dr; nf[(size_t)e * 3 + 1] = fy / dr; nf[(size_t)e * 3 + 2] = fz / dr;
+    const float f[12] = {(float)(x[a] - H.xmin), (float)(y[a] - H.ymin), (float)(z[a] - H.zmin),
+                         (float)dx12, (float)dy12, (float)dz12, (float)dx13, (float)dy13, (float)dz13,
+                         (float)(std::fabs(dx12) + std::fabs(dy12) + std::fabs(dz12)),
+                         (float)(std::fabs(dx13) + std::fabs(dy13) + std::fabs(dz13)), 0.f};
+    std::copy(f, f + 12, &tf[(size_t)e * 12]);
   }
-  std::vector<int> col_start(kHash * kHash + 1, 0), col_tri, col_kmax;
-  for (int q = 0; q < kHash * kHash; q++) {
-    auto &L = cols[q];
-    std::stable_sort(L.begin(), L.end(), [](const std::pair<int, int> &a, const std::pair<int, int> &b) {
-      return a.first > b.first;
-    });
-    col_start[q] = (int)col_tri.size();
-    for (auto &pr : L) { col_kmax.push_back(pr.first); col_tri.push_back(pr.second); }
-  }
-  col_start[kHash * kHash] = (int)col_tri.size();
-  std::vector<double> s_tab(kMaxTries + 1, 0.);
-  for (int q = 1; q <= kMaxTries; q++) s_tab[q] = glibc_rand_first((unsigned)q) / ((double)2147483647 + 1) - 0.5;
+  // (the offsets depend on nothing: formed once per process)
+  static const std::vector<double> offsets = [] {
+    std::vector<double> t(kMaxTries + 1, 0.);
+    for (int q = 1; q <= kMaxTries; q++) t[q] = glibc_rand_first((unsigned)q) / ((double)2147483647 + 1) - 0.5;
+    return t;
+  }();
+  std::copy(offsets.begin(), offsets.end(), s_tab);
 
-  // device copies in the handle's search buffers (grown on demand)
+  // device buffers of the handle's search (grown on demand): the body, two
+  // masks, the is-4 bytes, and box[7], failed rays and the boundary flag
   const size_t N = g.n();
-  void **buf = cx.scratch->buf;
-  size_t sizes[11] = {col_start.size() * 4, std::max<size_t>(col_tri.size(), 1) * 4,
-                      std::max<size_t>(col_kmax.size(), 1) * 4, tv.size() * 8, nf.size() * 8, s_tab.size() * 8,
-                      N * 8, N * 8, 4, N, 7 * 4};
+  IbmScratch &sc = *cx.scratch;
+  void **buf = sc.buf;
+  const int nbx = (g.mx - 2 + kCentBlock - 1) / kCentBlock, nby = (g.my - 2 + kCentBlock - 1) / kCentBlock,
+            nbz = (g.mz - 2 + kCentBlock - 1) / kCentBlock, nblocks = nbx * nby * nbz;
+  const bool dev = on_device(nvert);
+  const size_t sizes[IbmScratch::kBufs] = {total, N * 8, dev && !want_nodes ? 0 : N * 8, N, 9 * 4,
+                                           (size_t)nblocks * 6 * 8, (size_t)nblocks * 4};
   cudaStream_t st = cx.stream;
-  for (int q = 0; q < 11; q++)
-    if (cx.scratch->cap[q] < sizes[q]) {
+  for (int q = 0; q < IbmScratch::kBufs; q++)
+    if (sc.cap[q] < sizes[q]) {
       if (buf[q]) {
         cudaStreamSynchronize(st);
         cudaFree(buf[q]);
       }
       buf[q] = nullptr;
-      cx.scratch->cap[q] = 0;
+      sc.cap[q] = 0;
+      if (q == 5) sc.bbox_valid = false;
       if (cudaMalloc(&buf[q], sizes[q]) != cudaSuccess) {
         cudaGetLastError();
         buf[q] = nullptr;
         return fail(VFS_ENOMEM, "device allocation for the surface search failed");
       }
-      cx.scratch->cap[q] = sizes[q];
+      sc.cap[q] = sizes[q];
     }
-  const void *host[6] = {col_start.data(), col_tri.data(), col_kmax.data(), tv.data(), nf.data(), s_tab.data()};
-  size_t hsz[6] = {col_start.size() * 4, col_tri.size() * 4, col_kmax.size() * 4, tv.size() * 8, nf.size() * 8,
-                   s_tab.size() * 8};
-  for (int q = 0; q < 6; q++)
-    if (hsz[q]) cudaMemcpyAsync(buf[q], host[q], hsz[q], cudaMemcpyHostToDevice, st);
-  double *dnv = (double *)buf[6], *dtmp = (double *)buf[7];
-  int *dfail = (int *)buf[8];
-  const bool dev = on_device(nvert);
+  cudaMemcpyAsync(buf[0], pk, total, cudaMemcpyHostToDevice, st);
+  const unsigned char *db = (const unsigned char *)buf[0];
+  const Surface S{H, (const int *)(db + o_start), (const int *)(db + o_tri), (const int *)(db + o_kmax),
+                  (const double *)(db + o_tv), (const double *)(db + o_nf), (const double *)(db + o_s),
+                  (const float4 *)(db + o_tf)};
+  double *dnv = (double *)buf[1], *dtmp = (double *)buf[2], *bbox = (double *)buf[5];
+  uint8_t *dis4 = (uint8_t *)buf[3];
+  int *dbox = (int *)buf[4], *dfail = dbox + 7, *hits = (int *)buf[6];
   int b[6] = {0, 0, 0, 0, 0, 0};
   if (bctype)
     for (int q = 0; q < 6; q++) b[q] = bctype[q];
-  // the classification reads nvert where it lies (a host array is staged)
+  Walls W;
+  std::copy(b, b + 6, W.b);
+  const dim3 gi((g.mx - 2 + 127) / 128, g.my - 2, g.mz - 2), gd((g.mx + 127) / 128, g.my, g.mz);
+  int init[9] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0, 0, 0};
+  cudaMemcpyAsync(dbox, init, sizeof(init), cudaMemcpyHostToDevice, st);
+  if (!want_nodes) {
+    // nvert is updated in place (a host array in its staged copy)
+    double *nv = dev ? nvert : dtmp;
+    if (!dev) cudaMemcpyAsync(dtmp, nvert, N * 8, cudaMemcpyHostToDevice, st);
+    if (!sc.bbox_valid) {
+      k_cent_blocks<<<nblocks, 512, 0, st>>>(g, cx.cent, nbx, nby, bbox);
+      *cx.launches += 1;
+      sc.bbox_valid = true;
+    }
+    int state[2] = {0, 0};
+    auto read_state = [&] {
+      cudaMemcpyAsync(state, dfail, sizeof(state), cudaMemcpyDeviceToHost, st);
+      return cudaStreamSynchronize(st);
+    };
+    cudaError_t e = cudaSuccess;
+    if (ibi == 0) {
+      k_ibm_clear<<<152 * 8, 256, 0, st>>>(g, nv, dfail);
+      *cx.launches += 1;
+      e = read_state();
+    }
+    if (state[1]) {
+      // a boundary point that counts as a 4 marks cells far from the body,
+      // too: both passes over every point
+      k_ibm_classify_from<<<gd, 128, 0, st>>>(g, cx.cent, 1, S, nv, dnv, dis4, dfail);
+      k_ibm_dilate_finish_all<<<gd, 128, 0, st>>>(g, W, dnv, dis4, nv);
+      *cx.launches += 2;
+    } else {
+      k_ibm_box_hits<<<(nblocks + 255) / 256, 256, 0, st>>>(bbox, nblocks, H, dbox, hits);
+      k_ibm_box_cells<<<152 * 4, 256, 0, st>>>(g, cx.cent, nbx, nby, H, hits, dbox);
+      k_ibm_classify<<<152 * 8, 128, 0, st>>>(g, cx.cent, S, dbox, nv, dnv, dis4, dfail);
+      k_ibm_dilate_finish<<<152 * 8, 128, 0, st>>>(g, W, dbox, dnv, dis4, nv);
+      *cx.launches += 4;
+      if (ibi == 0 && std::any_of(b, b + 6, [](int v) { return v == -1 || v == -2; })) {
+        k_ibm_finish<<<gi, 128, 0, st>>>(g, b[0], b[1], b[2], b[3], b[4], b[5], nv);
+        *cx.launches += 1;
+      }
+    }
+    if (e == cudaSuccess) e = read_state();
+    if (e == cudaSuccess && !dev) e = cudaMemcpy(nvert, dtmp, N * 8, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(VFS_ECUDA, std::string("surface search: ") + cudaGetErrorString(e));
+    }
+    if (n_failed) *n_failed = state[0];
+    if (n_nodes) *n_nodes = 0;
+    return VFS_OK;
+  }
+  // with IB node records: every pass over all points (the classification
+  // reads nvert where it lies; a host array is staged)
   const double *src = nvert;
   if (!dev) {
     cudaMemcpyAsync(dtmp, nvert, N * 8, cudaMemcpyHostToDevice, st);
     src = dtmp;
   }
-  cudaMemsetAsync(dfail, 0, 4, st);
-  dim3 gi((g.mx - 2 + 127) / 128, g.my - 2, g.mz - 2), gd((g.mx + 127) / 128, g.my, g.mz);
-  uint8_t *dis4 = (uint8_t *)buf[9];
-  const int3 all_lo = make_int3(0, 0, 0), all_hi = make_int3(g.mx, g.my, g.mz);
-  if (!want_nodes && ibi > 0) {
-    // A body after the first changes only the cells whose centre lies in its
-    // hash box and, by the dilation, their neighbours: the earlier bodies'
-    // marks are finished (no 2 or 4 is left) and the wall rows' rule gives
-    // what it gave before.  So both passes run on that index box, grown by
-    // one cell for the dilation and by one more for the copy it reads.
-    int init[7] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0}, bx[6];
-    int *dbox = (int *)buf[10];
-    const int nbx = (g.mx - 2 + kCentBlock - 1) / kCentBlock, nby = (g.my - 2 + kCentBlock - 1) / kCentBlock,
-              nbz = (g.mz - 2 + kCentBlock - 1) / kCentBlock, nblocks = nbx * nby * nbz;
-    IbmScratch &sc = *cx.scratch;
-    if (!sc.bbox_valid) {
-      const size_t need = (size_t)nblocks * 6 * 8;
-      if (sc.bbox_cap < need) {
-        if (sc.bbox) {
-          cudaStreamSynchronize(st);
-          cudaFree(sc.bbox);
-        }
-        sc.bbox = nullptr;
-        sc.bbox_cap = 0;
-        if (cudaMalloc(&sc.bbox, need) != cudaSuccess) {
-          cudaGetLastError();
-          sc.bbox = nullptr;
-          return fail(VFS_ENOMEM, "device allocation for the surface search failed");
-        }
-        sc.bbox_cap = need;
-      }
-      k_cent_blocks<<<nblocks, 512, 0, st>>>(g, cx.cent, nbx, nby, sc.bbox);
-      *cx.launches += 1;
-      sc.bbox_valid = true;
-    }
-    if (sc.hits_cap < (size_t)nblocks * 4) {
-      if (sc.hits) {
-        cudaStreamSynchronize(st);
-        cudaFree(sc.hits);
-      }
-      sc.hits = nullptr;
-      sc.hits_cap = 0;
-      if (cudaMalloc(&sc.hits, (size_t)nblocks * 4) != cudaSuccess) {
-        cudaGetLastError();
-        sc.hits = nullptr;
-        return fail(VFS_ENOMEM, "device allocation for the surface search failed");
-      }
-      sc.hits_cap = (size_t)nblocks * 4;
-    }
-    cudaMemcpyAsync(dbox, init, sizeof(init), cudaMemcpyHostToDevice, st);
-    k_ibm_box_hits<<<(nblocks + 255) / 256, 256, 0, st>>>(sc.bbox, nblocks, H, dbox, sc.hits);
-    k_ibm_box_cells<<<152 * 4, 256, 0, st>>>(g, cx.cent, nbx, nby, H, sc.hits, dbox);
-    cudaMemcpyAsync(bx, dbox, sizeof(bx), cudaMemcpyDeviceToHost, st);
-    *cx.launches += 2;
-    cudaError_t eb = cudaStreamSynchronize(st);
-    if (eb != cudaSuccess) {
-      cudaGetLastError();
-      return fail(VFS_ECUDA, std::string("surface search: ") + cudaGetErrorString(eb));
-    }
-    if (n_failed) *n_failed = 0;
-    if (n_nodes) *n_nodes = 0;
-    if (bx[0] > bx[3]) return VFS_OK;  // no cell centre in the body's box: nothing changes
-    auto grow = [&](int m) {
-      return std::make_pair(make_int3(std::max(bx[0] - m, 0), std::max(bx[1] - m, 0), std::max(bx[2] - m, 0)),
-                            make_int3(std::min(bx[3] + m + 1, g.mx), std::min(bx[4] + m + 1, g.my),
-                                      std::min(bx[5] + m + 1, g.mz)));
-    };
-    const auto r2 = grow(2), r1 = grow(1);
-    auto grid_of = [](int3 lo, int3 hi) { return dim3((hi.x - lo.x + 127) / 128, hi.y - lo.y, hi.z - lo.z); };
-    if (!dev) cudaMemcpyAsync(dtmp, nvert, N * 8, cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(dfail, 0, 4, st);
-    k_ibm_classify_from<<<grid_of(r2.first, r2.second), 128, 0, st>>>(
-        g, cx.cent, ibi, H, (int *)buf[0], (int *)buf[1], (int *)buf[2], (double *)buf[3], (double *)buf[4],
-        (double *)buf[5], dev ? nvert : dtmp, dnv, dis4, dfail, r2.first, r2.second);
-    k_ibm_dilate_finish<<<grid_of(r1.first, r1.second), 128, 0, st>>>(g, b[0], b[1], b[2], b[3], b[4], b[5], dnv,
-                                                                      dis4, dev ? nvert : dtmp, r1.first, r1.second);
-    *cx.launches += 2;
-    int nfail = 0;
-    if (!dev) cudaMemcpyAsync(nvert, dtmp, N * 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&nfail, dfail, 4, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(VFS_ECUDA, std::string("surface search: ") + cudaGetErrorString(e));
-    }
-    if (n_failed) *n_failed = nfail;
-    return VFS_OK;
-  }
-  k_ibm_classify_from<<<gd, 128, 0, st>>>(g, cx.cent, ibi, H, (int *)buf[0], (int *)buf[1], (int *)buf[2],
-                                          (double *)buf[3], (double *)buf[4], (double *)buf[5], src, dnv,
-                                          want_nodes ? nullptr : dis4, dfail, all_lo, all_hi);
-  if (!want_nodes) {
-    // dilation and finish in one pass, straight into a device nvert
-    double *out = dev ? nvert : dtmp;
-    k_ibm_dilate_finish<<<gd, 128, 0, st>>>(g, b[0], b[1], b[2], b[3], b[4], b[5], dnv, dis4, out, all_lo, all_hi);
-    *cx.launches += 2;
-    int nfail = 0;
-    if (!dev) cudaMemcpyAsync(nvert, dtmp, N * 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&nfail, dfail, 4, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(VFS_ECUDA, std::string("surface search: ") + cudaGetErrorString(e));
-    }
-    if (n_failed) *n_failed = nfail;
-    if (n_nodes) *n_nodes = 0;
-    return VFS_OK;
-  }
+  k_ibm_classify_from<<<gd, 128, 0, st>>>(g, cx.cent, ibi == 0, S, src, dnv, nullptr, dfail);
   k_ibm_dilate<<<gd, 128, 0, st>>>(g, dnv, dtmp);
   int nodes_found = 0;
   if (want_nodes) {  // the IB nodes (marked 2) and their interpolation records
@@ -824,8 +962,7 @@ int ibm_search_impl(vfs_poisson *h, int ibi, int n_v, const double *xyz, int n_e
       k_ibm_mark_scatter<<<nb, 256, 0, st>>>(g, dtmp, dcount, dlist);
       if (nodes_found > 0)
         k_ibm_nodes<<<(nodes_found + 127) / 128, 128, 0, st>>>(g, cx.cent, dlist, nodes_found, n_elmt,
-                                                               (const double *)buf[3], (const double *)buf[4], dq,
-                                                               drad, body.nodes);
+                                                               S.tv, S.nf, dq, drad, body.nodes);
       *cx.launches += 3;
       ok = cudaStreamSynchronize(st) == cudaSuccess;
     }

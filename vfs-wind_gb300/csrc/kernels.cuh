@@ -264,16 +264,14 @@ struct IbmBody {
 };
 // device buffers of the surface search, kept by the handle and grown on
 // demand (no allocation or free, and so no device synchronisation, per body)
+// the body, two masks, the is-4 bytes, box and flags, bounds of the cell
+// centres over blocks of 8x8x8 interior cells (6 doubles each, formed by the
+// first search after the grid was set) and the blocks that meet a hash box
 struct IbmScratch {
-  void *buf[11] = {};
-  size_t cap[11] = {};
-  // bounds of the cell centres over blocks of 8x8x8 interior cells (6
-  // doubles each), formed by the first search after the grid was set
-  double *bbox = nullptr;
-  size_t bbox_cap = 0;
+  static constexpr int kBufs = 7;
+  void *buf[kBufs] = {};
+  size_t cap[kBufs] = {};
   bool bbox_valid = false;
-  int *hits = nullptr;  // the blocks that meet a body's hash box
-  size_t hits_cap = 0;
 };
 struct IbmContext {
   cudaStream_t stream;
