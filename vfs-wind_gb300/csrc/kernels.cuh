@@ -207,7 +207,8 @@ GS_DOTS_DECL(7)
 GS_DOTS_DECL(8)
 #undef GS_DOTS_DECL
 #define CGS_DOTS_DECL(NV) \
-  __global__ void k_cgs_dots##NV(size_t n, int v0, const double *const *Q, const double *w, double *partial);
+  __global__ void k_cgs_dots##NV(size_t n, int v0, const double *const *Q, const double *w, double *partial); \
+  __global__ void k_cgs_dots_small##NV(size_t n, int v0, const double *const *Q, const double *w, double *partial);
 CGS_DOTS_DECL(1)
 CGS_DOTS_DECL(2)
 CGS_DOTS_DECL(3)
@@ -217,9 +218,11 @@ CGS_DOTS_DECL(6)
 CGS_DOTS_DECL(7)
 CGS_DOTS_DECL(8)
 #undef CGS_DOTS_DECL
-__global__ void k_cgs_reduce(const double *partial, int nb, const double *dsv, double *red);
+__global__ void k_cgs_reduce(const double *partial, int nb, const double *dsv, double *red, double *hess);
 __global__ void k_cgs_update(size_t n, int nv, const double *const *Q, const double *red, double *w,
                              double *partial);
+__global__ void k_cgs_update_small(size_t n, int nv, const double *const *Q, const double *red, double *w,
+                                   double *partial);
 __global__ void k_gs_reduce(const double *partial, int nb, int nv, double *red);
 __global__ void k_gs_coef(int nv, double *red);
 __global__ void k_gs_update(size_t n, int nv, const double *const *Q, const double *red, double *u, double *w,
@@ -229,7 +232,7 @@ __global__ void k_scale_to(size_t n, const double *v, double s, const double *si
                            double *out);
 __global__ void k_scale_to32(size_t n, const double *v, float s, const float *sinv, const float *scale, float *out,
                              int split_nx);
-__global__ void k_reduce_norm(const double *partial, int nb, double *out, float *out32);
+__global__ void k_reduce_norm(const double *partial, int nb, double *out, float *out32, double *norm2);
 __global__ void k_to64(size_t n, const float *x32, const double *x64, double *out, int split_nx);
 __global__ void k_sumsq(size_t n, const double *x, double *partial);
 // history projection of the initial guess (at most kHistMax solutions:

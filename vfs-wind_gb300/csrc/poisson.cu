@@ -1525,8 +1525,8 @@ void vcycle(vfs_poisson *h, int li, int nu1, int nu2, T omega, int smoother) {
   if ((smoother == 3 || smoother == 4) && nu1 > 0 && omega == (T)1) {
     // the second colour's lines were just solved exactly (omega 1), so its
     // residual is zero up to rounding: form the first colour's only
+    // (and 0 on the second's)
     const int nh = (l.b.nx + 1) / 2;
-    vmemset(h, r, l.b.n() * sizeof(T));
     Prec<T>::residual(h, l, dim3((nh + 127) / 128, l.b.ny, l.b.nz), x, bb, r, 6, split_level<T>(h, li, smoother));
   } else {
     Prec<T>::residual(h, l, box_grid(l.b), x, bb, r, -1, split_level<T>(h, li, smoother));
@@ -1542,16 +1542,28 @@ void vcycle(vfs_poisson *h, int li, int nu1, int nu2, T omega, int smoother) {
   Prec<T>::xfinal(l) = x;
 }
 
+constexpr int kDirectLevels = 1;
 // Run one V-cycle on level 0 (rhs already in level 0's b buffer).
 template <typename T>
 int run_vcycle(vfs_poisson *h, const vfs_solve_opts &o) {
   const int p = std::is_same<T, float>::value ? 0 : 1;
-  h->pdl_prev = false;  // the V-cycle's first kernel waits for all earlier work
-  if (!o.use_graphs || h->prof) {  // live kernel timing runs the V-cycle without a graph
+  // A V-cycle with at most kDirectLevels levels above its tail is a dozen
+  // launches at most: issued one by one they start with the chain (a graph
+  // starts 10-14 us after its predecessor ends, and its launch takes as long as
+  // theirs): 24x16x24 1016 -> 985 us a solve, 64^3 1704 -> 1671, FP64 72x40x56
+  // 5866 -> 5812 (two levels above the tail: 6050).  Live kernel timing runs
+  // without a graph, too.
+  TailArgs ta;
+  size_t tsm;
+  int above = 0;
+  while (above <= kDirectLevels && above < (int)h->L.size() && !tail_plan<T>(h, above, o.nu1, o.smoother, &ta, &tsm))
+    above++;
+  if (!o.use_graphs || h->prof || above <= kDirectLevels) {
     h->pcount = 0;
     vcycle<T>(h, 0, o.nu1, o.nu2, (T)o.omega, o.smoother);
     return VFS_OK;
   }
+  h->pdl_prev = false;  // the graph waits for all earlier work
   const int key[4] = {o.nu1, o.nu2, (int)h->prof, o.smoother};
   vfs_poisson::GraphSlot *slot = nullptr, *victim = &h->gslot[p][0];
   for (auto &g : h->gslot[p]) {
@@ -1587,6 +1599,7 @@ int run_vcycle(vfs_poisson *h, const vfs_solve_opts &o) {
   slot->used = ++h->gclock;
   CUDA_TRY(cudaGraphLaunch(slot->exec, h->stream));
   h->launches += slot->nodes;
+  h->pdl_prev = false;
   return VFS_OK;
 }
 
@@ -1597,15 +1610,16 @@ int precondition(vfs_poisson *h, const double *v, double s, const double *sinv64
                  const vfs_solve_opts &o) {
   Level &l0 = h->L[0];
   const size_t n = h->box.n();
+  h->pdl_prev = false;  // the chain's first kernel waits for all earlier work
   if (o.precision == 0) {
     const int snx = split_level<float>(h, 0, o.smoother) ? l0.b.nx : 0;
-    LAUNCH(h, k_scale_to32, lin_grid(n), 256, n, v, (float)s, sinv32, h->scale32, l0.v32[1], snx);
+    launch_v(h, k_scale_to32, lin_grid(n), 256, 0, n, v, (float)s, sinv32, (const float *)h->scale32, l0.v32[1], snx);
     TRY(run_vcycle<float>(h, o));
-    LAUNCH(h, k_to64, lin_grid(n), 256, n, (const float *)l0.xfinal32, (const double *)nullptr, z, snx);
+    launch_v(h, k_to64, lin_grid(n), 256, 0, n, (const float *)l0.xfinal32, (const double *)nullptr, z, snx);
   } else {
-    LAUNCH(h, k_scale_to, kRedBlocks, 256, n, v, s, sinv64, h->scale, l0.v64[1]);
+    launch_v(h, k_scale_to, kRedBlocks, 256, 0, n, v, s, sinv64, (const double *)h->scale, l0.v64[1]);
     TRY(run_vcycle<double>(h, o));
-    LAUNCH(h, k_to64, lin_grid(n), 256, n, (const float *)nullptr, (const double *)l0.xfinal64, z, 0);
+    launch_v(h, k_to64, lin_grid(n), 256, 0, n, (const float *)nullptr, (const double *)l0.xfinal64, z, 0);
   }
   return VFS_OK;
 }
@@ -2029,13 +2043,15 @@ void gs_dots(vfs_poisson *h, int nv, int nb, size_t n, int v0, const double *u, 
   }
 }
 
+// Up to two blocks a SM, where a thread's loads may take all its registers.
+constexpr int kSmallBlocks = 304;
 // One classical Gram-Schmidt dots launch over basis vectors v0 .. v0+nv-1
 // (1 <= nv <= 8).
 void cgs_dots(vfs_poisson *h, int nv, int nb, size_t n, int v0, const double *w) {
   const double *const *Q = (const double *const *)h->dV;
   switch (nv) {
 #define CASE(NV) \
-  case NV: LAUNCH(h, k_cgs_dots##NV, nb, 256, n, v0, Q, w, h->partial); break;
+  case NV: launch_v(h, nb <= kSmallBlocks ? k_cgs_dots_small##NV : k_cgs_dots##NV, nb, 256, 0, n, v0, Q, w, h->partial); break;
     CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
 #undef CASE
   }
@@ -2047,32 +2063,44 @@ constexpr int kSpecHb = 620, kSpecStage = 610;
 
 // Enqueue Arnoldi step jj of FGMRES: precondition V_jj (unless Z_jj holds it
 // already: have_z), apply A, orthogonalise (orth 0 or DCGS2), reduce the new
-// vector's norm and copy the Hessenberg data to hbuf + hb (orth 0: h at
-// hb + 0..jj; the norm^2 at hb + kGsR + 3).
+// vector's norm and bring the Hessenberg data to hbuf + hb (orth 0: h at
+// hb + 0..jj; the norm^2 at hb + kGsR + 3), written there by the kernels
+// (pinned memory).  With orth 0 the whole step is one chain of dependent
+// launches.
 int arnoldi_enqueue(vfs_poisson *h, int jj, int nbd, const vfs_solve_opts &o, int hb, bool have_z = false) {
   const size_t n = h->box.n();
   const double *const *dV = (const double *const *)h->dV;
   if (!have_z) TRY(precondition(h, h->V[jj], 1.0, h->dsv + 2 * jj + 1, h->dsv32 + jj, h->Z[jj], o));
-  if (h->phase && hb == 0) cudaEventRecord(h->phev[1], h->stream);
+  else h->pdl_prev = false;
+  auto stamp = [&](int q) {
+    if (!h->phase || hb != 0) return;
+    cudaEventRecord(h->phev[q], h->stream);
+    h->pdl_prev = false;
+  };
+  stamp(1);
   double *w = h->V[jj + 1];
-  LAUNCH(h, k_apply64, box_grid(h->box), 128, h->box, h->A0, h->Z[jj], w);
-  if (h->phase && hb == 0) cudaEventRecord(h->phev[2], h->stream);
+  launch_v(h, k_apply64, box_grid(h->box), 128, 0, h->box, (const double *)h->A0, (const double *)h->Z[jj], w);
+  stamp(2);
+  double *back = h->hbuf + hb;
   if (o.orth == 0) {
     for (int v0 = 0; v0 <= jj; v0 += 8) cgs_dots(h, std::min(8, jj + 1 - v0), nbd, n, v0, w);
-    LAUNCH(h, k_cgs_reduce, jj + 1, 1024, h->partial, nbd, h->dsv, h->red);
-    LAUNCH(h, k_cgs_update, nbd, 256, n, jj + 1, dV, h->red, w, h->partial);
+    launch_v(h, k_cgs_reduce, jj + 1, 1024, 0, (const double *)h->partial, nbd, (const double *)h->dsv, h->red, back);
+    launch_v(h, nbd <= kSmallBlocks ? k_cgs_update_small : k_cgs_update, nbd, 256, 0, n, jj + 1, dV,
+             (const double *)h->red, w, h->partial);
   } else {
     for (int v0 = 0; v0 == 0 || v0 < jj; v0 += 8)
       gs_dots(h, std::min(8, jj - v0), nbd, n, v0, h->V[jj], w, v0 == 0);
     LAUNCH(h, k_gs_reduce, 2 * jj + 2, 1024, h->partial, nbd, jj, h->red);
     LAUNCH(h, k_gs_coef, 1, 32, jj, h->red);
     LAUNCH(h, k_gs_update, nbd, 256, n, jj, dV, h->red, h->V[jj], w, h->partial);
+    h->pdl_prev = false;
   }
-  LAUNCH(h, k_reduce_norm, 1, 1024, h->partial, nbd, h->dsv + 2 * (jj + 1), h->dsv32 + jj + 1);
-  if (h->phase && hb == 0) cudaEventRecord(h->phev[3], h->stream);
-  CUDA_TRY(cudaMemcpyAsync(h->hbuf + hb, h->red, (o.orth == 0 ? jj + 1 : kGsR + 3) * 8, cudaMemcpyDeviceToHost,
-                           h->stream));
-  CUDA_TRY(cudaMemcpyAsync(h->hbuf + hb + kGsR + 3, h->dsv + 2 * (jj + 1), 8, cudaMemcpyDeviceToHost, h->stream));
+  launch_v(h, k_reduce_norm, 1, 1024, 0, (const double *)h->partial, nbd, h->dsv + 2 * (jj + 1), h->dsv32 + jj + 1,
+           back + kGsR + 3);
+  h->pdl_prev = false;
+  stamp(3);
+  if (o.orth != 0)
+    CUDA_TRY(cudaMemcpyAsync(back, h->red, (kGsR + 3) * 8, cudaMemcpyDeviceToHost, h->stream));
   return VFS_OK;
 }
 

@@ -32,6 +32,14 @@ __device__ __forceinline__ bool colour_row(const Box &b, int color, int t, int k
   return t < b.nx && (color < 0 || (k & 1) == color);
 }
 
+// colours 6/7: the row's cell t of the other colour gets the residual 0 (no
+// clearing pass, which would also part the chain of dependent launches)
+template <typename T>
+__device__ __forceinline__ void clear_partner(const Box &b, int color, int t, uint32_t row, int k, T *__restrict__ r) {
+  const int par = (color + k) & 1, i = 2 * t + 1 - par;
+  if (i < b.nx) r[row + i] = (T)0;
+}
+
 template <typename T>
 __device__ __forceinline__ void residual_body(Box b, const T *__restrict__ A, const T *__restrict__ x,
                                               const T *__restrict__ rhs, T *__restrict__ r, int color) {
@@ -39,6 +47,7 @@ __device__ __forceinline__ void residual_body(Box b, const T *__restrict__ A, co
   pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
   int p;
+  if (color >= 6) clear_partner(b, color, t, (uint32_t)b.at(0, j, k), k, r);
   if (!colour_row(b, color, t, k, p)) return;
   const int i = split_cell(p, b.nx);
   uint32_t idx[NSLOT];
@@ -113,6 +122,7 @@ __device__ __forceinline__ void residual16_body(Box b, const __half2 *__restrict
     d = __ldcs(&D[cs]);
   }
   pdl_wait();
+  if (color >= 6) clear_partner(b, color, t, row, k, r);
   if (!ok) return;
   const float xc = __ldg(&x[c]);
   float s = 0.f;
@@ -140,7 +150,9 @@ __global__ void __launch_bounds__(128) k_residual16_split(Box b, const __half2 *
 // FP64 y = A x on the unscaled operator.
 __global__ void __launch_bounds__(256) k_apply64(Box b, const double *__restrict__ A, const double *__restrict__ x,
                                                  double *__restrict__ y) {
+  pdl_trigger();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  pdl_wait();
   if (i >= b.nx) return;
   uint32_t idx[NSLOT];
   stencil_index(b, i, j, k, idx);
@@ -732,13 +744,44 @@ __device__ __forceinline__ void gs_dots_body(size_t n, int v0, const double *con
     if (a < 2 * NV || first) partial[(size_t)row * gridDim.x + blockIdx.x] = s;
   }
 }
+// The warp sums of NV values per lane with warp_sum's additions, packed: a
+// step adds halves only, so two values share an instruction (lanes with bit o
+// take the second of a pair).  9 FP64 additions for 8 values instead of 40,
+// the same bits.  The sum of value v ends in lane packed_lane(v).
+template <int NV>
+__device__ __forceinline__ double warp_sum_packed(double (&a)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int m = NV;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int p = 0; p < (NV + 1) / 2; p++) {
+      if (2 * p + 1 < m) {
+        const bool up = lane & o;
+        const double keep = up ? a[2 * p + 1] : a[2 * p], send = up ? a[2 * p] : a[2 * p + 1];
+        a[p] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      } else if (2 * p < m) {
+        a[p] = a[2 * p] + __shfl_xor_sync(0xffffffffu, a[2 * p], o);
+      }
+    }
+    m = (m + 1) / 2;
+  }
+  return a[0];
+}
+__device__ __forceinline__ int packed_lane(int v) { return (v & 1) * 16 + (v & 2) * 4 + (v & 4); }
+
 // Classical Gram-Schmidt in one pass (the orthogonalisation of PETSc's
 // GMRES with its default refinement "never"): rows kGsB + v0 + v of the
 // block partials hold Q_{v0+v}.w, the basis vectors kept unnormalised.
-template <int NV>
+// Bound by the FP64 pipe on large boxes (a warp's sums were 0.6 of its
+// products before they were packed) and by latency on small ones, where every
+// load of a thread goes out at once (U = kGsTile).
+// 6 vectors of 128x96x128: 36 -> 25 us (the pipe: 19); 4 of 24x16x24: 8.2 -> 4.4.
+template <int NV, int U>
 __device__ __forceinline__ void cgs_dots_body(size_t n, int v0, const double *const *__restrict__ Q,
                                               const double *__restrict__ w, double *__restrict__ partial) {
   __shared__ double sh[8][NV];
+  pdl_trigger();
   double acc[NV];
   const double *q[NV];
 #pragma unroll
@@ -746,33 +789,45 @@ __device__ __forceinline__ void cgs_dots_body(size_t n, int v0, const double *co
     acc[v] = 0.;
     q[v] = Q[v0 + v];
   }
+  pdl_wait();
   const size_t base = (size_t)blockIdx.x * blockDim.x * kGsTile + threadIdx.x;
-#pragma unroll 2
-  for (int t = 0; t < kGsTile; t++) {
-    const size_t c = base + (size_t)t * blockDim.x;
-    if (c < n) {
-      const double wc = __ldg(&w[c]);
+#pragma unroll 1
+  for (int t0 = 0; t0 < kGsTile; t0 += U) {
+    double wc[U], qc[U][NV];
 #pragma unroll
-      for (int v = 0; v < NV; v++) acc[v] = fma(__ldcs(q[v] + c), wc, acc[v]);
+    for (int t = 0; t < U; t++) {
+      const size_t c = base + (size_t)(t0 + t) * blockDim.x;
+      const bool in = c < n;
+      wc[t] = in ? __ldg(&w[c]) : 0.;
+#pragma unroll
+      for (int v = 0; v < NV; v++) qc[t][v] = in ? __ldcs(q[v] + c) : 0.;
     }
+#pragma unroll
+    for (int t = 0; t < U; t++)
+#pragma unroll
+      for (int v = 0; v < NV; v++) acc[v] = fma(qc[t][v], wc[t], acc[v]);
   }
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const double s = warp_sum_packed<NV>(acc);
 #pragma unroll
-  for (int v = 0; v < NV; v++) {
-    const double s = warp_sum(acc[v]);
-    if (lane == 0) sh[wp][v] = s;
-  }
+  for (int v = 0; v < NV; v++)
+    if (lane == packed_lane(v)) sh[wp][v] = s;
   __syncthreads();
   if (threadIdx.x < NV) {
-    double s = 0.;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += sh[k][threadIdx.x];
-    partial[(size_t)(kGsB + v0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+    double r = 0.;
+#pragma unroll
+    for (int k = 0; k < 8; k++) r += sh[k][threadIdx.x];
+    partial[(size_t)(kGsB + v0 + threadIdx.x) * gridDim.x + blockIdx.x] = r;
   }
 }
 #define CGS_DOTS(NV)                                                                                            \
   __global__ void __launch_bounds__(256) k_cgs_dots##NV(size_t n, int v0, const double *const *Q,               \
                                                         const double *w, double *partial) {                     \
-    cgs_dots_body<NV>(n, v0, Q, w, partial);                                                                   \
+    cgs_dots_body<NV, 2>(n, v0, Q, w, partial);                                                                \
+  }                                                                                                            \
+  __global__ void __launch_bounds__(256, 1) k_cgs_dots_small##NV(size_t n, int v0, const double *const *Q,      \
+                                                                 const double *w, double *partial) {            \
+    cgs_dots_body<NV, kGsTile>(n, v0, Q, w, partial);                                                          \
   }
 CGS_DOTS(1)
 CGS_DOTS(2)
@@ -785,10 +840,13 @@ CGS_DOTS(8)
 #undef CGS_DOTS
 
 // One block per basis vector v: d = Q_v.w summed in a fixed order, then
-// h_v = d / ||Q_v|| (the Hessenberg entry, red[v]) and the update
-// coefficient h_v / ||Q_v|| (red[kGsB + v]); dsv[2v+1] = 1 / ||Q_v||.
+// h_v = d / ||Q_v|| (the Hessenberg entry, red[v] and the host's copy hess[v])
+// and the update coefficient h_v / ||Q_v|| (red[kGsB + v]);
+// dsv[2v+1] = 1 / ||Q_v||.
 __global__ void k_cgs_reduce(const double *__restrict__ partial, int nb, const double *__restrict__ dsv,
-                             double *red) {
+                             double *red, double *hess) {
+  pdl_trigger();
+  pdl_wait();
   const int v = blockIdx.x;
   double s = 0.;
   for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[(size_t)(kGsB + v) * nb + q];
@@ -797,13 +855,18 @@ __global__ void k_cgs_reduce(const double *__restrict__ partial, int nb, const d
     const double sinv = dsv[2 * v + 1], hv = s * sinv;
     red[v] = hv;
     red[kGsB + v] = hv * sinv;
+    hess[v] = hv;
   }
 }
 
-// w -= sum_v red[kGsB + v] Q_v; block partials of ||w||^2.
-__global__ void __launch_bounds__(256) k_cgs_update(size_t n, int nv, const double *const *__restrict__ Q,
-                                                    const double *__restrict__ red, double *__restrict__ w,
-                                                    double *partial) {
+// w -= sum_v red[kGsB + v] Q_v; block partials of ||w||^2.  VU vectors' loads
+// go out at once (small boxes: latency).
+template <int VU>
+__device__ __forceinline__ void cgs_update_body(size_t n, int nv, const double *const *__restrict__ Q,
+                                                const double *__restrict__ red, double *__restrict__ w,
+                                                double *partial) {
+  pdl_trigger();
+  pdl_wait();
   const size_t base = (size_t)blockIdx.x * blockDim.x * kGsTile + threadIdx.x;
   double aw[kGsTile];
 #pragma unroll
@@ -811,14 +874,24 @@ __global__ void __launch_bounds__(256) k_cgs_update(size_t n, int nv, const doub
     const size_t c = base + (size_t)t * blockDim.x;
     aw[t] = c < n ? w[c] : 0.;
   }
-  for (int v = 0; v < nv; v++) {
-    const double *p = Q[v];
-    const double cb = -red[kGsB + v];
+  for (int v0 = 0; v0 < nv; v0 += VU) {
+    double q[VU][kGsTile], cb[VU];
 #pragma unroll
-    for (int t = 0; t < kGsTile; t++) {
-      const size_t c = base + (size_t)t * blockDim.x;
-      if (c < n) aw[t] = fma(cb, __ldcs(&p[c]), aw[t]);
+    for (int v = 0; v < VU; v++) {
+      const int vv = min(v0 + v, nv - 1);
+      const double *p = Q[vv];
+      cb[v] = -red[kGsB + vv];
+#pragma unroll
+      for (int t = 0; t < kGsTile; t++) {
+        const size_t c = base + (size_t)t * blockDim.x;
+        q[v][t] = c < n ? __ldcs(&p[c]) : 0.;
+      }
     }
+#pragma unroll
+    for (int v = 0; v < VU; v++)
+      if (v0 + v < nv)
+#pragma unroll
+        for (int t = 0; t < kGsTile; t++) aw[t] = fma(cb[v], q[v][t], aw[t]);
   }
   double ss = 0.;
 #pragma unroll
@@ -831,6 +904,14 @@ __global__ void __launch_bounds__(256) k_cgs_update(size_t n, int nv, const doub
   }
   ss = block_sum(ss);
   if (threadIdx.x == 0) partial[blockIdx.x] = ss;
+}
+__global__ void __launch_bounds__(256) k_cgs_update(size_t n, int nv, const double *const *Q, const double *red,
+                                                    double *w, double *partial) {
+  cgs_update_body<1>(n, nv, Q, red, w, partial);
+}
+__global__ void __launch_bounds__(256, 1) k_cgs_update_small(size_t n, int nv, const double *const *Q,
+                                                             const double *red, double *w, double *partial) {
+  cgs_update_body<4>(n, nv, Q, red, w, partial);
 }
 
 #define GS_DOTS(NV)                                                                                            \
@@ -939,6 +1020,8 @@ __global__ void __launch_bounds__(256) k_axpy_multi(size_t n, int nv, const doub
 // multiplied by sinv[0] (the inverse norm of v, formed on the device).
 __global__ void k_scale_to(size_t n, const double *__restrict__ v, double s, const double *__restrict__ sinv,
                            const double *__restrict__ scale, double *__restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   if (sinv) s *= sinv[0];
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
     out[c] = s * v[c] * scale[c];
@@ -952,18 +1035,22 @@ __global__ void k_scale_to(size_t n, const double *__restrict__ v, double s, con
 __global__ void __launch_bounds__(256) k_scale_to32(size_t n, const double *__restrict__ v, float s,
                                                     const float *__restrict__ sinv, const float *__restrict__ scale,
                                                     float *__restrict__ out, int split_nx) {
-  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
-  size_t o = c;
+  uint32_t o = c;
   if (split_nx > 0) {
-    const uint32_t i = (uint32_t)(c % (uint32_t)split_nx);
+    const uint32_t i = c % (uint32_t)split_nx;
     o = c - i + split_pos((int)i, split_nx);
   }
   out[o] = (float)v[c] * ((sinv ? s * sinv[0] : s) * scale[c]);
 }
-// ||V||^2 from the block partials into out[0], 1/||V|| into out[1] and
-// out32[0] (0 for a zero vector); one block
-__global__ void k_reduce_norm(const double *partial, int nb, double *out, float *out32) {
+// ||V||^2 from the block partials into out[0] and the host's copy norm2[0],
+// 1/||V|| into out[1] and out32[0] (0 for a zero vector); one block
+__global__ void k_reduce_norm(const double *partial, int nb, double *out, float *out32, double *norm2) {
+  pdl_trigger();
+  pdl_wait();
   double s = 0.;
   for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[q];
   s = block_sum(s);
@@ -972,6 +1059,7 @@ __global__ void k_reduce_norm(const double *partial, int nb, double *out, float 
     out[0] = s;
     out[1] = inv;
     out32[0] = (float)inv;
+    norm2[0] = s;
   }
 }
 // out = x (the V-cycle's result in FP32 or FP64, widened), one element per thread
@@ -979,11 +1067,13 @@ __global__ void k_reduce_norm(const double *partial, int nb, double *out, float 
 __global__ void __launch_bounds__(256) k_to64(size_t n, const float *__restrict__ x32,
                                               const double *__restrict__ x64, double *__restrict__ out,
                                               int split_nx) {
-  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
-  size_t o = c;
+  uint32_t o = c;
   if (x32 && split_nx > 0) {
-    const uint32_t i = (uint32_t)(c % (uint32_t)split_nx);
+    const uint32_t i = c % (uint32_t)split_nx;
     o = c - i + split_pos((int)i, split_nx);
   }
   out[c] = x32 ? (double)x32[o] : x64[c];
