@@ -161,16 +161,15 @@ LINE_FUSED_DECL(k_line_fused16_z)
 // offsets ox, ot, ob, orr; rows of rs words, columns at their split
 // positions), the operator too (oA) when it fits (res).
 constexpr int kTailLevels = 10, kTailThreads = 512, kTailDofs = 384;
-// FP32 works on units of 8 rows x 4 columns, one a warp at a time
-constexpr int kTailUnits = 4 * (kTailThreads / 32);
 struct TailLevel {
   Box b;
-  FastDiv dnh, dcw, dq, dP, dnq, dr4;  // by (nx + 1) / 2, cw, q, P, nq and the copies of an operator row
-  int cx, cy, cz;                      // coarsening to the next level
+  FastDiv dq, dP, dnu, dr4;  // by q, P, nu and the copies of an operator row
+  int cx, cy, cz;            // coarsening to the next level
   int q, res, rs;
-  int P, cw, nq;  // chunks of a j-line (at most 32), columns a warp takes (32 / P), column quads of a colour
+  int P, nu;  // chunks of a j-line, warps that the cells of a colour of one plane take (visit)
   const void *A, *D, *Asp, *inv, *cp, *w;  // FP32: A the packed couplings, D the diagonal; FP64: A the 19 planes
   const uint8_t *blank;
+  uint32_t ogh;  // the line recurrences' products of a lane's cells (0: not kept)
   uint32_t ox, ot, ob, orr, oA, obl;  // obl: blank flags (the first level: the CTA's planes; the others: all)
 };
 struct TailArgs {

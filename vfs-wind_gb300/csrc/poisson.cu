@@ -1398,14 +1398,12 @@ void tail_limits(vfs_poisson *h) {
 }
 
 // The tail kernel's arguments for the levels li .. coarsest; false when they
-// do not suit it.  Cells per CTA bound a phase's time: a colour of 256 cells a
-// CTA takes 2.6 us there and 4.2 us as a launch, one of 2048 cells 5 and 4.6
-// us, one of 3072 cells 9 and 5 us (FP64: 720 cells 7.5 and 9.5 us).  Solves
-// with limits of 0, 512, 2048, 4096 cells: 24x16x24 1525, 1321, 1220, 1210 us;
-// 64^3 2165, 1924, 1908, 1902; 128x96x128 6022, 5649, 5651, 5838; FP64
-// 72x40x56 6833, 6141, 6084, 6137.  A coarsest inverse of more than kTailDofs
-// rows is better spread over the whole chip.
-constexpr size_t kTailCells[2] = {2048, 2048};
+// do not suit it: a lane takes one cell of each colour at most, 16 warps a CTA
+// (24x16x24 cells need 12 and 32^3 would need 32: with two cells a lane there
+// a phase took 5 us, its launch 4.6), and a coarsest inverse of more than
+// kTailDofs rows is better spread over the whole chip.  Solves without and
+// with the tail: 24x16x24 1250 and 925 us, 64^3 1882 and 1629, 128x96x128
+// 5525 and 5230, FP64 72x40x56 6620 and 5795.
 template <typename T>
 bool tail_plan(vfs_poisson *h, int li, int nu1, int smoother, TailArgs *a, size_t *smem) {
   constexpr int p = std::is_same<T, double>::value;
@@ -1431,25 +1429,24 @@ bool tail_plan(vfs_poisson *h, int li, int nu1, int smoother, TailArgs *a, size_
     // FP32 rows of 4 (2 r + 1) words: 8 rows of 4 columns lie in 32 banks
     t.rs = p ? b.nx : ((b.nx + 3) / 4 | 1) * 4;
     t.b = b;
-    t.dnh.set((b.nx + 1) / 2);
     t.cx = l.cx; t.cy = l.cy; t.cz = l.cz;
     t.q = (b.nz + nc - 1) / nc;
     t.dq.set(t.q);
     t.res = 0;
     t.P = (b.ny + kLineChunk - 1) / kLineChunk;
-    t.nq = ((b.nx + 1) / 2 + 3) / 4;
-    if (t.P > 32 || (size_t)t.q * b.nx * b.ny > kTailCells[p] || (!p && t.q * t.nq * t.P > kTailUnits)) return false;
-    t.cw = 32 / t.P;
-    t.dcw.set(t.cw);
+    // up to 4 chunks of a column in one warp, else one chunk of 4 columns
+    const int nh = (b.nx + 1) / 2, cpw = t.P <= 4 ? 4 / t.P : 4;
+    t.nu = (nh + cpw - 1) / cpw * (t.P <= 4 ? 1 : t.P);
+    if (m < nl - 1 && t.q * t.nu > kTailThreads / 32) return false;
     t.dP.set(t.P);
-    t.dnq.set(t.nq);
+    t.dnu.set(t.nu);
     t.dr4.set(b.nx * sizeof(T) % 16 ? b.nx : (int)(b.nx * sizeof(T) / 16));
     t.blank = l.blank;
     const size_t slab = (size_t)t.rs * b.ny;
     t.obl = bytes(m ? b.n() : (size_t)t.q * b.nx * b.ny);
     t.ox = take((t.q + 2) * slab);
     t.ob = take(t.q * slab);
-    t.ot = t.orr = t.oA = 0;
+    t.ot = t.orr = t.oA = t.ogh = 0;
     t.A = t.D = t.Asp = t.inv = t.cp = t.w = nullptr;
     if (m == nl - 1) continue;
     t.ot = take((t.q + 2) * slab);
@@ -1472,6 +1469,11 @@ bool tail_plan(vfs_poisson *h, int li, int nu1, int smoother, TailArgs *a, size_
     if (used + words * sizeof(T) + 16 > h->tail_smem[p]) break;
     t.oA = take(words);
     t.res = 1;
+  }
+  for (int m = nl - 2; m >= 0; m--) {
+    TailLevel &t = a->lv[m];
+    const size_t words = (size_t)t.q * t.nu * 32 * 4;
+    if (t.P > 1 && used + words * sizeof(T) + 16 <= h->tail_smem[p]) t.ogh = take(words);
   }
   a->b = Prec<T>::v(h->L[li])[1];
   a->x = Prec<T>::v(h->L[li])[0];

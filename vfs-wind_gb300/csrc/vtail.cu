@@ -11,10 +11,8 @@
 // a border plane stores new values into its neighbour's copy of the plane too
 // (distributed shared memory), and every stencil read is local.  The
 // restriction and the prolongation read the few foreign planes they need in
-// their owner's memory.  What bounds a phase is latency: of 2.6 us at 16^3
-// cells, 1.0 are a cell's residual (one warp a quarter of an SM), 0.8 the
-// recurrences, 0.5 the stores, 0.3 the barrier.  Four levels from 24x16x24
-// cells on take 46 us instead of 95, three from 16^3 on 40 instead of 72.
+// their owner's memory.  What bounds a phase is the latency of one warp's
+// instructions (visit): 1.2-1.6 us, 0.3 of them the barrier.
 //
 // The arithmetic is that of the kernels it replaces, operation for operation
 // (k_residual16 / k_residual_f64, k_line_tri_*, k_restrict_*, k_prolong_*,
@@ -166,313 +164,257 @@ struct Halo {
   }
 };
 
-// The 19 values of cell (i, j, k) in slot order: columns of the parity of
-// (i + k) from xo, the others from xn.
+// The coefficients of a lane's cell: FP32 in registers, FP64 read at use.
 template <typename T>
-__device__ __forceinline__ void stencil_values(const Slab &v, const T *xo, const T *xn, int i, int j, int k,
-                                               T (&xs)[NSLOT]) {
-  const Box &b = v.l.b;
-  const int im = i > 0 ? i - 1 : (b.px ? b.nx - 1 : i), ip = i < b.nx - 1 ? i + 1 : (b.px ? 0 : i);
-  const int km = k > 0 ? k - 1 : (b.pz ? b.nz - 1 : k), kp = k < b.nz - 1 ? k + 1 : (b.pz ? 0 : k);
-  const int jm = j > 0 ? j - 1 : (b.py ? b.ny - 1 : j), jp = j < b.ny - 1 ? j + 1 : (b.py ? 0 : j);
-  const int s0 = v.slot(k), sl = v.slot_at(km, 0u), su = v.slot_at(kp, (uint32_t)(v.l.q + 1) * v.slab);
-  const int pc = (i & 1 ? v.nh : 0) + (i >> 1), pe = (ip & 1 ? v.nh : 0) + (ip >> 1), pw = (im & 1 ? v.nh : 0) + (im >> 1);
-  const int r0 = j * v.l.rs, rm = jm * v.l.rs, rp = jp * v.l.rs;
-  auto col = [&](int ii, int kk) { return ((ii + kk) ^ (i + k)) & 1 ? xn : xo; };
-  const T *c = xo + s0 + pc, *e = col(ip, k) + s0 + pe, *w = col(im, k) + s0 + pw, *t = col(i, kp) + su + pc,
-          *bt = col(i, km) + sl + pc;
-  xs[CP] = c[r0];
-  xs[EP] = e[r0];
-  xs[WP] = w[r0];
-  xs[NP] = c[rp];
-  xs[SP] = c[rm];
-  xs[TP] = t[r0];
-  xs[BP] = bt[r0];
-  xs[NE] = e[rp];
-  xs[SE] = e[rm];
-  xs[NW] = w[rp];
-  xs[SW] = w[rm];
-  xs[TN] = t[rp];
-  xs[BN] = bt[rp];
-  xs[TS] = t[rm];
-  xs[BS] = bt[rm];
-  xs[TE] = (col(ip, kp) + su + pe)[r0];
-  xs[BE] = (col(ip, km) + sl + pe)[r0];
-  xs[TW] = (col(im, kp) + su + pw)[r0];
-  xs[BW] = (col(im, km) + sl + pw)[r0];
-}
-
-// rhs - A x of a cell from its 19 values; FP32: the difference form over the
-// packed couplings, in the order of k_residual16.
-__device__ __forceinline__ float row_residual(const Op<float> &o, uint32_t row, float rhs, const float (&xs)[NSLOT]) {
-  const float xc = xs[CP];
-  float s = 0.f;
+struct Row;
+template <>
+struct Row<float> {
+  __half2 h[10];
+  float d;
+  __device__ __forceinline__ void load(const Op<float> &o, uint32_t at) {
 #pragma unroll
-  for (int m = 0; m < 9; m++) {
-    const float2 f = __half22float2(o.C[m * o.st + row]);
-    s = fmaf(f.x, xs[2 * m + 1] - xc, s);
-    s = fmaf(f.y, xs[2 * m + 2] - xc, s);
+    for (int m = 0; m < 10; m++) h[m] = o.C[m * o.st + at];
+    d = o.D[at];
   }
-  s = fmaf(__low2float(o.C[9 * o.st + row]), xc, s);
-  return fmaf(-o.D[row], s, rhs);
-}
-__device__ __forceinline__ double row_residual(const Op<double> &o, uint32_t row, double rhs,
-                                               const double (&xs)[NSLOT]) {
-  double s = 0.;
+  __device__ __forceinline__ float residual(const Op<float> &, uint32_t, float rhs, const float (&xs)[NSLOT]) const {
+    const float xc = xs[CP];
+    float s = 0.f;
 #pragma unroll
-  for (int m = 0; m < NSLOT; m++) s = fma(o.A[m * o.st + row], xs[m], s);
-  return rhs - s;
-}
+    for (int m = 0; m < 9; m++) {
+      const float2 f = __half22float2(h[m]);
+      s = fmaf(f.x, xs[2 * m + 1] - xc, s);
+      s = fmaf(f.y, xs[2 * m + 2] - xc, s);
+    }
+    s = fmaf(__low2float(h[9]), xc, s);
+    return fmaf(-d, s, rhs);
+  }
+};
+template <>
+struct Row<double> {
+  __device__ __forceinline__ void load(const Op<double> &, uint32_t) {}
+  __device__ __forceinline__ double residual(const Op<double> &o, uint32_t at, double rhs,
+                                             const double (&xs)[NSLOT]) const {
+    double s = 0.;
+#pragma unroll
+    for (int m = 0; m < NSLOT; m++) s = fma(o.A[m * o.st + at], xs[m], s);
+    return rhs - s;
+  }
+};
 
-// What a phase does with the cells of one colour: a sweep's colour (from a
-// zero guess: the residual is b), or the weighted residual that is restricted
-// (kWeighted1: the other colour's is zero).
-enum { kSweep, kSweepZero, kWeighted, kWeighted1 };
+// A lane's cell of one colour and what does not change during a stay on the
+// level: its place in an x-like vector and that of the columns beside it, the
+// right-hand side, the line's row (av, iv, cv), the products g, h of the line
+// recurrences over the chunk, and the restriction weight.
+template <typename T>
+struct Cell {
+  int pc, pe, pw;
+  bool in, eo, wo;  // eo, wo: the column beside has the cell's colour
+  T rhs, av, iv, cv, g, h, wt;
+  Row<T> row;
+};
 
-// FP32.  A unit is a chunk of 8 rows of 4 columns, one cell a lane: the
-// operator rows (stride 4 times an odd number of words) and the columns'
-// split positions make every read of the warp conflict-free, a unit's chunk
-// recurrences run through shuffles of its 8 lanes, and only the joins of a
-// column's chunks go through shared memory (ends).  One lane a chunk took
-// 2.4 times as long: 8 cells' worth of straight-line code for one warp.
-__device__ __noinline__ void phase32(const Slab &v, uint32_t oxo, uint32_t oxn, uint32_t oxd, float omega, int color,
-                                     int mode, float2 *ends) {
+// One stay on a level: `sweeps` sweeps from the vector at byte offset ox into
+// the one at ot, swapped each time, then with `weigh` the residual times the
+// restriction weight into r.
+// A lane has one cell of each colour at most.  A unit of 8 rows of a column
+// (a chunk of the line) takes 8 lanes, so that the chunk recurrences run
+// through shuffles; up to 4 chunks a column (P <= 4) lie in one warp and are
+// joined by shuffles, too, longer columns through shared memory (ends).
+// Operator rows are a multiple of 4 times an odd number of words apart and
+// columns at their split positions: reads of 8 rows of 4 columns meet no bank
+// conflict.
+// A phase costs the instructions that one warp needs for one cell, and the
+// first pass through them fetches them from L2: everything that does not
+// change is taken out of the loop (Cell), and the loop over phases holds one
+// copy of the code, the two colours' cells changing places.
+// A phase at 8^3 cells: 1.2 us (2.6 with addresses and coefficients formed in
+// each phase, 3.7 with a lane per chunk).
+template <typename T>
+__device__ __noinline__ void visit(const Slab &v, uint32_t ox, uint32_t ot, int sweeps, bool zero, bool weigh, bool half,
+                                   T omega, T *ends) {
+  constexpr uint32_t W = sizeof(T);
+  constexpr int NE = kTailThreads / 32 * 4;
+  auto cl = cg::this_cluster();
   const TailLevel &l = v.l;
-  const Op<float> o(v);
-  const float *xo = (const float *)(sm + oxo), *xn = (const float *)(sm + oxn), *bb = (const float *)(sm + l.ob);
-  float *own = (float *)(sm + (mode >= kWeighted ? l.orr : oxd + v.slab * 4u));
-  const int nx = l.b.nx, ny = l.b.ny, P = l.P, rs = l.rs, nh = v.nh, k0 = v.k0;
-  const int lane = threadIdx.x & 31, e = lane & 7, warp = threadIdx.x >> 5;
-  const int units = (v.k1 - k0) * l.nq * P;
-  struct Unit {
-    int kl, k, t, m, par, j, ch;
-  };
-  const FastDiv dP = l.dP, dnq = l.dnq;
-  const int nq = l.nq;
-  auto unit = [&](int u) {
-    Unit a;
-    const int rest = (int)dP.div(u);
-    a.ch = u - rest * P;
-    a.kl = (int)dnq.div(rest);
-    a.k = k0 + a.kl;
-    a.t = (rest - a.kl * nq) * 4 + (lane >> 3);
-    a.par = (color + a.k) & 1;
-    a.m = a.par ? nx - nh : nh;
-    a.j = a.ch * kLineChunk + e;
-    return a;
-  };
+  const Box &b = l.b;
+  const Op<T> o(v);
+  const int nx = b.nx, ny = b.ny, nz = b.nz, P = l.P, rs = l.rs, nh = v.nh, slab = (int)v.slab;
+  const int lane = threadIdx.x & 31, e = lane & 7, sub = lane >> 3, u = threadIdx.x >> 5;
+  // the warp's unit(s): columns cpw of nu / (planes) groups; chunk 0 of the
+  // lane's column in lanes 8 cb ..
+  const bool inwarp = P <= 4, active = u < v.planes() * l.nu;
+  const int cpw = inwarp ? 4 / P : 4, kl = active ? (int)l.dnu.div(u) : 0, k = v.k0 + kl, grp = u - kl * l.nu;
+  const int quad = inwarp ? grp : (int)l.dP.div(grp), ci = !inwarp || P == 1 ? sub : P == 2 ? sub >> 1 : 0;
+  const int cb = inwarp ? ci * P : 0, ch = inwarp ? min(sub - cb, P - 1) : grp - quad * P;
+  const int t = sub >= cpw * (inwarp ? P : 1) ? nx : quad * cpw + ci;
+  const int j = ch * kLineChunk + e, cnt = min(kLineChunk, ny - ch * kLineChunk), jc = min(j, ny - 1);
+  const int at0 = slab + (kl * ny + jc) * rs;  // the cell's row in an x-like vector
+  const int dm = ((jc > 0 ? jc - 1 : (b.py ? ny - 1 : jc)) - jc) * rs, dp = ((jc < ny - 1 ? jc + 1 : (b.py ? 0 : jc)) - jc) * rs;
+  const int km = k > 0 ? k - 1 : (b.pz ? nz - 1 : k), kp = k < nz - 1 ? k + 1 : (b.pz ? 0 : k);
+  const int dn = (int)v.slot_at(km, 0u) - (kl + 1) * slab, du = (int)v.slot_at(kp, (uint32_t)(l.q + 1) * v.slab) - (kl + 1) * slab;
+  // a neighbour has the cell's colour where a side clamps it onto the cell
+  // itself or an odd extent wraps
+  const bool to = !((kp ^ k) & 1), bo = !((km ^ k) & 1);
+  // the neighbours' copies, by byte offset in this CTA's memory: plane kl of
+  // a vector is their plane q + 1 or 0
+  const uint32_t base = smem_addr(sm);
+  const bool lo = active && v.lo >= 0 && kl == 0, hi = active && v.hi >= 0 && k == v.k1 - 1;
+  const uint32_t rlo = lo ? map_rank(base, v.lo) + (uint32_t)(l.q - kl) * v.slab * W : 0u,
+                 rhi = hi ? map_rank(base, v.hi) - (uint32_t)(kl + 1) * v.slab * W : 0u;
+  const uint32_t orow = (uint32_t)(kl * ny + jc) * o.rs;
+  T *ys = ends, *gs = ends + NE, *hs = ends + NE * 3;  // of the chunks: y, g and h per colour
+  Cell<T> A{}, B{};  // of the colour at work and of the other one
 #pragma unroll 1
-  for (int u = warp; u < units; u += kTailThreads / 32) {
-    const Unit a = unit(u);
-    const bool in = a.t < a.m && a.j < ny;
-    // (a lane without a cell reads another one's)
-    const int t = max(min(a.t, a.m - 1), 0), j = min(a.j, ny - 1), i = min(2 * t + a.par, nx - 1),
-              p = min(a.par ? nh + t : t, nx - 1), row = a.kl * ny + j, at = row * rs + p;
-    float y = bb[at];
-    float w = 0.f;
-    if (mode >= kWeighted) w = ((const float *)l.w)[(uint32_t)(k0 * ny + row) * nx + i];
-    if (mode != kSweepZero) {
-      float xs[NSLOT];
-      stencil_values<float>(v, xo, xn, i, j, a.k, xs);
-      y = row_residual(o, row * o.rs + p, y, xs);
-    }
-    if (mode >= kWeighted) y = mul_rn(y, w);
-    if (in) own[at] = y;
-    if (mode == kWeighted1 && a.j < ny && a.t < nx - a.m) own[row * rs + (a.par ? a.t : nh + a.t)] = 0.f;
-  }
-  if (mode >= kWeighted) return;
-  constexpr int U = kTailUnits / (kTailThreads / 32);
-  float y[U], g[U], c[U];
-#pragma unroll
-  for (int m = 0; m < U; m++) {
-    const int u = warp + m * (kTailThreads / 32);
-    if (u < units) {
-      const Unit a = unit(u);
-      const int t = max(min(a.t, a.m - 1), 0), j = min(a.j, ny - 1), p = min(a.par ? nh + t : t, nx - 1),
-                row = a.kl * ny + j, at = row * o.rs + p;
-      const float av = a.j > 0 ? o.S[at] : 0.f, iv = o.inv[at], r = own[row * rs + p];
-      c[m] = a.j < ny - 1 ? o.cp[at] : 0.f;
-      const float f = -av * iv;
-      float Y = (r - av * 0.f) * iv, G = f;
-#pragma unroll
-      for (int s = 1; s < kLineChunk; s++) {
-        const float yp = __shfl_up_sync(0xffffffffu, Y, 1, 8), gp = __shfl_up_sync(0xffffffffu, G, 1, 8);
-        if (e == s) {
-          Y = (r - av * yp) * iv;
-          G = gp * f;
-        }
-      }
-      y[m] = Y;
-      g[m] = G;
-      const int last = min(kLineChunk, ny - a.ch * kLineChunk) - 1;
-      if (P > 1 && e == last) ends[u * 4 + (lane >> 3)] = make_float2(Y, G);
-    }
-  }
-  if (P > 1) __syncthreads();
-#pragma unroll
-  for (int m = 0; m < U; m++) {
-    const int u = warp + m * (kTailThreads / 32);
-    if (u < units) {
-      const int ch = u - (int)dP.div(u) * P, cnt = min(kLineChunk, ny - ch * kLineChunk);
+  for (int c = 0; c < 2; c++) {
+    Cell<T> n{};
+    const int par = (c + k) & 1, m = par ? nx - nh : nh, tt = max(min(t, m - 1), 0);
+    n.in = active && t < m && j < ny;
+    const int i = min(2 * tt + par, nx - 1), im = i > 0 ? i - 1 : (b.px ? nx - 1 : i), ip = i < nx - 1 ? i + 1 : (b.px ? 0 : i);
+    const int p = split_pos(i, nx);
+    n.pc = at0 + p;
+    n.pe = at0 + split_pos(ip, nx);
+    n.pw = at0 + split_pos(im, nx);
+    n.eo = !((ip ^ i) & 1);
+    n.wo = !((im ^ i) & 1);
+    if (active) {
+      const uint32_t at = orow + p;
+      n.rhs = ((const T *)(sm + l.ob))[n.pc - slab];
+      n.av = j > 0 ? o.S[at] : (T)0;
+      n.iv = o.inv[at];
+      n.cv = j < ny - 1 ? o.cp[at] : (T)0;
+      n.row.load(o, at);
+      if (weigh && (c == 0 || !half)) n.wt = ((const T *)l.w)[(uint32_t)((v.k0 + kl) * ny + jc) * nx + i];
       if (P > 1) {
-        float Y = 0.f;
-        for (int s = 0; s < ch; s++) {
-          const float2 q = ends[(u - ch + s) * 4 + (lane >> 3)];
-          Y = q.x + q.y * Y;
+        // (the way down leaves the products for the way up where they fit)
+        T *keep = (T *)(sm + l.ogh) + ((size_t)c * l.q * l.nu * 32 + threadIdx.x) * 2;
+        T G = -n.av * n.iv, H = -n.cv;
+        if (l.ogh && !weigh) {
+          G = keep[0];
+          H = keep[1];
+        } else {
+          const T f = G;
+#pragma unroll 1
+          for (int s = 1; s < kLineChunk; s++) {  // (lane cnt - 1 starts h)
+            const T gp = __shfl_up_sync(0xffffffffu, G, 1, 8), hp = __shfl_down_sync(0xffffffffu, H, 1, 8);
+            if (e == s) G = gp * f;
+            if (e == kLineChunk - 1 - s && e < cnt - 1) H = hp * -n.cv;
+          }
+          if (l.ogh) {
+            keep[0] = G;
+            keep[1] = H;
+          }
         }
-        y[m] += g[m] * Y;
+        n.g = G;
+        n.h = H;
+        if (!inwarp && e == cnt - 1) gs[c * NE + u * 4 + sub] = G;
+        if (!inwarp && e == 0) hs[c * NE + u * 4 + sub] = H;
       }
-      const float r = y[m];
-      float X = r, H = -c[m];
+    }
+    A = B;
+    B = n;
+  }
+  // 2 sweeps phases, then the weighted residuals of the colours
+  const int phases = 2 * sweeps + (weigh ? 2 : 0);
+#pragma unroll 1
+  for (int ph = 0; ph < phases; ph++) {
+    const int c = ph & 1;
+    const bool solve = ph < 2 * sweeps, first = zero && ph == 0;
+    T y = A.rhs;
+    if (active && !first) {
+      const uint32_t on = solve && c ? ot : ox;
+      const T *xo = (const T *)(sm + ox), *xn = (const T *)(sm + on);
+      const T *C = xo + A.pc, *E = (A.eo ? xo : xn) + A.pe, *Wt = (A.wo ? xo : xn) + A.pw,
+              *Tp = (to ? xo : xn) + A.pc + du, *Bt = (bo ? xo : xn) + A.pc + dn;
+      const T xs[NSLOT] = {C[0], E[0], Wt[0], C[dp], C[dm], Tp[0], Bt[0], E[dp], E[dm], Wt[dp], Wt[dm], Tp[dp], Bt[dp],
+                           Tp[dm], Bt[dm], ((A.eo == to ? xo : xn) + A.pe + du)[0],
+                           ((A.eo == bo ? xo : xn) + A.pe + dn)[0], ((A.wo == to ? xo : xn) + A.pw + du)[0],
+                           ((A.wo == bo ? xo : xn) + A.pw + dn)[0]};
+      y = A.row.residual(o, orow + (uint32_t)(A.pc - at0), A.rhs, xs);
+    }
+    if (!solve) {
+      // (with omega 1 the second colour's lines were just solved: its residual
+      // is zero)
+      if (A.in) ((T *)(sm + l.orr))[A.pc - slab] = c && half ? (T)0 : mul_rn(y, A.wt);
+    } else {
+      if (active) {
+        const T r = y;
+        y = (r - A.av * (T)0) * A.iv;
 #pragma unroll
-      for (int s = kLineChunk - 2; s >= 0; s--) {
-        const float xp = __shfl_down_sync(0xffffffffu, X, 1, 8), hp = __shfl_down_sync(0xffffffffu, H, 1, 8);
-        if (e == s && s < cnt - 1) {
-          X = r - c[m] * xp;
-          H = hp * -c[m];
+        for (int q = 1; q < kLineChunk; q++) {
+          const T yp = __shfl_up_sync(0xffffffffu, y, 1, 8);
+          if (e == q) y = (r - A.av * yp) * A.iv;
+        }
+        if (inwarp) {
+          T Y = (T)0;
+          for (int q = 0; q < P - 1; q++) {
+            const int w = ((cb + q) * 8 + kLineChunk - 1) & 31;
+            const T ye = __shfl_sync(0xffffffffu, y, w), G = __shfl_sync(0xffffffffu, A.g, w);
+            if (q < ch) Y = ye + G * Y;
+          }
+          if (P > 1) y += A.g * Y;
+        } else if (e == cnt - 1) {
+          ys[u * 4 + sub] = y;
         }
       }
-      y[m] = X;
-      g[m] = H;
-    }
-  }
-  if (P > 1) {
-    __syncthreads();  // (ends is read above)
-#pragma unroll
-    for (int m = 0; m < U; m++) {
-      const int u = warp + m * (kTailThreads / 32);
-      if (u < units && e == 0) ends[u * 4 + (lane >> 3)] = make_float2(y[m], g[m]);
-    }
-    __syncthreads();
-  }
-  const Halo<float> halo(v, (const float *)(sm + oxd));
-#pragma unroll
-  for (int m = 0; m < U; m++) {
-    const int u = warp + m * (kTailThreads / 32);
-    if (u < units) {
-      const Unit a = unit(u);
-      if (P > 1) {
-        float X = 0.f;
-        for (int s = P - 1; s > a.ch; s--) {
-          const float2 q = ends[(u - a.ch + s) * 4 + (lane >> 3)];
-          X = q.x + q.y * X;
+      if (!inwarp) {
+        __syncthreads();
+        if (active) {
+          T Y = (T)0;
+          for (int q = 0; q < ch; q++) {
+            const int w = (u - ch + q) * 4 + sub;
+            Y = ys[w] + gs[c * NE + w] * Y;
+          }
+          y += A.g * Y;
         }
-        y[m] += g[m] * X;
+        __syncthreads();  // (ys is written again)
       }
-      if (a.t < a.m && a.j < ny) {
-        const uint32_t pl = (uint32_t)(a.j * rs + (a.par ? nh + a.t : a.t)), at = a.kl * v.slab + pl;
-        const float old = mode == kSweepZero ? 0.f : xo[v.slab + at], val = old + omega * y[m];
-        own[at] = val;
-        if (halo.lo && a.kl == 0) store_remote(halo.lo + pl * 4u, val);
-        if (halo.hi && a.k == v.k1 - 1) store_remote(halo.hi + pl * 4u, val);
-      }
-    }
-  }
-}
-
-// FP64.  A lane's FP64 operation holds its quarter of the SM for 64 cycles
-// whether 32 lanes work or one: the residuals are spread over all warps, one
-// lane a cell (r), and the lines over as few as hold them, one lane a chunk
-// of 8 cells, the P chunks of a column in lanes ch cw + c of one warp and
-// joined by shuffles.
-__device__ __noinline__ void phase64(const Slab &v, uint32_t oxo, uint32_t oxn, uint32_t oxd, double omega, int color,
-                                     int mode) {
-  constexpr int M = kLineChunk;
-  const TailLevel &l = v.l;
-  const Op<double> o(v);
-  const double *xo = (const double *)(sm + oxo), *xn = (const double *)(sm + oxn), *bb = (const double *)(sm + l.ob);
-  double *r = (double *)(sm + l.orr);
-  const int nx = l.b.nx, ny = l.b.ny, P = l.P, cw = l.cw, rs = l.rs, nh = v.nh, ncol = v.planes() * nh;
-  if (mode != kSweepZero) {
-    const uint32_t cells = (uint32_t)(v.planes() * ny * nh);
-    for (uint32_t q = threadIdx.x; q < cells; q += kTailThreads) {
-      const uint32_t row = l.dnh.div(q), kl = l.b.dy.div(row);
-      const int t = (int)(q - row * nh), j = (int)(row - kl * ny), k = v.k0 + (int)kl, par = (color + k) & 1;
-      if (t < (par ? nx - nh : nh)) {
-        const uint32_t p = par ? nh + t : t, at = row * rs + p;
-        double xs[NSLOT];
-        stencil_values<double>(v, xo, xn, 2 * t + par, j, k, xs);
-        double y = row_residual(o, row * o.rs + p, bb[at], xs);
-        if (mode >= kWeighted) y = mul_rn(y, ((const double *)l.w)[(uint32_t)(v.k0 * ny + row) * nx + 2 * t + par]);
-        r[at] = y;
-      }
-      if (mode == kWeighted1 && t < (par ? nh : nx - nh)) r[row * rs + (par ? t : nh + t)] = 0.;
-    }
-    if (mode >= kWeighted) return;
-    __syncthreads();
-  }
-  const double *rhs = mode == kSweepZero ? bb : r;
-  const int lane = threadIdx.x & 31, ch = (int)l.dcw.div((uint32_t)lane), c = lane - ch * cw, j0 = ch * M;
-  const Halo<double> halo(v, (const double *)(sm + oxd));
-  double *own = (double *)(sm + oxd);
-  for (int c0 = (int)(threadIdx.x >> 5) * cw; c0 < ncol; c0 += (kTailThreads / 32) * cw) {
-    const int col = min(c0 + c, ncol - 1), kl = (int)l.dnh.div((uint32_t)col), t = col - kl * nh, k = v.k0 + kl;
-    const int par = (color + k) & 1, m = par ? nx - nh : nh;
-    const int cnt = c0 + c < ncol && ch < P && t < m ? max(0, min(M, ny - j0)) : 0;
-    // (a lane without a chunk reads in bounds and stores nothing)
-    const int tt = max(min(t, m - 1), 0), p = min(par ? nh + tt : tt, nx - 1);
-    double y[M], iv[M], f[M], g[M];
-    double yp = 0., gp = 1.;
+      if (active) {
+        const T r = y;
 #pragma unroll
-    for (int e = 0; e < M; e++) {
-      const int row = kl * ny + min(j0 + e, ny - 1), at = row * o.rs + p;
-      f[e] = j0 + e > 0 ? o.S[at] : 0.;
-      iv[e] = o.inv[at];
-      y[e] = rhs[row * rs + p];
-    }
-#pragma unroll
-    for (int e = 0; e < M; e++) {
-      if (e < cnt) {
-        yp = (y[e] - f[e] * yp) * iv[e];
-        gp = gp * (-f[e] * iv[e]);
+        for (int q = kLineChunk - 2; q >= 0; q--) {
+          const T xp = __shfl_down_sync(0xffffffffu, y, 1, 8);
+          if (e == q && q < cnt - 1) y = r - A.cv * xp;
+        }
+        if (inwarp) {
+          T X = (T)0;
+          for (int q = P - 1; q > 0; q--) {
+            const int w = ((cb + q) * 8) & 31;
+            const T xe = __shfl_sync(0xffffffffu, y, w), H = __shfl_sync(0xffffffffu, A.h, w);
+            if (q > ch) X = xe + H * X;
+          }
+          if (P > 1) y += A.h * X;
+        } else if (e == 0) {
+          ys[u * 4 + sub] = y;
+        }
       }
-      y[e] = yp;
-      g[e] = gp;
-    }
-    if (P > 1) {
-      double Y = 0., in = 0.;
-      for (int s = 0; s < P; s++) {
-        const double ye = __shfl_sync(0xffffffffu, yp, s * cw + c), G = __shfl_sync(0xffffffffu, gp, s * cw + c);
-        if (s == ch) in = Y;
-        Y = ye + G * Y;
+      if (!inwarp) {
+        __syncthreads();
+        if (active) {
+          T X = (T)0;
+          for (int q = P - 1; q > ch; q--) {
+            const int w = (u - ch + q) * 4 + sub;
+            X = ys[w] + hs[c * NE + w] * X;
+          }
+          y += A.h * X;
+        }
       }
-#pragma unroll
-      for (int e = 0; e < M; e++) y[e] += g[e] * in;
-    }
-#pragma unroll
-    for (int e = 0; e < M; e++)
-      f[e] = j0 + e < ny - 1 ? o.cp[(kl * ny + min(j0 + e, ny - 1)) * o.rs + p] : 0.;
-    double xl = 0., hp = 1.;
-#pragma unroll
-    for (int e = M - 1; e >= 0; e--) {
-      if (e < cnt) {
-        xl = y[e] - f[e] * xl;
-        hp = hp * (-f[e]);
+      if (A.in) {
+        const T old = first ? (T)0 : ((const T *)(sm + ox))[A.pc], val = old + omega * y;
+        const uint32_t at = ot + (uint32_t)A.pc * W;
+        *(T *)(sm + at) = val;
+        if (lo) store_remote(rlo + at, val);
+        if (hi) store_remote(rhi + at, val);
       }
-      y[e] = xl;
-      g[e] = hp;
-    }
-    if (P > 1) {
-      double X = 0., in = 0.;
-      for (int s = P - 1; s >= 0; s--) {
-        const double xe = __shfl_sync(0xffffffffu, xl, s * cw + c), H = __shfl_sync(0xffffffffu, hp, s * cw + c);
-        if (s == ch) in = X;
-        X = xe + H * X;
-      }
-#pragma unroll
-      for (int e = 0; e < M; e++) y[e] += g[e] * in;
-    }
-    const bool lo = halo.lo && k == v.k0, hi = halo.hi && k == v.k1 - 1;
-#pragma unroll
-    for (int e = 0; e < M; e++) {
-      if (e < cnt) {
-        const uint32_t pl = (uint32_t)((j0 + e) * rs + p), at = v.slot(k) + pl;
-        const double val = (mode == kSweepZero ? 0. : xo[at]) + omega * y[e];
-        own[at] = val;
-        if (lo) store_remote(halo.lo + pl * 8u, val);
-        if (hi) store_remote(halo.hi + pl * 8u, val);
+      cl.sync();
+      if (c) {
+        const uint32_t q = ox;
+        ox = ot;
+        ot = q;
       }
     }
+    const Cell<T> q = A;
+    A = B;
+    B = q;
   }
 }
 
@@ -646,7 +588,7 @@ __device__ __forceinline__ void copy_operator(const Slab &v) {
 template <typename T>
 __device__ __forceinline__ void vtail_body(const TailArgs &a) {
   __shared__ __align__(16) unsigned char slabs[kTailLevels * sizeof(Slab)];
-  __shared__ float2 ends[sizeof(T) == 4 ? kTailUnits * 4 : 1];
+  __shared__ T ends[kTailThreads / 32 * 20];
   Slab *lv = (Slab *)slabs;
   auto cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
@@ -688,33 +630,9 @@ __device__ __forceinline__ void vtail_body(const TailArgs &a) {
   asm volatile("cp.async.wait_group 1;" ::: "memory");
   cl.sync();
   const T omega = (T)a.omega;
-  auto phase = [&](const Slab &v, uint32_t oxo, uint32_t oxn, uint32_t oxd, int color, int mode) {
-    if constexpr (sizeof(T) == 4) phase32(v, oxo, oxn, oxd, omega, color, mode, ends);
-    else phase64(v, oxo, oxn, oxd, omega, color, mode);
-  };
-  // one sweep of the vector at ox into the one at ot, which are then swapped
-  auto smooth = [&](const Slab &v, uint32_t &ox, uint32_t &ot, bool zero) {
-#pragma unroll 1
-    for (int color = 0; color < 2; color++) {
-      phase(v, ox, color ? ot : ox, ot, color, zero && !color ? kSweepZero : kSweep);
-      cl.sync();
-    }
-    const uint32_t u = ox;
-    ox = ot;
-    ot = u;
-  };
   for (int li = 0; li + 1 < a.nl; li++) {
     const Slab &v = lv[li], &c = lv[li + 1];
-    uint32_t ox = v.l.ox, ot = v.l.ot;
-    for (int s = 0; s < a.nu1; s++) smooth(v, ox, ot, s == 0);
-    // (with omega 1 the second colour's lines were just solved: its residual
-    // is zero)
-    if (a.nu1 > 0 && omega == (T)1) {
-      phase(v, ox, ox, 0u, 0, kWeighted1);
-    } else {
-      phase(v, ox, ox, 0u, 0, kWeighted);
-      phase(v, ox, ox, 0u, 1, kWeighted);
-    }
+    visit<T>(v, v.l.ox, v.l.ot, a.nu1, true, true, a.nu1 > 0 && omega == (T)1, omega, ends);
     clear((T *)(sm + c.l.ox), (uint32_t)(c.l.q + 2) * c.slab);
     if (li == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
     cl.sync();
@@ -728,13 +646,13 @@ __device__ __forceinline__ void vtail_body(const TailArgs &a) {
     const Slab &v = lv[li], &c = lv[li + 1];
     // the buffer that holds a level's x after s sweeps
     auto at = [&](const TailLevel &m, int s) { return s & 1 ? m.ot : m.ox; };
-    uint32_t ox = at(v.l, a.nu1), ot = at(v.l, a.nu1 + 1);
+    const uint32_t ox = at(v.l, a.nu1);
     prolong_phase<T>(v, c, li == 0, at(c.l, li + 2 == a.nl ? 0 : a.nu1 + a.nu2), ox);
     cl.sync();
-    for (int s = 0; s < a.nu2; s++) smooth(v, ox, ot, false);
+    visit<T>(v, ox, at(v.l, a.nu1 + 1), a.nu2, false, false, false, omega, ends);
     if (li == 0) {
       const TailLevel &l = v.l;
-      const T *x = (const T *)(sm + ox) + v.slab;
+      const T *x = (const T *)(sm + at(l, a.nu1 + a.nu2)) + v.slab;
       const uint32_t plane = (uint32_t)l.b.nx * l.b.ny, cells = (uint32_t)v.planes() * plane;
       T *out = (T *)a.x + (uint32_t)v.k0 * plane;
       for (uint32_t e = threadIdx.x; e < cells; e += kTailThreads) {
