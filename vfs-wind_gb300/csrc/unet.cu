@@ -8,8 +8,8 @@
 // box of a level (C a multiple of 16); gradients of activations are FP32.
 // Convolutions are implicit GEMMs on mma.sync m16n8k16 (A = 16 voxels along
 // x by 16 input channels of one tap, B = 16 input by 8 output channels):
-//   * k_conv: a CTA computes a 16x8x4 voxel tile for CT output channels; the
-//     input tile with its one-voxel halo (18x10x6 voxels x 16 channels) is
+//   * k_conv: a CTA computes a 16x8x4 (or 16x4x2) voxel tile for CT output
+//     channels; the input tile with its one-voxel halo x 16 channels is
 //     staged in shared memory one 16-channel group at a time, rows padded to
 //     48 bytes so that ldmatrix rows fall in distinct banks; weights are
 //     pre-packed in mma fragment order and read through L1.  The loader
@@ -46,6 +46,7 @@ constexpr int HX = TX + 2, HY = TY + 2, HZ = TZ + 2;         // with halo
 constexpr int HVOX = HX * HY * HZ;                           // 1080
 constexpr int ROWB = 48;                                     // 16 ch + pad, bytes
 constexpr int CONV_SMEM = HVOX * ROWB;                       // 51840
+constexpr int CONV_SMALL = 2 * HX * 6 * 4 * ROWB;            // two stages of the 16x4x2 tile
 constexpr int CONV_THREADS = 256;                            // 8 warps x 4 rows
 
 struct Src {
@@ -114,16 +115,75 @@ __device__ void load_group(const ConvGeom &G, int g, int x0, int y0, int z0, uns
   cp_async_wait_all();
 }
 
+// ldmatrix at a constant offset from a register
+template <int OFF>
+__device__ __forceinline__ void ldsm_x4_at(uint32_t *r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4 + %5];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr), "n"(OFF));
+}
+// The taps of a plane dz (dy, dx unrolled: every A row at a constant offset
+// of the warp's row addresses).
+template <int TAP, int HYV, int MT, int NT>
+__device__ __forceinline__ void conv_taps(float (&acc)[MT][NT][4], const uint32_t (&row)[MT], const uint2 *wp,
+                                          size_t tap_stride) {
+  constexpr int dz = TAP / 9, dy = (TAP / 3) % 3, dx = TAP % 3;
+  uint2 b[NT];
+#pragma unroll
+  for (int n = 0; n < NT; n++) b[n] = __ldg(wp + n * 32);
+#pragma unroll
+  for (int m = 0; m < MT; m++) {
+    uint32_t a[4];
+    ldsm_x4_at<((dz * HYV + dy) * HX + dx) * ROWB>(a, row[m]);
+#pragma unroll
+    for (int n = 0; n < NT; n++) mma_bf16(acc[m][n], a, b[n].x, b[n].y);
+  }
+  if constexpr (TAP < 26) conv_taps<TAP + 1, HYV, MT, NT>(acc, row, wp + tap_stride, tap_stride);
+}
+
+// Stage channel group g of the concatenated input around the output tile
+// origin (x0, y0, z0) into `tile` (rows of HX voxels, HYV x HZV of them); zeros
+// outside.  A warp takes whole rows, so that bounds in y and z and the row's
+// address are formed once for its 36 copies; the copies are one group.
+template <int HYV, int HZV>
+__device__ __forceinline__ void load_rows(const ConvGeom &G, int g, int x0, int y0, int z0, unsigned char *tile) {
+  const int g0 = G.s0.c / 16;
+  const bool first = g < g0;
+  const bf16 *p = first ? G.s0.p : G.s1.p;
+  const int C = first ? G.s0.c : G.s1.c, up = first ? G.s0.up : G.s1.up, coff = (first ? g : g - g0) * 16;
+  const int sx = up ? G.nx / 2 : G.nx, sy = up ? G.ny / 2 : G.ny, lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < HYV * HZV; r += CONV_THREADS / 32) {
+    const int hy = r % HYV, hz = r / HYV, gy = y0 - 1 + hy, gz = z0 - 1 + hz;
+    const bool in = gy >= 0 && gz >= 0 && gy < G.ny && gz < G.nz;
+    const bf16 *src = p + ((size_t)(gz >> up) * sy + (gy >> up)) * sx * C + coff;
+    unsigned char *dst = tile + r * HX * ROWB;
+    for (int q = lane; q < HX * 2; q += 32) {
+      const int v = q >> 1, half = q & 1, gx = x0 - 1 + v;
+      unsigned char *d = dst + v * ROWB + half * 16;
+      if (!in || gx < 0 || gx >= G.nx) *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
+      else cp_async16(smem_u32(d), src + (size_t)(gx >> up) * C + half * 8);
+    }
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+}
+
 // Forward (FWD: + bias, ReLU, BF16 out) or data-gradient (FP32 out split
-// into two destinations at channel `split`) 3x3x3 convolution.
-template <int CT, bool FWD>
-__global__ void __launch_bounds__(CONV_THREADS) k_conv(ConvGeom G, const uint2 *__restrict__ wpk,
+// into two destinations at channel `split`) 3x3x3 convolution.  Tiles of
+// 16 x TYV x TZV voxels; STAGES 2: the next channel group is on its way while
+// the present one is multiplied.
+// Bound by issue: a tap of an m-tile is one ldmatrix and NT mma since their
+// addresses are constants (with addresses formed at run time and a division
+// per staged voxel a 16-channel layer of 64^3 voxels took 20.2 us, now 15.5: 234
+// TFLOP/s, about what mma.sync gives here).
+template <int CT, bool FWD, int TYV, int TZV, int STAGES>
+__global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(ConvGeom G, const uint2 *__restrict__ wpk,
                                                        const float *__restrict__ bias, int relu, bf16 *out_b,
                                                        float *out0, float *out1, int split) {
   extern __shared__ __align__(16) unsigned char tile[];
-  constexpr int NT = CT / 8, MT = 4;
+  constexpr int NT = CT / 8, MT = TYV * TZV / (CONV_THREADS / 32), HYV = TYV + 2, HZV = TZV + 2;
+  constexpr int TILE = HX * HYV * HZV * ROWB;
   const int tiles_x = (G.nx + TX - 1) / TX;
-  const int x0 = (blockIdx.x % tiles_x) * TX, y0 = (blockIdx.x / tiles_x) * TY, z0 = blockIdx.y * TZ;
+  const int x0 = (blockIdx.x % tiles_x) * TX, y0 = (blockIdx.x / tiles_x) * TYV, z0 = blockIdx.y * TZV;
   const int slice = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float acc[MT][NT][4];
@@ -132,32 +192,34 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv(ConvGeom G, const uint2 *
 #pragma unroll
     for (int n = 0; n < NT; n++) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
   const uint32_t tbase = smem_u32(tile);
+  load_rows<HYV, HZV>(G, 0, x0, y0, z0, tile);
   for (int g = 0; g < G.groups; g++) {
+    const int buf = STAGES == 2 ? g & 1 : 0;
+    if (STAGES == 2 && g + 1 < G.groups) {
+      load_rows<HYV, HZV>(G, g + 1, x0, y0, z0, tile + (buf ^ 1) * TILE);
+      asm volatile("cp.async.wait_group 1;\n" ::);
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::);
+    }
     __syncthreads();
-    load_group(G, g, x0, y0, z0, tile);
-    __syncthreads();
-    for (int tap = 0; tap < 27; tap++) {
-      const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;  // halo offsets 0..2
-      uint2 b[NT];
-      const uint2 *wp = wpk + ((size_t)(tap * G.groups + g) * G.nt_tot + slice * NT) * 32 + lane;
+    uint32_t row[MT];
 #pragma unroll
-      for (int n = 0; n < NT; n++) b[n] = __ldg(wp + n * 32);
-#pragma unroll
-      for (int m = 0; m < MT; m++) {
-        const int r = warp * MT + m, yy = r % TY, zz = r / TY;
-        const int hv = ((zz + dz) * HY + (yy + dy)) * HX + (lane & 15) + dx;
-        uint32_t a[4];
-        ldsm_x4(a, tbase + hv * ROWB + (lane >> 4) * 16);
-#pragma unroll
-        for (int n = 0; n < NT; n++) mma_bf16(acc[m][n], a, b[n].x, b[n].y);
-      }
+    for (int m = 0; m < MT; m++) {
+      const int r = warp * MT + m, yy = r % TYV, zz = r / TYV;
+      row[m] = tbase + buf * TILE + ((zz * HYV + yy) * HX + (lane & 15)) * ROWB + (lane >> 4) * 16;
+    }
+    conv_taps<0, HYV, MT, NT>(acc, row, wpk + ((size_t)g * G.nt_tot + slice * NT) * 32 + lane,
+                              (size_t)G.groups * G.nt_tot * 32);
+    if (g + 1 < G.groups) {
+      __syncthreads();
+      if (STAGES == 1) load_rows<HYV, HZV>(G, g + 1, x0, y0, z0, tile);
     }
   }
   // epilogue: rows lane/4 and lane/4 + 8 of each m-tile, channels pairs
   const int cout = G.nt_tot * 8;
 #pragma unroll
   for (int m = 0; m < MT; m++) {
-    const int r = warp * MT + m, y = y0 + r % TY, z = z0 + r / TY;
+    const int r = warp * MT + m, y = y0 + r % TYV, z = z0 + r / TYV;
     if (y >= G.ny || z >= G.nz) continue;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -180,6 +242,26 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv(ConvGeom G, const uint2 *
         }
       }
     }
+  }
+}
+
+// Tiles of 16x8x4 voxels and the widest channel slice while they fill the
+// chip (two CTAs a SM), else tiles of 16x4x2 and slices of 16: eight times as
+// many CTAs of a quarter of a warp's work (32^3 voxels of 32 channels had 64
+// CTAs on 152 SMs, 16^3 of 64 had 16: the 11 such convolutions of a training
+// step took 332 us, now 175).
+template <bool FWD>
+void launch_conv(cudaStream_t st, const ConvGeom &G, const uint2 *w, const float *bias, bf16 *out_b, float *out0,
+                 float *out1, int split) {
+  const int cout = G.nt_tot * 8, tx = (G.nx + TX - 1) / TX;
+  const bool wide = cout % 32 == 0;
+  const dim3 big(tx * ((G.ny + TY - 1) / TY), (G.nz + TZ - 1) / TZ, cout / (wide ? 32 : 16));
+  if ((size_t)big.x * big.y * big.z >= 304) {
+    if (wide) k_conv<32, FWD, TY, TZ, 1><<<big, CONV_THREADS, CONV_SMEM, st>>>(G, w, bias, 1, out_b, out0, out1, split);
+    else k_conv<16, FWD, TY, TZ, 1><<<big, CONV_THREADS, CONV_SMEM, st>>>(G, w, bias, 1, out_b, out0, out1, split);
+  } else {
+    const dim3 small(tx * ((G.ny + 3) / 4), (G.nz + 1) / 2, cout / 16);
+    k_conv<16, FWD, 4, 2, 2><<<small, CONV_THREADS, CONV_SMALL, st>>>(G, w, bias, 1, out_b, out0, out1, split);
   }
 }
 
@@ -671,8 +753,8 @@ int configure_kernels() {
   std::lock_guard<std::mutex> lk(cfg_mu);
   if (kernels_configured) return VFS_OK;
   const int wg = CONV_SMEM + TX * TY * TZ * 16;  // + gradient tile rows of (2 COUT + 16) bytes
-  bool ok = smem_attr(k_conv<16, true>, CONV_SMEM) && smem_attr(k_conv<32, true>, CONV_SMEM) &&
-            smem_attr(k_conv<16, false>, CONV_SMEM) && smem_attr(k_conv<32, false>, CONV_SMEM) &&
+  bool ok = smem_attr(k_conv<16, true, TY, TZ, 1>, CONV_SMEM) && smem_attr(k_conv<32, true, TY, TZ, 1>, CONV_SMEM) &&
+            smem_attr(k_conv<16, false, TY, TZ, 1>, CONV_SMEM) && smem_attr(k_conv<32, false, TY, TZ, 1>, CONV_SMEM) &&
             smem_attr(k_wgrad<16>, wg + TX * TY * TZ * 32) && smem_attr(k_wgrad<32>, wg + TX * TY * TZ * 64) &&
             smem_attr(k_wgrad<64>, wg + TX * TY * TZ * 128);
   if (!ok) {
@@ -693,21 +775,9 @@ ConvGeom geom(const Conv &c, int nx, int ny, int nz, const bf16 *s0, const bf16 
   return G;
 }
 
-dim3 conv_grid(int nx, int ny, int nz, int slices) {
-  return dim3(((nx + TX - 1) / TX) * ((ny + TY - 1) / TY), (nz + TZ - 1) / TZ, slices);
-}
-
 void conv_fwd(vfs_unet *u, int li, int nx, int ny, int nz, const bf16 *s0, const bf16 *s1, bf16 *out) {
   const Conv &c = u->conv[li];
-  ConvGeom G = geom(c, nx, ny, nz, s0, s1);
-  const uint2 *w = u->pk + c.pk;
-  const float *b = u->params + c.b;
-  if (c.cout % 32 == 0)
-    k_conv<32, true><<<conv_grid(nx, ny, nz, c.cout / 32), CONV_THREADS, CONV_SMEM, u->stream>>>(
-        G, w, b, 1, out, nullptr, nullptr, 0);
-  else
-    k_conv<16, true><<<conv_grid(nx, ny, nz, c.cout / 16), CONV_THREADS, CONV_SMEM, u->stream>>>(
-        G, w, b, 1, out, nullptr, nullptr, 0);
+  launch_conv<true>(u->stream, geom(c, nx, ny, nz, s0, s1), u->pk + c.pk, u->params + c.b, out, nullptr, nullptr, 0);
   u->launches++;
 }
 
@@ -716,14 +786,7 @@ void conv_fwd(vfs_unet *u, int li, int nx, int ny, int nz, const bf16 *s0, const
 void conv_dgrad(vfs_unet *u, int li, int nx, int ny, int nz, const bf16 *gp, float *d0, float *d1) {
   const Conv &c = u->conv[li];
   Conv t{c.cout, c.cin, c.cout, 0, 0, 0, 0, 0, 0};
-  ConvGeom G = geom(t, nx, ny, nz, gp, nullptr);
-  const uint2 *w = u->pk + c.pkt;
-  if (c.cin % 32 == 0)
-    k_conv<32, false><<<conv_grid(nx, ny, nz, c.cin / 32), CONV_THREADS, CONV_SMEM, u->stream>>>(
-        G, w, nullptr, 0, nullptr, d0, d1, c.c0);
-  else
-    k_conv<16, false><<<conv_grid(nx, ny, nz, c.cin / 16), CONV_THREADS, CONV_SMEM, u->stream>>>(
-        G, w, nullptr, 0, nullptr, d0, d1, c.c0);
+  launch_conv<false>(u->stream, geom(t, nx, ny, nz, gp, nullptr), u->pk + c.pkt, nullptr, nullptr, d0, d1, c.c0);
   u->launches++;
 }
 
