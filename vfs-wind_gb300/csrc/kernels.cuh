@@ -226,7 +226,11 @@ __global__ void k_gs_reduce(const double *partial, int nb, int nv, double *red);
 __global__ void k_gs_coef(int nv, double *red);
 __global__ void k_gs_update(size_t n, int nv, const double *const *Q, const double *red, double *u, double *w,
                             double *partial);
-__global__ void k_axpy_multi(size_t n, int nv, const double *const *Z, const double *coef, double *x);
+struct AxpyCoef {
+  double c[64];
+};
+__global__ void k_axpy_multi(size_t n, int nv, const double *const *Z, const __grid_constant__ AxpyCoef coef,
+                             double *x);
 __global__ void k_scale_to(size_t n, const double *v, double s, const double *sinv, const double *scale,
                            double *out);
 __global__ void k_scale_to32(size_t n, const double *v, float s, const float *sinv, const float *scale, float *out,
@@ -234,6 +238,8 @@ __global__ void k_scale_to32(size_t n, const double *v, float s, const float *si
 __global__ void k_reduce_norm(const double *partial, int nb, double *out, float *out32, double *norm2);
 __global__ void k_to64(size_t n, const float *x32, const double *x64, double *out, int split_nx);
 __global__ void k_sumsq(size_t n, const double *x, double *partial);
+__global__ void k_sumsq_copy(size_t n, const double *x, double *partial, double *copy);
+__global__ void k_first_norm(const double *partial, int nb, double *out, float *out32, double *norm2);
 // history projection of the initial guess (at most kHistMax solutions:
 // the newest and the differences of consecutive ones)
 constexpr int kHistMax = 12;

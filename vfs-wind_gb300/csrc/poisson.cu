@@ -473,7 +473,7 @@ struct vfs_poisson {
   double **dV = nullptr, **dZ = nullptr;
   // dsv[2q] = ||V_q||^2 and dsv[2q+1] = 1 / ||V_q||; dsv32[q] the latter in FP32
   double *fsum = nullptr;  // over the fluid cells of the mask: sum of aj, count
-  double *partial = nullptr, *red = nullptr, *coef = nullptr, *dsv = nullptr;
+  double *partial = nullptr, *red = nullptr, *dsv = nullptr;
   float *dsv32 = nullptr;
   size_t partial_len = 0;
   double *hbuf = nullptr;  // pinned host readback
@@ -567,6 +567,8 @@ struct vfs_poisson {
   // the solve's copy of phi to a host array, beside the history push
   cudaStream_t dl_stream = nullptr;
   cudaEvent_t dl_ev[2] = {nullptr, nullptr};
+  cudaEvent_t it_ev = nullptr;  // end of the results a solve's host waits for
+  bool phi_queued = false;      // phi_da of the solve's x is formed (queue_phi)
   double *spartial = nullptr, *sred = nullptr;  // side-stream reductions
   bool spec_enable = true;                      // VFS_GUESS_SPECULATE=0 turns it off
   bool spec_next = false, spec_valid = false;
@@ -1644,8 +1646,7 @@ void prof_collect(vfs_poisson *h) {
 
 // reduce `nrow` rows of `nb` partials on the device and read them back
 int reduce_read(vfs_poisson *h, int nb, int nrow, double *out) {
-  LAUNCH(h, k_reduce_rows, nrow, 1024, h->partial, nb, nrow, h->red);
-  CUDA_TRY(cudaMemcpyAsync(h->hbuf, h->red, nrow * 8, cudaMemcpyDeviceToHost, h->stream));
+  LAUNCH(h, k_reduce_rows, nrow, 1024, h->partial, nb, nrow, h->hbuf);
   TRY(sync(h));
   for (int q = 0; q < nrow; q++) out[q] = h->hbuf[q];
   return VFS_OK;
@@ -1654,12 +1655,31 @@ int reduce_read(vfs_poisson *h, int nb, int nrow, double *out) {
 // r = b - A x in FP64 and ||r||: the residual kernel without a reduction,
 // then the fixed-shape sum of squares (faster than block partials formed in
 // the stencil kernel, whose barriers hold its loads back)
-int residual_norm(vfs_poisson *h, const double *x, double *r, double *norm) {
+// (residual_queue: launched only; ||r||^2 arrives in hbuf[0])
+int residual_queue(vfs_poisson *h, const double *x, double *r) {
   LAUNCH(h, k_residual64r, box_grid(h->box), 128, h->box, h->A0, x, h->b, r);
   LAUNCH(h, k_sumsq, kRedBlocks, 256, h->box.n(), r, h->partial);
-  double s;
-  TRY(reduce_read(h, kRedBlocks, 1, &s));
-  *norm = std::sqrt(s);
+  LAUNCH(h, k_reduce_rows, 1, 1024, h->partial, kRedBlocks, 1, h->hbuf);
+  return VFS_OK;
+}
+int residual_norm(vfs_poisson *h, const double *x, double *r, double *norm) {
+  TRY(residual_queue(h, x, r));
+  TRY(sync(h));
+  *norm = std::sqrt(h->hbuf[0]);
+  return VFS_OK;
+}
+
+// phi_da from x: Remove_Nullspace of phi (Source/poisson_hypre.c:604-608), its
+// shift applied by the DA output
+int queue_phi(vfs_poisson *h) {
+  const size_t n = h->box.n();
+  const bool shift = h->desc.bctype3 != -10 && !(h->ls_on && h->ls_bc5 == 4);
+  if (shift) {
+    LAUNCH(h, k_mean_partial, kRedBlocks, 256, n, h->fluid, h->x, h->partial);
+    LAUNCH(h, k_mean_shift, 1, 1024, h->partial, kRedBlocks, h->fsum, h->red);
+  }
+  LAUNCH(h, k_box_to_da_phi, lin_grid(h->g.n()), 256, h->g, h->box, h->rowtype0, h->fluid, h->x, h->phi_da,
+         shift ? (const double *)h->red : nullptr);
   return VFS_OK;
 }
 
@@ -2005,12 +2025,11 @@ int ensure_krylov(vfs_poisson *h, int m) {
   const size_t n = h->box.n();
   for (int q = 0; q <= m; q++) TRY(dalloc(h, &h->V[q], n));
   for (int q = 0; q < m; q++) TRY(dalloc(h, &h->Z[q], n));
-  dfree(h, h->dV); dfree(h, h->dZ); dfree(h, h->coef); dfree(h, h->dsv); dfree(h, h->dsv32);
+  dfree(h, h->dV); dfree(h, h->dZ); dfree(h, h->dsv); dfree(h, h->dsv32);
   TRY(dalloc(h, &h->dsv, 2 * (m + 1)));
   TRY(dalloc(h, &h->dsv32, m + 1));
   TRY(dalloc(h, &h->dV, m + 1));
   TRY(dalloc(h, &h->dZ, m));
-  TRY(dalloc(h, &h->coef, m + 1));
   CUDA_TRY(cudaMemcpyAsync(h->dV, h->V.data(), (m + 1) * sizeof(double *), cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(cudaMemcpyAsync(h->dZ, h->Z.data(), m * sizeof(double *), cudaMemcpyHostToDevice, h->stream));
   if (h->hbuf) cudaFreeHost(h->hbuf);
@@ -2062,6 +2081,8 @@ void cgs_dots(vfs_poisson *h, int nv, int nb, size_t n, int v0, const double *w)
 // hbuf offsets: the read-back of the speculative step 0 and its staging of
 // the first basis norm (apart from the rows reduce_read and FGMRES use)
 constexpr int kSpecHb = 620, kSpecStage = 610;
+// hbuf offset of ||b||^2 of a solve from zero
+constexpr int kFirstNorm = 600;
 
 // Enqueue Arnoldi step jj of FGMRES: precondition V_jj (unless Z_jj holds it
 // already: have_z), apply A, orthogonalise (orth 0 or DCGS2), reduce the new
@@ -2069,11 +2090,12 @@ constexpr int kSpecHb = 620, kSpecStage = 610;
 // hb + 0..jj; the norm^2 at hb + kGsR + 3), written there by the kernels
 // (pinned memory).  With orth 0 the whole step is one chain of dependent
 // launches.
-int arnoldi_enqueue(vfs_poisson *h, int jj, int nbd, const vfs_solve_opts &o, int hb, bool have_z = false) {
+int arnoldi_enqueue(vfs_poisson *h, int jj, int nbd, const vfs_solve_opts &o, int hb, bool have_z = false,
+                    bool z_last = false) {
   const size_t n = h->box.n();
   const double *const *dV = (const double *const *)h->dV;
   if (!have_z) TRY(precondition(h, h->V[jj], 1.0, h->dsv + 2 * jj + 1, h->dsv32 + jj, h->Z[jj], o));
-  else h->pdl_prev = false;
+  else if (!z_last) h->pdl_prev = false;  // (z_last: forming Z_jj was the last thing launched)
   auto stamp = [&](int q) {
     if (!h->phase || hb != 0) return;
     cudaEventRecord(h->phev[q], h->stream);
@@ -2110,6 +2132,10 @@ int arnoldi_enqueue(vfs_poisson *h, int jj, int nbd, const vfs_solve_opts &o, in
 // V-cycles with opts.nu2_near post sweeps.
 constexpr double kNearStart = 32.;
 
+// The reduction a solve's first step is taken to reach at best, where the
+// next V-cycle is launched ahead.
+constexpr double kFirstGain = 0.02;
+
 // The options of a solve that may resume from the speculative step 0: the
 // same preconditioner and orthogonalisation.
 bool spec_matches(const vfs_solve_opts &a, const vfs_solve_opts &b) {
@@ -2144,12 +2170,25 @@ int fgmres(vfs_poisson *h, const vfs_solve_opts &oin, vfs_solve_stats *st) {
   if (m > h->m_alloc) h->spec_valid = h->z0_valid = false;
   TRY(ensure_krylov(h, m));
   const int nbd = (int)((n + 256 * kGsTile - 1) / (256 * kGsTile));
-  double bn2;
-  LAUNCH(h, k_sumsq, kRedBlocks, 256, n, h->b, h->partial);
-  TRY(reduce_read(h, kRedBlocks, 1, &bn2));
-  const double bn = std::sqrt(bn2);
+  // A solve from zero that has steps to do starts on the device: V_0 = b, its
+  // norm stays there and the first step is launched before the host knows it
+  // (bn < 0 until the first step's wait; the relative residual is 1).
+  const bool from_zero = !o.warm_start && 1. > o.rtol;
+  double bn = -1.;
+  if (from_zero) {
+    LAUNCH(h, k_sumsq_copy, kRedBlocks, 256, n, h->b, h->partial, h->V[0]);
+    LAUNCH(h, k_first_norm, 1, 1024, h->partial, kRedBlocks, h->dsv, h->dsv32, h->hbuf + kFirstNorm);
+  } else {
+    double bn2;
+    LAUNCH(h, k_sumsq, kRedBlocks, 256, n, h->b, h->partial);
+    TRY(reduce_read(h, kRedBlocks, 1, &bn2));
+    bn = std::sqrt(bn2);
+  }
   int it = 0;
   double rel = 0., beta = 0.;
+  h->phi_queued = false;
+  // what the host does not wait for ahead of time: profiled solves are timed step by step
+  const bool ahead = !h->phase && !h->prof;
   // Hraw: Hessenberg columns as formed; R: the same after the Givens rotations
   std::vector<double> Hraw((size_t)(m + 1) * m, 0.), R((size_t)(m + 1) * m, 0.), cs(m), sn(m), gv(m + 1),
       gsave(m + 1), y(m);
@@ -2173,11 +2212,11 @@ int fgmres(vfs_poisson *h, const vfs_solve_opts &oin, vfs_solve_stats *st) {
     beta = h->r0_norm;
   } else if (o.warm_start) {
     TRY(residual_norm(h, h->x, h->V[0], &beta));
-  } else {  // zero initial guess: r = b
+  } else if (!from_zero) {  // zero initial guess: r = b
     CUDA_TRY(cudaMemcpyAsync(h->V[0], h->b, n * 8, cudaMemcpyDeviceToDevice, h->stream));
     beta = bn;
   }
-  rel = beta / bn;
+  rel = from_zero ? 1. : beta / bn;
   st->initial_rel_residual = rel;
   if (o.nu2_near > 0 && rel <= kNearStart * o.rtol) o.nu2 = o.nu2_near;
   // rotate the formed column j by rotations 0..j-1, form rotation j and
@@ -2198,24 +2237,49 @@ int fgmres(vfs_poisson *h, const vfs_solve_opts &oin, vfs_solve_stats *st) {
     gv[j + 1] = -sn[j] * gv[j];
     gv[j] = cs[j] * gv[j];
   };
+  double gain = 2. * kFirstGain;  // the largest reduction of the estimate by one step so far
   while (rel > o.rtol && it < o.max_it) {
-    h->hbuf[400] = beta * beta;  // pinned staging: pageable copies cost ~0.5 ms each
-    h->hbuf[401] = 1.0 / beta;
-    reinterpret_cast<float *>(h->hbuf + 402)[0] = (float)(1.0 / beta);
-    CUDA_TRY(cudaMemcpyAsync(h->dsv, h->hbuf + 400, 16, cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(h->dsv32, h->hbuf + 402, 4, cudaMemcpyHostToDevice, h->stream));
+    h->phi_queued = false;
+    if (bn >= 0.) {
+      h->hbuf[400] = beta * beta;  // pinned staging: pageable copies cost ~0.5 ms each
+      h->hbuf[401] = 1.0 / beta;
+      reinterpret_cast<float *>(h->hbuf + 402)[0] = (float)(1.0 / beta);
+      CUDA_TRY(cudaMemcpyAsync(h->dsv, h->hbuf + 400, 16, cudaMemcpyHostToDevice, h->stream));
+      CUDA_TRY(cudaMemcpyAsync(h->dsv32, h->hbuf + 402, 4, cudaMemcpyHostToDevice, h->stream));
+    }
     std::fill(gv.begin(), gv.end(), 0.);
     std::fill(Hraw.begin(), Hraw.end(), 0.);
     gv[0] = beta;
     int jj = 0;
+    bool have_z = have_z0 && it == 0, z_last = false;
     for (; jj < m && it < o.max_it; jj++) {
       const auto t0 = h->phase ? std::chrono::steady_clock::now() : std::chrono::steady_clock::time_point();
       if (h->phase) cudaEventRecord(h->phev[0], h->stream);
       const bool pre = resume && it == 0 && jj == 0;  // enqueued by the guess
       const int hb = pre ? kSpecHb : 0;
-      if (!pre) TRY(arnoldi_enqueue(h, jj, nbd, o, 0, have_z0 && it == 0 && jj == 0));
+      if (!pre) TRY(arnoldi_enqueue(h, jj, nbd, o, 0, have_z, z_last));
       const auto t2 = h->phase ? std::chrono::steady_clock::now() : t0;
-      TRY(sync(h));
+      // The next step's V-cycle goes to the device before the host has this
+      // step's estimate, unless this step may be the last one: twice the
+      // largest reduction by a step so far (kFirstGain at first) would end the
+      // solve.  A wrong guess costs that V-cycle and changes nothing: Z_{jj+1}
+      // is formed anew or not used.
+      const double before = bn < 0. ? 1. : std::fabs(gv[jj]) / bn;
+      have_z = z_last = ahead && !pre && jj + 1 < m && it + 1 < o.max_it && before * (0.5 * gain) > o.rtol;
+      if (have_z) {
+        CUDA_TRY(cudaEventRecord(h->it_ev, h->stream));
+        TRY(precondition(h, h->V[jj + 1], 1.0, h->dsv + 2 * jj + 3, h->dsv32 + jj + 1, h->Z[jj + 1], o));
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaEventSynchronize(h->it_ev));
+      } else {
+        TRY(sync(h));
+      }
+      if (bn < 0.) {
+        gv[0] = beta = bn = std::sqrt(h->hbuf[kFirstNorm]);
+        rel = bn == 0. ? 0. : beta / bn;
+        st->initial_rel_residual = st->rel_residual = rel;
+        if (!(rel > o.rtol)) return VFS_OK;  // b is zero or not finite: x stays zero
+      }
       const auto t3 = h->phase ? std::chrono::steady_clock::now() : t0;
       if (h->phase && !pre) {
         h->host_ms[0] += std::chrono::duration<double, std::milli>(t2 - t0).count();
@@ -2250,17 +2314,30 @@ int fgmres(vfs_poisson *h, const vfs_solve_opts &oin, vfs_solve_stats *st) {
       Hraw[(size_t)(jj + 1) * m + jj] = wn;
       rotate(jj);
       if (h->phase) h->host_ms[3] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-      if (std::fabs(gv[jj + 1]) / bn <= o.rtol || wn == 0.) { jj++; break; }
+      const double after = std::fabs(gv[jj + 1]) / bn;
+      if (before > 0.) gain = it == 1 ? after / before : std::min(gain, after / before);
+      if (after <= o.rtol || wn == 0.) { jj++; break; }
     }
     for (int i = jj - 1; i >= 0; i--) {
       double s = gv[i];
       for (int q = i + 1; q < jj; q++) s -= R[(size_t)i * m + q] * y[q];
       y[i] = R[(size_t)i * m + i] != 0. ? s / R[(size_t)i * m + i] : 0.;
     }
-    for (int i = 0; i < jj; i++) h->hbuf[400 + 64 + i] = y[i];
-    CUDA_TRY(cudaMemcpyAsync(h->coef, h->hbuf + 464, jj * 8, cudaMemcpyHostToDevice, h->stream));
-    LAUNCH(h, k_axpy_multi, kRedBlocks, 256, n, jj, (const double *const *)h->dZ, h->coef, h->x);
-    TRY(residual_norm(h, h->x, h->V[0], &beta));
+    AxpyCoef coef;
+    for (int i = 0; i < jj; i++) coef.c[i] = y[i];
+    LAUNCH(h, k_axpy_multi, kRedBlocks, 256, n, jj, (const double *const *)h->dZ, coef, h->x);
+    if (ahead && (it >= o.max_it || jj < m)) {
+      // most likely the end: phi follows the residual, and the host waits for the norm only
+      TRY(residual_queue(h, h->x, h->V[0]));
+      CUDA_TRY(cudaEventRecord(h->it_ev, h->stream));
+      TRY(queue_phi(h));
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaEventSynchronize(h->it_ev));
+      beta = std::sqrt(h->hbuf[0]);
+      h->phi_queued = true;
+    } else {
+      TRY(residual_norm(h, h->x, h->V[0], &beta));
+    }
     rel = beta / bn;
   }
   st->iterations = it;
@@ -2381,6 +2458,10 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
                                        (size_t)16 * gb.x * gb.y * gb.z + 4096});
   }
   if ((rc = dalloc(h, &h->partial, h->partial_len))) return bail(rc);
+  if (cudaEventCreateWithFlags(&h->it_ev, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    return bail(fail(VFS_ECUDA, "cudaEventCreate failed"));
+  }
   if (cudaMallocHost(&h->hbuf, 1024 * 8) != cudaSuccess) { cudaGetLastError(); return bail(fail(VFS_ENOMEM, "pinned alloc")); }
   cudaMemsetAsync(h->phi_da, 0, N * 8, h->stream);
   cudaMemsetAsync(h->gid_da, 0xff, N * 4, h->stream);  // -1 on the boundary layer for good
@@ -2412,6 +2493,7 @@ void vfs_poisson_destroy(vfs_poisson *h) {
     if (h->phev[q]) cudaEventDestroy(h->phev[q]);
   if (h->ev_feat) cudaEventDestroy(h->ev_feat);
   if (h->side) cudaStreamDestroy(h->side);
+  if (h->it_ev) cudaEventDestroy(h->it_ev);
   for (cudaEvent_t e : h->dl_ev)
     if (e) cudaEventDestroy(e);
   if (h->dl_stream) cudaStreamDestroy(h->dl_stream);
@@ -2743,14 +2825,7 @@ int vfs_poisson_solve(vfs_poisson *h, double *phi, const vfs_solve_opts *opts, v
   TRY(fgmres(h, o, &st));
   const auto tf1 = std::chrono::steady_clock::now();
   if (h->phase) cudaEventRecord(h->phev[0], h->stream);
-  // Remove_Nullspace of phi (:604-608), its shift applied by the DA output
-  const bool shift = h->desc.bctype3 != -10 && !(h->ls_on && h->ls_bc5 == 4);
-  if (shift) {
-    LAUNCH(h, k_mean_partial, kRedBlocks, 256, n, h->fluid, h->x, h->partial);
-    LAUNCH(h, k_mean_shift, 1, 1024, h->partial, kRedBlocks, h->fsum, h->red);
-  }
-  LAUNCH(h, k_box_to_da_phi, lin_grid(h->g.n()), 256, h->g, h->box, h->rowtype0, h->fluid, h->x, h->phi_da,
-         shift ? (const double *)h->red : nullptr);
+  if (!h->phi_queued) TRY(queue_phi(h));
   // phi to a host array on a side stream, while the solution enters the
   // history on the handle's stream (it reads x, b and the residual, not
   // phi); the handle's stream waits for the copy before the call returns

@@ -1007,10 +1007,11 @@ __global__ void __launch_bounds__(256) k_gs_update(size_t n, int nv, const doubl
 
 // x += sum_v coef[v] Z_v
 __global__ void __launch_bounds__(256) k_axpy_multi(size_t n, int nv, const double *const *__restrict__ Z,
-                                                    const double *__restrict__ coef, double *__restrict__ x) {
+                                                    const __grid_constant__ AxpyCoef coef,
+                                                    double *__restrict__ x) {
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
     double acc = x[c];
-    for (int v = 0; v < nv; v++) acc = fma(coef[v], __ldcs(&Z[v][c]), acc);
+    for (int v = 0; v < nv; v++) acc = fma(coef.c[v], __ldcs(&Z[v][c]), acc);
     x[c] = acc;
   }
 }
@@ -1078,12 +1079,39 @@ __global__ void __launch_bounds__(256) k_to64(size_t n, const float *__restrict_
   }
   out[c] = x32 ? (double)x32[o] : x64[c];
 }
-__global__ void k_sumsq(size_t n, const double *__restrict__ x, double *partial) {
+template <bool COPY>
+__device__ __forceinline__ void sumsq_body(size_t n, const double *__restrict__ x, double *partial,
+                                           double *__restrict__ copy) {
   double s = 0.;
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
-    s = fma(x[c], x[c], s);
+  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
+    const double v = x[c];
+    if (COPY) copy[c] = v;
+    s = fma(v, v, s);
+  }
   s = block_sum(s);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+__global__ void k_sumsq(size_t n, const double *__restrict__ x, double *partial) {
+  sumsq_body<false>(n, x, partial, nullptr);
+}
+__global__ void k_sumsq_copy(size_t n, const double *__restrict__ x, double *partial, double *__restrict__ copy) {
+  sumsq_body<true>(n, x, partial, copy);
+}
+// The norm of a solve's first basis vector from the block partials (summed in
+// k_reduce_rows' order): ||V_0||^2 as the square of the rounded norm, as the
+// host forms it where it knows the norm, its reciprocal, and the plain sum of
+// squares to the host; one block
+__global__ void k_first_norm(const double *partial, int nb, double *out, float *out32, double *norm2) {
+  double s = 0.;
+  for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[q];
+  s = block_sum(s);
+  if (threadIdx.x == 0) {
+    const double beta = sqrt(s), inv = s > 0. ? 1. / beta : 0.;
+    out[0] = beta * beta;
+    out[1] = inv;
+    out32[0] = (float)inv;
+    norm2[0] = s;
+  }
 }
 
 // ---- history projection of the initial guess ----
