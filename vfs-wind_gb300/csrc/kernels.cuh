@@ -24,9 +24,10 @@ struct MetricPtrs {
 // The factors of Projection's correction, v dt st / coeff, and which of them
 // differ from 1 (ops bits 0..2), decided on the host: a comparison per face
 // would go to the FP64 pipe.  Bit 3: coeff lies in 2^-100..2^100, so the
-// division may go through rcoeff = RN(1 / coeff).
+// division may go through rcoeff = RN(1 / coeff) and its rest rlow (bit 4: its
+// shorter form does, see markstein3).
 struct ProjScale {
-  double dt, st, coeff, rcoeff;
+  double dt, st, coeff, rcoeff, rlow;
   int ops;
 };
 

@@ -491,7 +491,7 @@ struct vfs_poisson {
   double *rprev = nullptr, *rlearn = nullptr, *r0 = nullptr;
   float *prev32 = nullptr;
   double *ucat = nullptr;  // Contra2Cart output staging (3 per DA point, host arrays only)
-  // what Contra2Cart takes from the grid (k_contra2cart_coef: 11 planes over
+  // what Contra2Cart takes from the grid (k_contra2cart_coef: 12 planes over
   // the box), formed by its first call after the grid was set
   double *c2c = nullptr;
   bool c2c_valid = false;
@@ -754,7 +754,7 @@ int contra2cart(vfs_poisson *h, const double *u, double *v, int zero_solid) {
   const Grid &g = h->g;
   const size_t n = h->box.n();
   if (!h->c2c_valid) {
-    if (!h->c2c) TRY(dalloc(h, &h->c2c, 11 * n));
+    if (!h->c2c) TRY(dalloc(h, &h->c2c, 12 * n));
     LAUNCH(h, k_contra2cart_coef, lin_grid(n), 256, g, h->box, h->met, h->c2c);
     h->c2c_valid = true;
   }
@@ -3373,7 +3373,10 @@ int vfs_poisson_projection(vfs_poisson *h, double *ucont, double dt, double st, 
   ps.dt = dt; ps.st = st; ps.coeff = coeff;
   ps.rcoeff = 1.0 / coeff;
   const double ac = std::fabs(coeff);
-  ps.ops = (dt != 1.0 ? 1 : 0) | (st != 1.0 ? 2 : 0) | (coeff != 1.0 ? 4 : 0) | (ac > 0x1p-100 && ac < 0x1p100 ? 8 : 0);
+  const double delta = std::fma(-coeff, ps.rcoeff, 1.0);
+  ps.rlow = delta * ps.rcoeff;
+  ps.ops = (dt != 1.0 ? 1 : 0) | (st != 1.0 ? 2 : 0) | (coeff != 1.0 ? 4 : 0) |
+           (ac > 0x1p-100 && ac < 0x1p100 ? 8 : 0) | (std::fabs(delta) <= 0x1p-54 ? 16 : 0);
   if (h->ls_on) {
     LevelSet pls;
     pls.rho = h->ls_rho; pls.level = h->ls_level; pls.on = 1;

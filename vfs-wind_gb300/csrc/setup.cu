@@ -712,16 +712,21 @@ __global__ void __launch_bounds__(256, 8) k_rhs(Grid g, Box b, const uint8_t *__
   const int sj = 3 * g.mx, sk = 3 * g.mx * g.my;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
     double val = 0.;
-    if (fluid[c]) {
-      int i, j, k;
-      box_ijk(b, c, i, j, k);
-      const double *__restrict__ u = ucont + g.at(i + 1, j + 1, k + 1) * 3;
+    int i, j, k;
+    box_ijk(b, c, i, j, k);
+    const double *__restrict__ u = ucont + g.at(i + 1, j + 1, k + 1) * 3;
+    // (loaded with the byte, not after it)
+    const bool on = fluid[c];
+    const double u0 = u[0], u1 = u[1], u2 = u[2], x0 = u[i == 0 && g.px ? 3 * (b.nx - 1) : -3],
+                 y0 = u[1 + (j == 0 && g.py ? (b.ny - 1) * sj : -sj)],
+                 z0 = u[2 + (k == 0 && g.pz ? (ptrdiff_t)(b.nz - 1) * sk : -(ptrdiff_t)sk)];
+    if (on) {
       // (0 - U_i) + U_{i-1} as one subtraction: the same value
-      val = u[i == 0 && g.px ? 3 * (b.nx - 1) : -3] - u[0];
-      val -= u[1];
-      val += u[1 + (j == 0 && g.py ? (b.ny - 1) * sj : -sj)];
-      val -= u[2];
-      val += u[2 + (k == 0 && g.pz ? (ptrdiff_t)(b.nz - 1) * sk : -(ptrdiff_t)sk)];
+      val = x0 - u0;
+      val -= u1;
+      val += y0;
+      val -= u2;
+      val += z0;
       val *= f;
       sb += val;
     }
@@ -798,33 +803,45 @@ __global__ void k_reduce_rows(const double *partial, int nb, int nrow, double *o
   if (threadIdx.x == 0) out[r] = s;
 }
 
-// The reference's per-cell quotient (-sum aj) / sum_aj, correctly rounded
-// (the bits of the division) in five FP64 operations instead of a division
-// per cell: y = RN(1 / sum_aj) once, q = RN(a y), then two of Markstein's
-// corrections q <- RN(q + RN(a - q sum_aj) y) with the exact FMA remainder
-// (P. Markstein, IBM J. Res. Dev. 34 (1990) 111-119; a start within 1 ulp
-// and y correctly rounded give the correctly rounded quotient, and the
-// first correction brings RN(a y) within 1 ulp).  A sum_aj without a finite
-// reciprocal takes the division.
-__device__ __forceinline__ double markstein(double a, double d, double y) {
-  double q = a * y;
-  double r = fma(-q, d, a);
-  q = fma(r, y, q);
-  r = fma(-q, d, a);
-  return fma(r, y, q);
+// The reference's quotients by one divisor, correctly rounded (the bits of the
+// division) without a division: with y = RN(1 / d) and a start q within 1 ulp
+// of a / d, Markstein's correction RN(q + RN(a - q d) y), its remainder exact,
+// is the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34 (1990)
+// 111-119).  Two starts reach 1 ulp:
+//   RN(a y)             when delta = 1 - d y (exact by FMA) is at most 2^-54:
+//                       a/d delta is then below half an ulp, and so is the rounding
+//                       (three operations in all; 2^-54 holds for 1.5 and 3);
+//   RN(a y + RN(a yl))  with yl = RN(delta y), the reciprocal's rest (1 / d to
+//                       about 2^-105): the quotient to just over half an ulp (four).
+// The remainder must not leave the normal range; the callers see to it.
+__device__ __forceinline__ double markstein3(double a, double d, double y) {
+  const double q = a * y;
+  return fma(fma(-q, d, a), y, q);
+}
+__device__ __forceinline__ double markstein4(double a, double d, double y, double yl) {
+  const double q = fma(a, y, a * yl);
+  return fma(fma(-q, d, a), y, q);
 }
 
+// 256x192x256: 0.135 ms (0.196 with five operations and loads behind the byte's;
+// the five operations left are 0.11 ms of the FP64 pipe).
 __global__ void __launch_bounds__(256, 8) k_rhs_nullspace(Box b, const uint8_t *__restrict__ fluid,
                                                           const double *__restrict__ aj_box, const double *sums,
                                                           const double *fsum, double *__restrict__ rhs) {
-  const double sum = sums[0], sum_aj = fsum[0], y = 1.0 / sum_aj;
-  const bool fast = isfinite(y);
+  const double sum = sums[0], sum_aj = fsum[0], y = 1.0 / sum_aj, delta = fma(-sum_aj, y, 1.0), yl = delta * y;
+  const bool fast = isfinite(y), three = fabs(delta) <= 0x1p-54;
   const size_t n = b.n();
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    if (!fluid[c]) continue;
-    const double a = -sum * aj_box[c];
-    rhs[c] += fast ? markstein(a, sum_aj, y) : a / sum_aj;
-  }
+  auto shift = [&](auto quotient_of) {
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
+      const bool f = fluid[c];
+      const double aj = aj_box[c], r = rhs[c];
+      if (f) rhs[c] = r + quotient_of(-sum * aj);
+    }
+  };
+  // (three loops: a choice inside one is computed all three ways)
+  if (!fast) shift([&](double a) { return a / sum_aj; });
+  else if (three) shift([&](double a) { return markstein3(a, sum_aj, y); });
+  else shift([&](double a) { return markstein4(a, sum_aj, y, yl); });
 }
 
 // FullyBlocked (Source/poisson.c:1909-1993): per interior (i, j) column the
@@ -1082,19 +1099,44 @@ __device__ __forceinline__ double scale_down(double x, int e) {
 // v * dt * st / coeff / r in the reference's left-to-right order.  A
 // factor or divisor of exactly 1 leaves its operand unchanged, so those
 // operations are skipped: the same bits.  The division by coeff is Markstein's
-// (the quotient's bits in five operations) while quotient and remainders
-// stay in the normal range.
+// (the quotient's bits in three or four operations) while quotient and
+// remainders stay in the normal range.
 template <bool LS>
 __device__ __forceinline__ double proj_scale(double v, const ProjScale &ps, double r) {
   if (ps.ops & 1) v = v * ps.dt;
   if (ps.ops & 2) v = v * ps.st;
   if (ps.ops & 4) {
     const int ex = (__double2hiint(v) >> 20) & 0x7ff;
-    v = ex > 200 && ex < 1900 && (ps.ops & 8) ? markstein(v, ps.coeff, ps.rcoeff) : v / ps.coeff;
+    if (ex > 200 && ex < 1900 && (ps.ops & 8))
+      v = ps.ops & 16 ? markstein3(v, ps.coeff, ps.rcoeff) : markstein4(v, ps.coeff, ps.rcoeff, ps.rlow);
+    else if ((ps.ops & 8) && ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0)
+      v = v * ps.rcoeff;  // a zero of the quotient's sign
+    else
+      v = v / ps.coeff;
   }
   if (LS && r != 1.0) v = v / r;
   return v;
 }
+
+// a + b against kThr and 5, without FP64 for the values masks hold (0, 1, 3:
+// no two of them add up to 5)
+struct MaskSum {
+  bool above, below, five;
+  __device__ MaskSum(double a, double b) {
+    const int ha = __double2hiint(a), hb = __double2hiint(b);
+    auto plain = [](int h) { return h == 0 || h == 0x3ff00000 || h == 0x40080000; };
+    if ((__double2loint(a) | __double2loint(b)) == 0 && plain(ha) && plain(hb)) {
+      above = (ha | hb) != 0;
+      below = !above;
+      five = false;
+    } else {
+      const double s = a + b;
+      above = s > kThr;
+      below = s < kThr;
+      five = (int)s == 5;
+    }
+  }
+};
 
 // A tangential difference of a face (face offset f, tangential stride s):
 // (P[t+op] + P[t+f+op] - P[t+om] - P[t+f+om]) 2^-e, central (op, om = s, -s;
@@ -1110,14 +1152,14 @@ struct Tangent {
   }
   // the reference's tests (e.g. poisson.c:2773-2796), nv at the cell
   __device__ void masked(const double *__restrict__ nv, int f, int c, int m, bool per, int s) {
-    const double np = nv[s] + nv[f + s], nm = nv[-s] + nv[f - s];
+    const MaskSum np(nv[s], nv[f + s]), nm(nv[-s], nv[f - s]);
     op = s;
     om = -s;
-    if ((c == m - 2 && !per) || np > kThr) {
-      e = nm < kThr && c != 1 ? 1 : 0;
+    if ((c == m - 2 && !per) || np.above) {
+      e = nm.below && c != 1 ? 1 : 0;
       op = 0;
-    } else if ((c == 1 && !per) || nm > kThr) {
-      e = np < kThr ? 1 : 0;
+    } else if ((c == 1 && !per) || nm.above) {
+      e = np.below ? 1 : 0;
       om = 0;
     } else {
       e = 2;
@@ -1131,10 +1173,11 @@ struct Tangent {
 
 // One thread per cell, its three upper faces; cells in linear order, so that
 // no lane of the FP64 instructions idles on narrow boxes.  Bound by the FP64
-// pipe (83 % busy, 78 instructions per cell with dt != 1 and coeff 1.5, 57
-// with neither; about 150 when every blanking test was an FP64 sum and
-// comparison: near says where they are needed).  256x192x256, dt != 1, coeff
-// 1.5: 1.83 ms (3.42 ms before); the bytes alone would take 0.3 ms.
+// pipe (85 % busy, 69 instructions per cell with dt != 1 and coeff 1.5, of which
+// the reference's roundings ask for 60; 78 with five for the quotient and FP64
+// sums of the masks near bodies, about 150 with those everywhere: near says
+// where they are needed).  256x192x256, dt != 1, coeff 1.5: 1.63 ms (1.83 and
+// 3.42 ms before; the bytes alone would take 0.3 ms).
 template <bool LS>
 __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__restrict__ nvert,
                                                 const uint8_t *__restrict__ near, const double *__restrict__ phi,
@@ -1167,7 +1210,7 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
     } else {
       a.masked(nv, 1, j, my, jp, sj);
       e.masked(nv, 1, k, mz, kp, sk);
-      on = nv[0] + nv[1] < kThr;
+      on = MaskSum(nv[0], nv[1]).below;
     }
     if (on) {
       const double dpdc = P[i == mx - 2 ? 1 - i : 1] - P[0], dpde = a.diff(P, 1), dpdz = e.diff(P, 1);
@@ -1184,8 +1227,8 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
     } else {
       a.masked(nv, sj, i, mx, ip, 1);
       e.masked(nv, sj, k, mz, kp, sk);
-      const double s = nv[0] + nv[sj];
-      on = s < kThr || (int)s == 5;
+      const MaskSum s(nv[0], nv[sj]);
+      on = s.below || s.five;
     }
     if (on) {
       const double dpde = LS && ls.bc3 == 4 && j == my - 2 ? P[0] - P[-sj]
@@ -1204,7 +1247,7 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
     } else {
       a.masked(nv, sk, i, mx, ip, 1);
       e.masked(nv, sk, j, my, jp, sj);
-      on = nv[0] + nv[sk] < kThr;
+      on = MaskSum(nv[0], nv[sk]).below;
     }
     if (on) {
       double dpdz;
@@ -1465,64 +1508,80 @@ namespace vfs {
 // Faces between a fluid cell and an IB cell (0.1 < nvert < 1.1), visited
 // once each from the cell below them in i, j or k: s = 0 the cell is fluid
 // and the face's neighbour IB, s = 1 the reverse.
-struct VfluxFace {
-  double *u;
-  double a;
-  int s;
-};
-__device__ inline int vflux_faces(Grid g, const double *nvert, MetricPtrs m, double *ucont, int i, int j, int k,
-                                  VfluxFace f[6]) {
-  const size_t t = g.at(i, j, k);
-  const size_t nb[3] = {g.at(i + 1, j, k), g.at(i, j + 1, k), g.at(i, j, k + 1)};
-  const bool in[3] = {i < g.mx - 2, j < g.my - 2, k < g.mz - 2};
-  const double *met[3] = {m.csi, m.eta, m.zet};
-  int nf = 0;
-  for (int s = 0; s < 2; s++) {
-    if (s == 0 && !(nvert[t] < 0.1)) continue;
-    if (s == 1 && !(nvert[t] > 0.1 && nvert[t] < 1.1)) continue;
-    for (int q = 0; q < 3; q++) {
-      const double nn = nvert[nb[q]];
-      const bool face = s == 0 ? (nn > 0.1 && nn < 1.1) : (nn < 0.1);
-      if (!face || !in[q]) continue;
-      const double *mm = &met[q][t * 3];
-      f[nf].u = &ucont[t * 3 + q];
-      f[nf].a = sqrt(mm[0] * mm[0] + mm[1] * mm[1] + mm[2] * mm[2]);
-      f[nf].s = s;
-      nf++;
+// 0: fluid, 1: IB, 2: neither, without FP64 for the values masks hold
+__device__ __forceinline__ int mask_kind(double nv) {
+  const int h = __double2hiint(nv);
+  if (__double2loint(nv) == 0) {
+    if (h == 0) return 0;
+    if (h == 0x3ff00000) return 1;
+    if (h == 0x40080000) return 2;
+  }
+  return nv < 0.1 ? 0 : nv > 0.1 && nv < 1.1 ? 1 : 2;
+}
+// f(flux, area, s) for each such face of cell (i, j, k), i before j before k
+template <class F>
+__device__ __forceinline__ void vflux_faces(const Grid &g, const double *__restrict__ nvert, const MetricPtrs &m,
+                                            double *ucont, int i, int j, int k, F &&f) {
+  const uint32_t t = (uint32_t)g.at(i, j, k);  // (fewer than 2^32 / 19 points)
+  const double nv = nvert[t], n0 = nvert[t + 1], n1 = nvert[t + g.mx], n2 = nvert[t + g.mx * g.my];
+  const int s = mask_kind(nv);
+  if (s == 2) return;
+  const uint32_t on = (i < g.mx - 2 && mask_kind(n0) == 1 - s ? 1u : 0u) |
+                      (j < g.my - 2 && mask_kind(n1) == 1 - s ? 2u : 0u) |
+                      (k < g.mz - 2 && mask_kind(n2) == 1 - s ? 4u : 0u);
+  for (int q = 0; q < 3; q++) {
+    if (!(on >> q & 1)) continue;
+    const double *mm = (q == 0 ? m.csi : q == 1 ? m.eta : m.zet) + 3 * (size_t)t;
+    f(ucont + 3 * (size_t)t + q, sqrt(mm[0] * mm[0] + mm[1] * mm[1] + mm[2] * mm[2]), s);
+  }
+}
+// f(c) for this thread's cells of the near plane, in ascending order: the grid's
+// stride apart, the bytes of eight cells loaded at a time (one after the other,
+// each waits for the last one's latency)
+template <class F>
+__device__ __forceinline__ void near_cells(size_t n, const uint8_t *__restrict__ near, F &&f) {
+  const uint32_t stride = gridDim.x * blockDim.x, end = (uint32_t)n;
+  for (uint32_t c0 = blockIdx.x * blockDim.x + threadIdx.x; c0 < end; c0 += 8 * stride) {
+    uint32_t hit = 0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const uint32_t c = c0 + u * stride;
+      hit |= (c < end && near[c] ? 1u : 0u) << u;
+    }
+    while (hit) {
+      const int u = __ffs(hit) - 1;
+      hit &= hit - 1;
+      f(c0 + u * stride);
     }
   }
-  return nf;
 }
 
 // Both passes look only at the cells of the near plane (elsewhere no face
 // qualifies): one byte per cell instead of five nvert values and a 64-bit
-// index division.  256x192x256: 0.22 ms for the two passes (0.89 ms as three
-// passes over every cell).
+// index division, the bytes of eight cells in flight, masks told apart without
+// FP64, all blocks of the fixed grid resident.  256x192x256: 0.17 ms for the two
+// passes (0.22 before those; 0.89 ms as three passes over every cell).
 //
 // First pass: zero |U| <= 1e-8 and sum flux, |U| (or |U| / area for flg 3)
 // and area
-__global__ void __launch_bounds__(256) k_vflux_sum(Grid g, Box b, const double *__restrict__ nvert,
+__global__ void __launch_bounds__(256, 8) k_vflux_sum(Grid g, Box b, const double *__restrict__ nvert,
                                                    const uint8_t *__restrict__ near, MetricPtrs m, double *ucont,
                                                    int flg, double *partial) {
   double sf = 0, sab = 0, sa = 0;
-  const size_t n = b.n();
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    if (!near[c]) continue;
+  near_cells(b.n(), near, [&](size_t c) {
     int i, j, k;
     box_ijk(b, c, i, j, k);
-    VfluxFace f[6];
-    const int nf = vflux_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, f);
-    for (int q = 0; q < nf; q++) {
-      const double u = *f[q].u;
+    vflux_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, [&](double *pu, double area, int s) {
+      const double u = *pu;
       if (fabs(u) > 1.e-8) {
-        sf += f[q].s == 0 ? u : -u;
-        sab += flg == 3 ? fabs(u) / f[q].a : fabs(u);
-        sa += f[q].a;
+        sf += s == 0 ? u : -u;
+        sab += flg == 3 ? fabs(u) / area : fabs(u);
+        sa += area;
       } else {
-        *f[q].u = 0.;
+        *pu = 0.;
       }
-    }
-  }
+    });
+  });
   const double t0 = block_sum(sf), t1 = block_sum(sab), t2 = block_sum(sa);
   if (threadIdx.x == 0) {
     partial[blockIdx.x] = t0;
@@ -1554,32 +1613,28 @@ __global__ void k_vflux_corr(const double *partial, int nb, int flg, double flux
 
 // Second pass: the correction, and the flux and area after it (each face
 // belongs to one cell, so its new value is final)
-__global__ void __launch_bounds__(256) k_vflux_apply(Grid g, Box b, const double *__restrict__ nvert,
+__global__ void __launch_bounds__(256, 8) k_vflux_apply(Grid g, Box b, const double *__restrict__ nvert,
                                                      const uint8_t *__restrict__ near, MetricPtrs m, double *ucont,
                                                      int flg, const double *corr, double *partial) {
   const double cr = *corr;
   double sf = 0, sa = 0;
-  const size_t n = b.n();
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    if (!near[c]) continue;
+  near_cells(b.n(), near, [&](size_t c) {
     int i, j, k;
     box_ijk(b, c, i, j, k);
-    VfluxFace f[6];
-    const int nf = vflux_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, f);
-    for (int q = 0; q < nf; q++) {
-      double u = *f[q].u;
+    vflux_faces(g, nvert, m, ucont, i + 1, j + 1, k + 1, [&](double *pu, double area, int s) {
+      double u = *pu;
       if (fabs(u) > 1.e-8) {
         double dlt;
-        if (flg == 3) dlt = cr * fabs(u) / f[q].a;
+        if (flg == 3) dlt = cr * fabs(u) / area;
         else if (flg == 2) dlt = cr * fabs(u);
-        else dlt = f[q].a * cr;
-        u = f[q].s == 0 ? u - dlt : u + dlt;
-        *f[q].u = u;
+        else dlt = area * cr;
+        u = s == 0 ? u - dlt : u + dlt;
+        *pu = u;
       }
-      sf += f[q].s == 0 ? u : -u;
-      sa += f[q].a;
-    }
-  }
+      sf += s == 0 ? u : -u;
+      sa += area;
+    });
+  });
   const double t0 = block_sum(sf), t1 = block_sum(sa);
   if (threadIdx.x == 0) {
     partial[blockIdx.x] = t0;
@@ -1590,6 +1645,11 @@ __global__ void __launch_bounds__(256) k_vflux_apply(Grid g, Box b, const double
 // ---- VolumeFlux, the overload for immersed != 1, 2 (Source/poisson.c:3299-3493) ----
 // Faces between a fluid cell (nvert < 0.1) and a blanked one (nvert > 0.1),
 // visited from the cell below them; the area term is the cell metric's norm.
+struct VfluxFace {
+  double *u;
+  double a;
+  int s;
+};
 __device__ inline int vflux0_faces(Grid g, const double *nvert, MetricPtrs m, double *ucont, int i, int j, int k,
                                    VfluxFace f[6]) {
   const size_t t = g.at(i, j, k);
@@ -1680,8 +1740,9 @@ __global__ void k_periodic_cmpnts(Grid g, double *u) {
 }
 
 // What Contra2Cart takes from the grid alone: the nine minors of the cell
-// metrics, their determinant and its reciprocal (0 where a quotient by it may
-// leave the normal range), 11 planes over the box, formed once per grid.
+// metrics, their determinant, its reciprocal (0 where a quotient by it may leave
+// the normal range) and the reciprocal's rest, 12 planes over the box, formed
+// once per grid.
 __global__ void __launch_bounds__(256) k_contra2cart_coef(Grid g, Box b, MetricPtrs m, double *__restrict__ cc) {
   const size_t n = b.n(), c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
@@ -1698,15 +1759,17 @@ __global__ void __launch_bounds__(256) k_contra2cart_coef(Grid g, Box b, MetricP
   for (int p = 0; p < 9; p++) cc[p * n + c] = q[p];
   cc[9 * n + c] = det;
   const int ex = (__double2hiint(det) >> 20) & 0x7ff;
-  cc[10 * n + c] = ex > 700 && ex < 1300 ? 1.0 / det : 0.0;
+  const double y = ex > 700 && ex < 1300 ? 1.0 / det : 0.0;
+  cc[10 * n + c] = y;
+  cc[11 * n + c] = fma(-det, y, 1.0) * y;
 }
 
-// a / d from y = RN(1 / d): Markstein's quotient where a lies well inside the
+// a / d from y = RN(1 / d) and its rest yl: Markstein's quotient where a lies well inside the
 // normal range (its remainders are then exact), a y where a is a zero (the
 // quotient's sign), the division elsewhere and for y = 0.
-__device__ __forceinline__ double quotient(double a, double d, double y) {
+__device__ __forceinline__ double quotient(double a, double d, double y, double yl) {
   const int hi = __double2hiint(a), ex = (hi >> 20) & 0x7ff;
-  if (y != 0.0 && ex > 500 && ex < 1500) return markstein(a, d, y);
+  if (y != 0.0 && ex > 500 && ex < 1500) return markstein4(a, d, y, yl);
   if (y != 0.0 && ((hi & 0x7fffffff) | __double2loint(a)) == 0) return a * y;
   return a / d;
 }
@@ -1721,11 +1784,12 @@ __device__ __forceinline__ bool solid(double nv) {
 
 // Contra2Cart's change of basis by Cramer's rule, in place on ucat.  Bound by
 // the FP64 pipe: with the minors and the reciprocal of the determinant from
-// the grid (88 bytes more per cell) a cell takes 33 FP64 instructions instead
+// the grid (96 bytes more per cell) a cell takes 30 FP64 instructions instead
 // of about 100, halves and comparisons go through the integer pipe.  zero:
 // also clears solid cells, except on the two outermost layers (k_zero_rim
 // follows once the periodic ghosts have been copied).
-// 192x128x192: 0.72 -> 0.34 ms (79 % of the FP64 pipe for 33 instructions a cell).
+// 192x128x192: 0.72 -> 0.315 ms (77 % of the FP64 pipe; 0.34 ms with Markstein's
+// second correction in place of the reciprocal's rest).
 __global__ void __launch_bounds__(256) k_contra2cart(Grid g, Box b, const double *__restrict__ nvert,
                                                      const uint8_t *__restrict__ near, const double *__restrict__ cc,
                                                      const double *__restrict__ u, double *__restrict__ ucat,
@@ -1750,14 +1814,14 @@ __global__ void __launch_bounds__(256) k_contra2cart(Grid g, Box b, const double
   const double q0 = scale_down(u[tx * 3] + u[t * 3], 1), q1 = scale_down(u[ty * 3 + 1] + u[t * 3 + 1], 1),
                q2 = scale_down(u[tz * 3 + 2] + u[t * 3 + 2], 1);
 #define CC(p) __ldcs(&cc[(p) * n + c])
-  const double det = CC(9), y = CC(10);
+  const double det = CC(9), y = CC(10), yl = CC(11);
   const double d0 = q0 * CC(0) - q1 * CC(1) + q2 * CC(2);
   const double d1 = -q0 * CC(3) + q1 * CC(4) - q2 * CC(5);
   const double d2 = q0 * CC(6) - q1 * CC(7) + q2 * CC(8);
 #undef CC
-  ucat[t * 3 + 0] = quotient(d0, det, y);
-  ucat[t * 3 + 1] = quotient(d1, det, y);
-  ucat[t * 3 + 2] = quotient(d2, det, y);
+  ucat[t * 3 + 0] = quotient(d0, det, y, yl);
+  ucat[t * 3 + 1] = quotient(d1, det, y, yl);
+  ucat[t * 3 + 2] = quotient(d2, det, y, yl);
 }
 // the solid points among the two outermost layers of every side
 __global__ void k_zero_rim(Grid g, const double *__restrict__ nvert, double *ucat) {
