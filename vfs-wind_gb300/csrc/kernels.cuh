@@ -91,7 +91,7 @@ __global__ void k_fluid_mask(Grid g, Box b, const double *nvert, const double *a
                              double *partial);
 __global__ void k_mean_shift(const double *partial, int nb, const double *fsum, double *shift);
 __global__ void k_box_to_da_phi(Grid g, Box b, const uint8_t *rowtype, const uint8_t *fluid, const double *x,
-                                double *phi, const double *shift);
+                                double *phi, const double *shift, double *out);
 __global__ void k_da_to_box(Grid g, Box b, const double *da, double *x);
 __global__ void k_box_to_da(Grid g, Box b, const double *x, double *da);
 __global__ void k_near_body(Grid g, Box b, const double *nvert, uint8_t *near);
@@ -231,7 +231,7 @@ struct AxpyCoef {
   double c[64];
 };
 __global__ void k_axpy_multi(size_t n, int nv, const double *const *Z, const __grid_constant__ AxpyCoef coef,
-                             double *x);
+                             double *x, int zero);
 __global__ void k_scale_to(size_t n, const double *v, double s, const double *sinv, const double *scale,
                            double *out);
 __global__ void k_scale_to32(size_t n, const double *v, float s, const float *sinv, const float *scale, float *out,

@@ -706,6 +706,8 @@ __global__ void k_level_masks_rows(Grid g, Box b, const double *nvert, uint8_t *
 __global__ void __launch_bounds__(256, 8) k_rhs(Grid g, Box b, const uint8_t *__restrict__ fluid,
                                                 const double *__restrict__ ucont, double dt, double st, double coeff,
                                                 double *__restrict__ rhs, double *partial) {
+  pdl_trigger();
+  pdl_wait();
   double sb = 0;
   const size_t n = b.n();
   const double f = -1.0 / dt * st * coeff;  // the reference's factor, formed once
@@ -795,6 +797,8 @@ __global__ void k_rhs2_shift(Grid g, Box b, const double *__restrict__ nvert, co
 // sums row blockIdx.x of `nb` block partials in a fixed tree order (launch
 // one block per row)
 __global__ void k_reduce_rows(const double *partial, int nb, int nrow, double *out) {
+  pdl_trigger();
+  pdl_wait();
   const int r = blockIdx.x;
   if (r >= nrow) return;
   double s = 0;
@@ -828,6 +832,8 @@ __device__ __forceinline__ double markstein4(double a, double d, double y, doubl
 __global__ void __launch_bounds__(256, 8) k_rhs_nullspace(Box b, const uint8_t *__restrict__ fluid,
                                                           const double *__restrict__ aj_box, const double *sums,
                                                           const double *fsum, double *__restrict__ rhs) {
+  pdl_trigger();
+  pdl_wait();
   const double sum = sums[0], sum_aj = fsum[0], y = 1.0 / sum_aj, delta = fma(-sum_aj, y, 1.0), yl = delta * y;
   const bool fast = isfinite(y), three = fabs(delta) <= 0x1p-54;
   const size_t n = b.n();
@@ -900,6 +906,8 @@ __global__ void k_nullspace_apply(Grid g, const double *__restrict__ nvert, cons
 // count over nvert < 0.1
 __global__ void __launch_bounds__(256, 8) k_mean_partial(size_t n, const uint8_t *__restrict__ fluid,
                                                          const double *__restrict__ x, double *partial) {
+  pdl_trigger();
+  pdl_wait();
   double s = 0;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
     if (fluid[c]) s += x[c];
@@ -968,6 +976,8 @@ __global__ void __launch_bounds__(256, 8) k_fluid_sums(size_t n, const uint8_t *
 // Remove_Nullspace's shift, -sum / count, from the block partials of the
 // fluid sum (in k_reduce_rows' order) and the mask's count; one block
 __global__ void k_mean_shift(const double *partial, int nb, const double *fsum, double *shift) {
+  pdl_trigger();
+  pdl_wait();
   double s = 0;
   for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[q];
   s = block_sum(s);
@@ -980,11 +990,13 @@ __global__ void k_mean_shift(const double *partial, int nb, const double *fsum, 
 // fluid cells (nvert < 0.1) is applied on the way (x itself is left as is).
 // One thread per point in linear order (a row of 258 points would leave the
 // third block of a row-wise launch nearly empty), the dof and fluid tests from
-// byte planes: 18 bytes per point.
+// byte planes: 18 bytes per point, 26 with the caller's copy (out).
 __global__ void __launch_bounds__(256) k_box_to_da_phi(Grid g, Box b, const uint8_t *__restrict__ rowtype,
                                                        const uint8_t *__restrict__ fluid,
                                                        const double *__restrict__ x, double *__restrict__ phi,
-                                                       const double *shift) {
+                                                       const double *shift, double *__restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.n()) return;
   int i, j, k, a, bb, c, fi, fj, fk;
@@ -999,6 +1011,7 @@ __global__ void __launch_bounds__(256) k_box_to_da_phi(Grid g, Box b, const uint
     }
   }
   phi[t] = v;
+  if (out) out[t] = v;
 }
 // DA -> box copy of the interior (warm start / inspection input)
 __global__ void k_da_to_box(Grid g, Box b, const double *da, double *x) {
@@ -1060,6 +1073,8 @@ __global__ void __launch_bounds__(256) k_update_pressure(Grid g, const double *_
                                                          const uint8_t *__restrict__ near,
                                                          const double *__restrict__ phi, double *__restrict__ p,
                                                          double *__restrict__ phi_out) {
+  pdl_trigger();
+  pdl_wait();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.n()) return;
   int i, j, k;
@@ -1076,6 +1091,8 @@ __global__ void __launch_bounds__(256) k_update_pressure(Grid g, const double *_
   if (nvert[t] > 1.1) p[t] = 0;
 }
 __global__ void k_periodic_copy2(Grid g, double *p, double *phi, double *phi2) {
+  pdl_trigger();
+  pdl_wait();
   int i, j, k, a, b, c, fi, fj, fk;
   if (!shell_point(g, (size_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
   g.remap(i, j, k, a, b, c, fi, fj, fk);
@@ -1171,7 +1188,7 @@ struct Tangent {
   }
 };
 
-// One thread per cell, its three upper faces; cells in linear order, so that
+// One thread per cell, its three upper faces (small boxes: one each); cells in linear order, so that
 // no lane of the FP64 instructions idles on narrow boxes.  Bound by the FP64
 // pipe (85 % busy, 69 instructions per cell with dt != 1 and coeff 1.5, of which
 // the reference's roundings ask for 60; 78 with five for the quotient and FP64
@@ -1201,8 +1218,11 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
     r3 = k == mz - 2 ? rho[t] : ls_mean(rho[t], rho[g.at(i, j, k + 1)]);
   }
   const bool body = near[c];
+  // a grid of three rows: a thread for each face (its loads and its chain of FP64
+  // operations beside the other faces', where the SMs have room for them)
+  const int faces = gridDim.y == 3 ? 1 << blockIdx.y : 7;
   Tangent a, e;
-  if (i < mx - 2 || ip) {
+  if ((faces & 1) && (i < mx - 2 || ip)) {
     bool on = true;
     if (!body) {
       a.plain(j, my, jp, sj);
@@ -1219,7 +1239,7 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
                                          ps, r1);
     }
   }
-  if (j < my - 2 || jp || (LS && ls.bc3 == 4)) {
+  if ((faces & 2) && (j < my - 2 || jp || (LS && ls.bc3 == 4))) {
     bool on = true;
     if (!body) {
       a.plain(i, mx, ip, 1);
@@ -1239,7 +1259,7 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
                                          ps, r2);
     }
   }
-  if (k < mz - 2 || kp || (LS && ls.bc5 == 4)) {
+  if ((faces & 4) && (k < mz - 2 || kp || (LS && ls.bc5 == 4))) {
     bool on = true;
     if (!body) {
       a.plain(i, mx, ip, 1);
@@ -1270,16 +1290,22 @@ __device__ __forceinline__ void projection_body(Grid g, Box b, const double *__r
 __global__ void __launch_bounds__(256) k_projection(Grid g, Box b, const double *nvert, const uint8_t *near,
                                                     const double *phi, const double *pc, ProjScale ps, double *ucont,
                                                     MetricPtrs m) {
+  pdl_trigger();
+  pdl_wait();
   projection_body<false>(g, b, nvert, near, phi, pc, ps, ucont, m, LevelSet{});
 }
 __global__ void __launch_bounds__(256) k_projection_ls(Grid g, Box b, const double *nvert, const uint8_t *near,
                                                        const double *phi, const double *pc, ProjScale ps,
                                                        double *ucont, MetricPtrs m, LevelSet ls) {
+  pdl_trigger();
+  pdl_wait();
   projection_body<true>(g, b, nvert, near, phi, pc, ps, ucont, m, ls);
 }
 
 // periodic face copy of Ucont (poisson.c:2996-3036)
 __global__ void k_periodic_faces(Grid g, double *ucont) {
+  pdl_trigger();
+  pdl_wait();
   int i, j, k, a, b, c, fi, fj, fk;
   if (!shell_point(g, (size_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
   g.remap(i, j, k, a, b, c, fi, fj, fk);
@@ -1299,6 +1325,8 @@ __global__ void k_periodic_faces(Grid g, double *ucont) {
 // over.
 __global__ void __launch_bounds__(256, 8) k_divergence(Grid g, Box b, const double *__restrict__ nvert, const uint8_t *__restrict__ near,
                              const double *__restrict__ ucont, const double *__restrict__ aj, double *partial) {
+  pdl_trigger();
+  pdl_wait();
   long long best = 0;
   const size_t n = b.n();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
@@ -1320,6 +1348,8 @@ __global__ void __launch_bounds__(256, 8) k_divergence(Grid g, Box b, const doub
   if (threadIdx.x == 0) partial[blockIdx.x] = m;
 }
 __global__ void k_reduce_max(const double *partial, int nb, double *out) {
+  pdl_trigger();
+  pdl_wait();
   double m = 0.;
   for (int q = threadIdx.x; q < nb; q += blockDim.x) m = partial[q] > m ? partial[q] : m;
   m = block_max(m);

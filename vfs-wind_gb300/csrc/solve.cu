@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(256) k_apply64(Box b, const double *__restrict
 __global__ void __launch_bounds__(256) k_residual64r(Box b, const double *__restrict__ A,
                                                      const double *__restrict__ x, const double *__restrict__ rhs,
                                                      double *__restrict__ r) {
+  pdl_trigger();
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
   if (i >= b.nx) return;
   uint32_t idx[NSLOT];
@@ -1008,9 +1010,11 @@ __global__ void __launch_bounds__(256) k_gs_update(size_t n, int nv, const doubl
 // x += sum_v coef[v] Z_v
 __global__ void __launch_bounds__(256) k_axpy_multi(size_t n, int nv, const double *const *__restrict__ Z,
                                                     const __grid_constant__ AxpyCoef coef,
-                                                    double *__restrict__ x) {
+                                                    double *__restrict__ x, int zero) {
+  pdl_trigger();
+  pdl_wait();
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    double acc = x[c];
+    double acc = zero ? 0. : x[c];
     for (int v = 0; v < nv; v++) acc = fma(coef.c[v], __ldcs(&Z[v][c]), acc);
     x[c] = acc;
   }
@@ -1082,6 +1086,8 @@ __global__ void __launch_bounds__(256) k_to64(size_t n, const float *__restrict_
 template <bool COPY>
 __device__ __forceinline__ void sumsq_body(size_t n, const double *__restrict__ x, double *partial,
                                            double *__restrict__ copy) {
+  pdl_trigger();
+  pdl_wait();
   double s = 0.;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
     const double v = x[c];
@@ -1102,6 +1108,8 @@ __global__ void k_sumsq_copy(size_t n, const double *__restrict__ x, double *par
 // host forms it where it knows the norm, its reciprocal, and the plain sum of
 // squares to the host; one block
 __global__ void k_first_norm(const double *partial, int nb, double *out, float *out32, double *norm2) {
+  pdl_trigger();
+  pdl_wait();
   double s = 0.;
   for (int q = threadIdx.x; q < nb; q += blockDim.x) s += partial[q];
   s = block_sum(s);
