@@ -680,6 +680,24 @@ int sync(vfs_poisson *h) {
 
 dim3 da_grid(const Grid &g, int bx = 128) { return dim3((g.mx + bx - 1) / bx, g.my, g.mz); }
 dim3 box_grid(const Box &b, int bx = 128) { return dim3((b.nx + bx - 1) / bx, b.ny, b.nz); }
+// Grid and block of a kernel that gives `cells` of every row (j, k) a thread:
+// blocks of whole rows (or equal parts of rows longer than 128), as many rows as
+// leave the fewest idle lanes in 128 to 256 threads.  One row in blocks of 128
+// left half the lanes idle at 64 cells a row (a colour of 128) and a quarter at 96:
+// the residual of a colour with its line solve 16.9 -> 12.3 us at 128x96x128.
+struct RowGrid {
+  dim3 grid, block;
+};
+RowGrid row_grid(int cells, int ny, int nz) {
+  const int parts = (cells + 127) / 128, w = (cells + parts - 1) / parts;
+  int rows = 1, best = 1 << 30;
+  for (int r = std::min(ny, (127 + w) / w); r == 1 || r * w <= 256; r++) {
+    const int idle = (int)(((r * w + 31) / 32 * 32 - r * w) * 4096ll / (r * w));
+    if (idle < best) { best = idle; rows = r; }
+    if (r >= ny) break;
+  }
+  return {dim3(parts, (ny + rows - 1) / rows, nz), dim3(w, rows)};
+}
 unsigned lin_grid(size_t n, int bx = 256) { return (unsigned)((n + bx - 1) / bx); }
 // grid of the passes over the periodic ghost layers (shell_point); 0: no periodic axis
 unsigned shell_grid(const Grid &g) {
@@ -1194,10 +1212,10 @@ struct Prec;
 template <>
 struct Prec<float> {
   static constexpr auto sweep = k_line_sweep_f32;
-  static void residual(vfs_poisson *h, Level &l, dim3 g, const float *x, const float *bb, float *r, int color,
+  static void residual(vfs_poisson *h, Level &l, RowGrid g, const float *x, const float *bb, float *r, int color,
                        bool split) {
-    if (split) launch_v(h, k_residual16_split, g, 128, 0, l.b, l.C16, l.D32, x, bb, r, color);
-    else launch_v(h, k_residual16, g, 128, 0, l.b, l.C16, l.D32, x, bb, r, color);
+    if (split) launch_v(h, k_residual16_split, g.grid, g.block, 0, l.b, l.C16, l.D32, x, bb, r, color);
+    else launch_v(h, k_residual16, g.grid, g.block, 0, l.b, l.C16, l.D32, x, bb, r, color);
   }
   static constexpr auto restrict_ = k_restrict_f32;
   static constexpr auto prolong = k_prolong_f32;
@@ -1221,9 +1239,9 @@ struct Prec<float> {
 template <>
 struct Prec<double> {
   static constexpr auto sweep = k_line_sweep_f64;
-  static void residual(vfs_poisson *h, Level &l, dim3 g, const double *x, const double *bb, double *r, int color,
+  static void residual(vfs_poisson *h, Level &l, RowGrid g, const double *x, const double *bb, double *r, int color,
                        bool) {
-    launch_v(h, k_residual_f64, g, 128, 0, l.b, l.A64, x, bb, r, color);
+    launch_v(h, k_residual_f64, g.grid, g.block, 0, l.b, l.A64, x, bb, r, color);
   }
   static constexpr auto restrict_ = k_restrict_f64;
   static constexpr auto prolong = k_prolong_f64;
@@ -1331,14 +1349,14 @@ void smooth(vfs_poisson *h, Level &l, int li, int smoother, bool zero_guess, T o
              zero_guess ? 1 : 0);
     std::swap(x, t);
   } else if (smoother == 1) {
-    if (!zero_guess) Prec<T>::residual(h, l, box_grid(l.b), x, bb, r, -1, false);
+    if (!zero_guess) Prec<T>::residual(h, l, row_grid(l.b.nx, l.b.ny, l.b.nz), x, bb, r, -1, false);
     launch_v(h, Prec<T>::tri, lg, lb, lsm, l.b, zero_guess ? bb : r, Asp, Prec<T>::inv(l), Prec<T>::cp(l), x,
              omega, zero_guess ? 1 : 0, -1);
   } else if (smoother == 2) {
     if (zero_guess) vmemset(h, x, l.b.n() * sizeof(T));
     for (int color = 0; color < 2; color++) {
       const bool skip_res = zero_guess && color == 0;  // x = 0: r = rhs
-      if (!skip_res) Prec<T>::residual(h, l, box_grid(l.b), x, bb, r, color, false);
+      if (!skip_res) Prec<T>::residual(h, l, row_grid(l.b.nx, l.b.ny, l.b.nz), x, bb, r, color, false);
       launch_v(h, Prec<T>::tri, lg, lb, lsm, l.b, skip_res ? bb : r, Asp, Prec<T>::inv(l), Prec<T>::cp(l), x,
                omega, 0, color);
     }
@@ -1360,7 +1378,8 @@ void smooth(vfs_poisson *h, Level &l, int li, int smoother, bool zero_guess, T o
     const bool split = split_level<T>(h, li, smoother);
     if (zero_guess && !split) vmemset(h, x, l.b.n() * sizeof(T));
     const int nh = (l.b.nx + 1) / 2;
-    dim3 cg((nh + TI - 1) / TI, l.b.nz), rg((nh + 127) / 128, l.b.ny, l.b.nz);
+    const dim3 cg((nh + TI - 1) / TI, l.b.nz);
+    const RowGrid rg = row_grid(nh, l.b.ny, l.b.nz);
     for (int color = 0; color < 2; color++) {
       const bool skip_res = zero_guess && color == 0;
       if (!skip_res) Prec<T>::residual(h, l, rg, x, bb, r, 2 + color, split);
@@ -1538,16 +1557,17 @@ void vcycle(vfs_poisson *h, int li, int nu1, int nu2, T omega, int smoother) {
     // residual is zero up to rounding: form the first colour's only
     // (and 0 on the second's)
     const int nh = (l.b.nx + 1) / 2;
-    Prec<T>::residual(h, l, dim3((nh + 127) / 128, l.b.ny, l.b.nz), x, bb, r, 6, split_level<T>(h, li, smoother));
+    Prec<T>::residual(h, l, row_grid(nh, l.b.ny, l.b.nz), x, bb, r, 6, split_level<T>(h, li, smoother));
   } else {
-    Prec<T>::residual(h, l, box_grid(l.b), x, bb, r, -1, split_level<T>(h, li, smoother));
+    Prec<T>::residual(h, l, row_grid(l.b.nx, l.b.ny, l.b.nz), x, bb, r, -1, split_level<T>(h, li, smoother));
   }
   Level &q = h->L[li + 1];
-  launch_v(h, Prec<T>::restrict_, box_grid(q.b), 128, 0, l.b, q.b, l.cx, l.cy, l.cz, r, Prec<T>::w(l), q.blank,
+  const RowGrid qg = row_grid(q.b.nx, q.b.ny, q.b.nz), pg = row_grid(l.b.nx, (l.b.ny + 1) / 2, l.b.nz);
+  launch_v(h, Prec<T>::restrict_, qg.grid, qg.block, 0, l.b, q.b, l.cx, l.cy, l.cz, r, Prec<T>::w(l), q.blank,
            Prec<T>::v(q)[1]);
   vcycle<T>(h, li + 1, nu1, nu2, omega, smoother);
   const auto prolong = split_level<T>(h, li, smoother) ? Prec<T>::prolong_split : Prec<T>::prolong;
-  launch_v(h, prolong, dim3((l.b.nx + 127) / 128, (l.b.ny + 1) / 2, l.b.nz), 128, 0, l.b, q.b, l.cx, l.cy, l.cz,
+  launch_v(h, prolong, pg.grid, pg.block, 0, l.b, q.b, l.cx, l.cy, l.cz,
            (const T *)Prec<T>::xfinal(q), q.blank, l.blank, x, 1);
   for (int s = 0; s < nu2; s++) smooth<T>(h, l, li, smoother, false, omega, x, t, bb, r);
   Prec<T>::xfinal(l) = x;
@@ -1666,7 +1686,8 @@ int reduce_read(vfs_poisson *h, int nb, int nrow, double *out) {
 int residual_queue(vfs_poisson *h, const double *x, double *r) {
   const size_t n = h->box.n();
   const int nb = red_blocks(n);
-  launch_v(h, k_residual64r, box_grid(h->box), 128, 0, h->box, h->A0, x, h->b, r);
+  const RowGrid g = row_grid(h->box.nx, h->box.ny, h->box.nz);
+  launch_v(h, k_residual64r, g.grid, g.block, 0, h->box, h->A0, x, h->b, r);
   launch_v(h, k_sumsq, nb, 256, 0, n, r, h->partial);
   launch_v(h, k_reduce_rows, 1, 1024, 0, h->partial, nb, 1, h->hbuf);
   return VFS_OK;
@@ -2115,7 +2136,8 @@ int arnoldi_enqueue(vfs_poisson *h, int jj, int nbd, const vfs_solve_opts &o, in
   };
   stamp(1);
   double *w = h->V[jj + 1];
-  launch_v(h, k_apply64, box_grid(h->box), 128, 0, h->box, (const double *)h->A0, (const double *)h->Z[jj], w);
+  const RowGrid g = row_grid(h->box.nx, h->box.ny, h->box.nz);
+  launch_v(h, k_apply64, g.grid, g.block, 0, h->box, (const double *)h->A0, (const double *)h->Z[jj], w);
   stamp(2);
   double *back = h->hbuf + hb;
   if (o.orth == 0) {

@@ -1420,8 +1420,8 @@ __device__ __forceinline__ void restrict_body(Box bf, Box bc, int cx, int cy, in
                                               T *bc_out) {
   pdl_trigger();
   pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-  if (i >= bc.nx) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
+  if (i >= bc.nx || j >= bc.ny) return;
   size_t cc = bc.at(i, j, k);
   if (blank_c[cc]) { bc_out[cc] = (T)0; return; }
   int i1 = cx ? 2 * i + 1 : i, j1 = cy ? 2 * j + 1 : j, k1 = cz ? 2 * k + 1 : k;
@@ -1443,9 +1443,9 @@ __device__ __forceinline__ void prolong_body(Box bf, Box bc, int cx, int cy, int
                                              T *xf, int add) {
   pdl_trigger();
   pdl_wait();
-  // a thread takes rows j = blockIdx.y and blockIdx.y + gridDim.y of column
-  // i (when inside the box): all the loads of both cells first, then both
-  // results
+  // a thread takes a row j of the grid's and the one as many rows further on of
+  // column i (when inside the box): all the loads of both cells first, then
+  // both results
   const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.z;
   if (i >= bf.nx) return;
   const int mx = bf.nx + 2, my = bf.ny + 2, mz = bf.nz + 2;
@@ -1460,7 +1460,7 @@ __device__ __forceinline__ void prolong_body(Box bf, Box bc, int cx, int cy, int
   T X[2][2][2][2], xold[2];  // [row][i side][j side][k side]
 #pragma unroll
   for (int r = 0; r < 2; r++) {
-    const int j = blockIdx.y + r * gridDim.y;
+    const int j = (blockIdx.y + r * gridDim.y) * blockDim.y + threadIdx.y;
     valid[r] = j < bf.ny;
     if (!valid[r]) continue;
     c[r] = bf.at(i, j, k);

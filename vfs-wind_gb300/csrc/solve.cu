@@ -45,8 +45,9 @@ __device__ __forceinline__ void residual_body(Box b, const T *__restrict__ A, co
                                               const T *__restrict__ rhs, T *__restrict__ r, int color) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
   int p;
+  if (j >= b.ny) return;
   if (color >= 6) clear_partner(b, color, t, (uint32_t)b.at(0, j, k), k, r);
   if (!colour_row(b, color, t, k, p)) return;
   const int i = split_cell(p, b.nx);
@@ -100,15 +101,18 @@ __global__ void k_pack16_rows(Box b, const double *__restrict__ A, __half2 *__re
 // instead of 76.  Colours and layouts as in residual_body; SPLIT: x and rhs
 // in the parity-split row layout (r written as the colour selects).  The
 // operator's 44 bytes per row are loaded before pdl_wait (no kernel of the
-// V-cycle writes them), x and rhs after it.
+// V-cycle writes them), x and rhs after it.  48 registers: the operator's and the
+// neighbours' loads fly together (at 32 they take turns: 10.4 -> 9.2 us a colour at
+// 128x96x128, 26.7 -> 25.8 at 192x128x192, 5.5 TB/s).
 template <bool SPLIT>
 __device__ __forceinline__ void residual16_body(Box b, const __half2 *__restrict__ C, const float *__restrict__ D,
                                                 const float *__restrict__ x, const float *__restrict__ rhs,
                                                 float *__restrict__ r, int color) {
   pdl_trigger();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, jt = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
+  const int j = min(jt, b.ny - 1);  // (the threads past the last row load and store nothing)
   int p;
-  const bool ok = colour_row(b, color, t, k, p);
+  const bool ok = colour_row(b, color, t, k, p) && jt < b.ny;
   if (!ok) p = 0;  // (a row without a cell of the colour loads nothing)
   const int i = split_cell(p, b.nx);
   uint32_t idx[NSLOT];
@@ -122,7 +126,7 @@ __device__ __forceinline__ void residual16_body(Box b, const __half2 *__restrict
     d = __ldcs(&D[cs]);
   }
   pdl_wait();
-  if (color >= 6) clear_partner(b, color, t, row, k, r);
+  if (color >= 6 && jt < b.ny) clear_partner(b, color, t, row, k, r);
   if (!ok) return;
   const float xc = __ldg(&x[c]);
   float s = 0.f;
@@ -135,12 +139,12 @@ __device__ __forceinline__ void residual16_body(Box b, const __half2 *__restrict
   s = fmaf(__low2float(hc[9]), xc, s);
   r[color == 2 || color == 3 ? cs : cn] = rhs[SPLIT ? cs : cn] - d * s;
 }
-__global__ void __launch_bounds__(128) k_residual16(Box b, const __half2 *__restrict__ C,
+__global__ void __launch_bounds__(256, 5) k_residual16(Box b, const __half2 *__restrict__ C,
                                                     const float *__restrict__ D, const float *__restrict__ x,
                                                     const float *__restrict__ rhs, float *__restrict__ r, int color) {
   residual16_body<false>(b, C, D, x, rhs, r, color);
 }
-__global__ void __launch_bounds__(128) k_residual16_split(Box b, const __half2 *__restrict__ C,
+__global__ void __launch_bounds__(256, 5) k_residual16_split(Box b, const __half2 *__restrict__ C,
                                                           const float *__restrict__ D, const float *__restrict__ x,
                                                           const float *__restrict__ rhs, float *__restrict__ r,
                                                           int color) {
@@ -151,9 +155,9 @@ __global__ void __launch_bounds__(128) k_residual16_split(Box b, const __half2 *
 __global__ void __launch_bounds__(256) k_apply64(Box b, const double *__restrict__ A, const double *__restrict__ x,
                                                  double *__restrict__ y) {
   pdl_trigger();
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
   pdl_wait();
-  if (i >= b.nx) return;
+  if (i >= b.nx || j >= b.ny) return;
   uint32_t idx[NSLOT];
   stencil_index(b, i, j, k, idx);
   const uint32_t n = (uint32_t)b.n(), c = idx[CP];
@@ -171,8 +175,8 @@ __global__ void __launch_bounds__(256) k_residual64r(Box b, const double *__rest
                                                      double *__restrict__ r) {
   pdl_trigger();
   pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-  if (i >= b.nx) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
+  if (i >= b.nx || j >= b.ny) return;
   uint32_t idx[NSLOT];
   stencil_index(b, i, j, k, idx);
   const uint32_t n = (uint32_t)b.n(), c = idx[CP];
