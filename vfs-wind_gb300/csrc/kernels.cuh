@@ -237,7 +237,10 @@ __global__ void k_scale_to(size_t n, const double *v, double s, const double *si
 __global__ void k_scale_to32(size_t n, const double *v, float s, const float *sinv, const float *scale, float *out,
                              int split_nx);
 __global__ void k_reduce_norm(const double *partial, int nb, double *out, float *out32, double *norm2);
+__global__ void k_scale_to32_split4(size_t n4, const double *v, float s, const float *sinv, const float *scale,
+                                    float *out, int nx);
 __global__ void k_to64(size_t n, const float *x32, const double *x64, double *out, int split_nx);
+__global__ void k_to64_split4(size_t n4, const float *x32, double *out, int nx);
 __global__ void k_sumsq(size_t n, const double *x, double *partial);
 __global__ void k_sumsq_copy(size_t n, const double *x, double *partial, double *copy);
 __global__ void k_first_norm(const double *partial, int nb, double *out, float *out32, double *norm2);

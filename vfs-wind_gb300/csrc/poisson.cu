@@ -698,6 +698,13 @@ RowGrid row_grid(int cells, int ny, int nz) {
   }
   return {dim3(parts, (ny + rows - 1) / rows, nz), dim3(w, rows)};
 }
+// the same for the interpolation from a level coarsened by (cy, cz) along j and
+// k: pairs of rows and planes (prolong_quad), in FP64 of rows only (prolong_rows)
+template <typename T>
+RowGrid prolong_grid(const Box &b, int cy, int cz) {
+  if (std::is_same<T, double>::value) return row_grid(b.nx, (b.ny + 1) / 2, b.nz);
+  return row_grid(b.nx, cy ? b.ny / 2 + 1 : (b.ny + 1) / 2, cz ? b.nz / 2 + 1 : (b.nz + 1) / 2);
+}
 unsigned lin_grid(size_t n, int bx = 256) { return (unsigned)((n + bx - 1) / bx); }
 // grid of the passes over the periodic ghost layers (shell_point); 0: no periodic axis
 unsigned shell_grid(const Grid &g) {
@@ -1562,7 +1569,7 @@ void vcycle(vfs_poisson *h, int li, int nu1, int nu2, T omega, int smoother) {
     Prec<T>::residual(h, l, row_grid(l.b.nx, l.b.ny, l.b.nz), x, bb, r, -1, split_level<T>(h, li, smoother));
   }
   Level &q = h->L[li + 1];
-  const RowGrid qg = row_grid(q.b.nx, q.b.ny, q.b.nz), pg = row_grid(l.b.nx, (l.b.ny + 1) / 2, l.b.nz);
+  const RowGrid qg = row_grid(q.b.nx, q.b.ny, q.b.nz), pg = prolong_grid<T>(l.b, l.cy, l.cz);
   launch_v(h, Prec<T>::restrict_, qg.grid, qg.block, 0, l.b, q.b, l.cx, l.cy, l.cz, r, Prec<T>::w(l), q.blank,
            Prec<T>::v(q)[1]);
   vcycle<T>(h, li + 1, nu1, nu2, omega, smoother);
@@ -1644,9 +1651,17 @@ int precondition(vfs_poisson *h, const double *v, double s, const double *sinv64
   h->pdl_prev = false;  // the chain's first kernel waits for all earlier work
   if (o.precision == 0) {
     const int snx = split_level<float>(h, 0, o.smoother) ? l0.b.nx : 0;
-    launch_v(h, k_scale_to32, lin_grid(n), 256, 0, n, v, (float)s, sinv32, (const float *)h->scale32, l0.v32[1], snx);
+    // (split rows of a multiple of four cells: four a thread, in wide loads and stores)
+    const bool four = snx > 0 && snx % 4 == 0;
+    if (four)
+      launch_v(h, k_scale_to32_split4, lin_grid(n / 4), 256, 0, n / 4, v, (float)s, sinv32, (const float *)h->scale32,
+               l0.v32[1], snx);
+    else
+      launch_v(h, k_scale_to32, lin_grid(n), 256, 0, n, v, (float)s, sinv32, (const float *)h->scale32, l0.v32[1],
+               snx);
     TRY(run_vcycle<float>(h, o));
-    launch_v(h, k_to64, lin_grid(n), 256, 0, n, (const float *)l0.xfinal32, (const double *)nullptr, z, snx);
+    if (four) launch_v(h, k_to64_split4, lin_grid(n / 4), 256, 0, n / 4, (const float *)l0.xfinal32, z, snx);
+    else launch_v(h, k_to64, lin_grid(n), 256, 0, n, (const float *)l0.xfinal32, (const double *)nullptr, z, snx);
   } else {
     launch_v(h, k_scale_to, kRedBlocks, 256, 0, n, v, s, sinv64, (const double *)h->scale, l0.v64[1]);
     TRY(run_vcycle<double>(h, o));
@@ -3573,7 +3588,8 @@ int vfs_poisson_mg_interpolate(vfs_poisson *h, int fine, const double *xc, doubl
   Level &l = h->L[fine], &q = h->L[fine + 1];
   TRY(upload(h, h->stage, xc, q.g.n()));
   LAUNCH(h, k_da_to_box, lin_grid(q.b.n()), 256, q.g, q.b, h->stage, q.v64[0]);
-  LAUNCH(h, k_prolong_f64, box_grid(l.b), 128, l.b, q.b, l.cx, l.cy, l.cz, (const double *)q.v64[0], q.blank,
+  const RowGrid pg = prolong_grid<double>(l.b, l.cy, l.cz);
+  LAUNCH(h, k_prolong_f64, pg.grid, pg.block, l.b, q.b, l.cx, l.cy, l.cz, (const double *)q.v64[0], q.blank,
          l.blank, l.v64[2], 0);
   LAUNCH(h, k_box_to_da, lin_grid(l.g.n()), 256, l.g, l.b, l.v64[2], h->stage);
   TRY(download(h, ff, h->stage, l.g.n()));
