@@ -135,8 +135,22 @@ TYPED_DECL(float, f32)
 TYPED_DECL(double, f64)
 #undef TYPED_DECL
 
-__global__ void k_line_lu(Box b, const double *A64, double *inv64, double *cp64, float *inv32, float *cp32,
-                          const uint8_t *colflag);
+// The levels of one k_line_lu launch: a level's columns (i fastest, then k) in
+// blocks of 128 from block `first` on; colflag: the columns to form, null: all.
+constexpr int kMaxLevels = 24;
+struct LuLevel {
+  uint32_t first;
+  int nx, ny, nz;
+  const double *A;
+  double *inv64, *cp64;
+  float *inv32, *cp32;
+  const uint8_t *colflag;
+};
+struct LuArgs {
+  int levels;
+  LuLevel level[kMaxLevels];
+};
+__global__ void k_line_lu(const __grid_constant__ LuArgs args);
 __global__ void k_pack16(size_t n, const double *A, __half2 *C, float *D);
 __global__ void k_pack16_rows(Box b, const double *A, __half2 *C, float *D, float *A32, const int *rows,
                               const int *nrows);

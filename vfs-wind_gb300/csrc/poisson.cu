@@ -44,7 +44,6 @@ int fail(int code, const std::string &msg) {
     if (rc_ != VFS_OK) return rc_; \
   } while (0)
 
-constexpr int kMaxLevels = 24;
 constexpr int kRedBlocks = 1216;  // 8 x 152 SMs, fixed for deterministic reductions
 
 // device helper kernels that only the host orchestration needs
@@ -425,6 +424,7 @@ struct Level {
   int cx = 0, cy = 0, cz = 0;
   double *coor = nullptr, *nvert = nullptr;
   double *nvert_prev = nullptr;  // the restricted mask of the previous fill (coarse levels, incremental refill)
+  uint8_t *colflag = nullptr;    // j-columns that hold a row to refill (incremental refill)
   MetricPtrs met{};
   bool own_met = false;
   double *A64 = nullptr;
@@ -515,7 +515,6 @@ struct vfs_poisson {
   bool inc_enable = true, nvert_prev_valid = false, inc_rows = false;
   double *nvert_prev = nullptr;
   uint32_t *chg = nullptr;  // changed points, bits in words of 32 along i
-  uint8_t *colflag = nullptr;
   int *rows = nullptr, *nrows = nullptr;
   // history of the last hist_cnt (at most hist_cap) converged solutions for
   // the initial guess, held as the newest one X_n (the FGMRES iterate before
@@ -990,6 +989,7 @@ int build_coarsest(vfs_poisson *h, Level &l) {
 void free_level(vfs_poisson *h, Level &l, bool level0) {
   if (!level0) { dfree(h, l.coor); dfree(h, l.nvert); dfree(h, l.nvert_prev); dfree(h, l.rho); dfree(h, l.level); }
   if (l.own_met) free_metrics(h, l.met);
+  dfree(h, l.colflag);
   dfree(h, l.A64); dfree(h, l.A32); dfree(h, l.C16); dfree(h, l.D32); dfree(h, l.rowtype); dfree(h, l.blank);
   dfree(h, l.inv64); dfree(h, l.cp64); dfree(h, l.w64); dfree(h, l.inv32); dfree(h, l.cp32); dfree(h, l.w32);
   for (int q = 0; q < 4; q++) { dfree(h, l.v64[q]); dfree(h, l.v32[q]); }
@@ -1019,7 +1019,7 @@ LevelSet level_set(const vfs_poisson *h, const Level &l) {
   return ls;
 }
 
-// Operator, masks and line factors of one level (assembled from its
+// Operator and masks of one level (assembled from its
 // metrics, unless `assembled`: the fine level's operator formed together
 // with the FGMRES operator) into its buffers, allocated on the first build.
 int build_level_operator(vfs_poisson *h, Level &l, bool assembled = false) {
@@ -1047,12 +1047,9 @@ int build_level_operator(vfs_poisson *h, Level &l, bool assembled = false) {
            (const int *)h->rows, (const int *)h->nrows);
   else
     LAUNCH(h, k_level_masks, lin_grid(n), 256, l.g, l.b, l.nvert, l.blank, l.w64, l.w32);
-  // a level of an incremental refill: only the listed rows' copies and the
-  // j-columns that hold one are formed again
-  const uint8_t *cols = h->inc_rows ? h->colflag : nullptr;
-  LAUNCH(h, k_line_lu, dim3((l.b.nx + 127) / 128, l.b.nz), 128, l.b, (const double *)l.A64, l.inv64, l.cp64, l.inv32,
-         l.cp32, cols);
-  if (cols) {
+  // a level of an incremental refill: only the listed rows' copies are formed
+  // again (line_factors: and the j-columns that hold one)
+  if (h->inc_rows) {
     LAUNCH(h, k_pack16_rows, kRedBlocks, 256, l.b, (const double *)l.A64, l.C16, l.D32, l.A32, (const int *)h->rows,
            (const int *)h->nrows);
   } else {
@@ -1062,15 +1059,33 @@ int build_level_operator(vfs_poisson *h, Level &l, bool assembled = false) {
   return VFS_OK;
 }
 
+// The line factors of every level, whose operators are formed.
+int line_factors(vfs_poisson *h) {
+  LuArgs a;
+  a.levels = (int)h->L.size();
+  uint32_t blocks = 0;
+  for (int li = 0; li < a.levels; li++) {
+    const Level &l = h->L[li];
+    a.level[li] = {blocks, l.b.nx, l.b.ny, l.b.nz, l.A64, l.inv64, l.cp64, l.inv32, l.cp32,
+                   h->inc_rows ? l.colflag : nullptr};
+    blocks += lin_grid((size_t)l.b.nx * l.b.nz, 128);
+  }
+  LAUNCH(h, k_line_lu, blocks, 128, a);
+  return VFS_OK;
+}
+
 // The rows to refill after a new mask (src, copied to nvert on the way where
-// they differ) in place of the mask prev, with their j-columns.
-int list_rows(vfs_poisson *h, const Grid &g, const Box &b, const double *src, double *nvert, const double *prev) {
+// they differ) in place of the mask prev, with their j-columns (cols, its own
+// buffer for every level).
+int list_rows(vfs_poisson *h, const Grid &g, const Box &b, const double *src, double *nvert, const double *prev,
+              uint8_t **cols) {
+  if (!*cols) TRY(dalloc(h, cols, (size_t)b.nx * b.nz));
   const int wpr = (g.mx + 31) / 32;
   LAUNCH(h, k_changed_bits, kRedBlocks, 256, g, wpr, src, nvert, prev, h->chg);
   CUDA_TRY(cudaMemsetAsync(h->nrows, 0, sizeof(int), h->stream));
-  CUDA_TRY(cudaMemsetAsync(h->colflag, 0, (size_t)b.nx * b.nz, h->stream));
+  CUDA_TRY(cudaMemsetAsync(*cols, 0, (size_t)b.nx * b.nz, h->stream));
   LAUNCH(h, k_list_rows, lin_grid((size_t)b.ny * b.nz * wpr), 256, g, b, wpr, (const uint32_t *)h->chg, h->rows,
-         h->nrows, h->colflag);
+         h->nrows, *cols);
   return VFS_OK;
 }
 
@@ -1094,8 +1109,9 @@ int refresh_hierarchy(vfs_poisson *h) {
       if (!q.nvert_prev) TRY(dalloc(h, &q.nvert_prev, q.g.n()));
       std::swap(q.nvert, q.nvert_prev);
     }
-    LAUNCH(h, k_nvert_restrict, da_grid(q.g), 128, f.g, q.g, f.cx, f.cy, f.cz, f.nvert, h->stage);
-    LAUNCH(h, k_nvert_fill, da_grid(q.g), 128, q.g, h->stage, q.nvert);
+    const RowGrid qg = row_grid(q.g.mx, q.g.my, q.g.mz);
+    LAUNCH(h, k_nvert_restrict, qg.grid, qg.block, f.g, q.g, f.cx, f.cy, f.cz, f.nvert, h->stage);
+    LAUNCH(h, k_nvert_fill, qg.grid, qg.block, q.g, h->stage, q.nvert);
     if (h->ls_on) {
       LAUNCH(h, k_cellfield_restrict, da_grid(q.g), 128, f.g, q.g, f.cx, f.cy, f.cz, f.rho, q.rho);
       LAUNCH(h, k_cellfield_restrict, da_grid(q.g), 128, f.g, q.g, f.cx, f.cy, f.cz, f.level, q.level);
@@ -1108,10 +1124,11 @@ int refresh_hierarchy(vfs_poisson *h) {
       // the rows of this level within two points of a changed restricted
       // mask value (the list buffers of the finest level, consumed by its
       // launches above, are reused in stream order)
-      TRY(list_rows(h, l.g, l.b, l.nvert, l.nvert, l.nvert_prev));
+      TRY(list_rows(h, l.g, l.b, l.nvert, l.nvert, l.nvert_prev, &l.colflag));
     }
     TRY(build_level_operator(h, l, li == 0));
   }
+  TRY(line_factors(h));
   h->inc_rows = false;
   if (h->phase) TRY(sync(h));
   const auto t1 = std::chrono::steady_clock::now();
@@ -1207,6 +1224,7 @@ int build_hierarchy(vfs_poisson *h, int coarsest_max) {
     TRY(sync(h));
     // the coarse metrics stay for the assembly of later masks
   }
+  TRY(line_factors(h));
   TRY(build_coarsest(h, h->L.back()));
   h->hier_cmax = coarsest_max;
   h->hier_ls = h->ls_on != 0;
@@ -2603,7 +2621,6 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
   if (h->inc_enable && !h->nvert_prev) {
     TRY(dalloc(h, &h->nvert_prev, N));
     TRY(dalloc(h, &h->chg, (size_t)((h->g.mx + 31) / 32) * h->g.my * h->g.mz));
-    TRY(dalloc(h, &h->colflag, (size_t)h->box.nx * h->box.nz));
     TRY(dalloc(h, &h->rows, n));
     TRY(dalloc(h, &h->nrows, 1));
   }
@@ -2621,7 +2638,7 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
   if (incremental) {
     const bool dev = is_device_ptr(nvert);
     if (!dev) TRY(upload(h, h->nvert, nvert, N));
-    TRY(list_rows(h, h->g, h->box, dev ? nvert : h->nvert, h->nvert, h->nvert_prev));
+    TRY(list_rows(h, h->g, h->box, dev ? nvert : h->nvert, h->nvert, h->nvert_prev, &h->L[0].colflag));
     LAUNCH(h, k_assemble_fine_rows, kRedBlocks, 256, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
            h->L[0].A64, h->L[0].rowtype, fls, rows, nrows);
     LAUNCH(h, k_near_body_rows, kRedBlocks, 256, h->g, h->box, (const double *)h->nvert, h->near, rows, nrows);
@@ -2645,9 +2662,9 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
   LAUNCH(h, k_reduce_rows, 2, 1024, h->partial, kRedBlocks, 2, h->fsum);
   // setup_lidx2: dof numbering in k-j-i order
   const int nblk = (int)((n + 1023) / 1024);
-  LAUNCH(h, k_count_dofs, nblk, 1024, n, (const uint8_t *)h->rowtype0, h->blk);
+  LAUNCH(h, k_count_dofs, nblk, 256, n, (const uint8_t *)h->rowtype0, h->blk);
   LAUNCH(h, k_scan_blocks, 1, 1024, h->blk, nblk, h->total);
-  LAUNCH(h, k_number_dofs, nblk, 1024, h->g, h->box, (const uint8_t *)h->rowtype0, (const int *)h->blk, h->gid_da);
+  LAUNCH(h, k_number_dofs, nblk, 256, h->g, h->box, (const uint8_t *)h->rowtype0, (const int *)h->blk, h->gid_da);
   if (const unsigned nb = shell_grid(h->g)) LAUNCH(h, k_gid_ghosts, nb, 256, h->g, h->gid_da);
   int tot = 0;
   CUDA_TRY(cudaMemcpyAsync(&tot, h->total, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -3539,12 +3556,16 @@ int vfs_poisson_apply(vfs_poisson *h, const double *x, double *y) {
   if (!h || !x || !y) return fail(VFS_EINVAL, "null argument");
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come first");
   const size_t n = h->box.n();
-  TRY(upload(h, h->stage, x, h->g.n()));
-  double *tmp = h->L[0].v64[3];
-  LAUNCH(h, k_da_to_box, lin_grid(n), 256, h->g, h->box, h->stage, h->r);
-  LAUNCH(h, k_apply64, box_grid(h->box), 128, h->box, h->A0, h->r, tmp);
-  LAUNCH(h, k_box_to_da, lin_grid(h->g.n()), 256, h->g, h->box, tmp, h->stage);
-  TRY(download(h, y, h->stage, h->g.n()));
+  // device arrays are read and written where they lie
+  const double *xd = nullptr;
+  TRY(device_view(h, x, h->stage, h->g.n(), &xd));
+  const bool ydev = is_device_ptr(y);
+  double *tmp = h->L[0].v64[3], *yd = ydev ? y : h->stage;
+  const RowGrid g = row_grid(h->box.nx, h->box.ny, h->box.nz);
+  LAUNCH(h, k_da_to_box, lin_grid(n), 256, h->g, h->box, xd, h->r);
+  LAUNCH(h, k_apply64, g.grid, g.block, h->box, h->A0, h->r, tmp);
+  LAUNCH(h, k_box_to_da, lin_grid(h->g.n()), 256, h->g, h->box, tmp, yd);
+  if (!ydev) TRY(download(h, y, yd, h->g.n()));
   return sync(h);
 }
 
