@@ -873,12 +873,12 @@ __global__ void k_cgs_reduce(const double *__restrict__ partial, int nb, const d
   }
 }
 
-// w -= sum_v red[kGsB + v] Q_v; block partials of ||w||^2.  VU vectors' loads
-// go out at once (small boxes: latency).
-template <int VU>
-__device__ __forceinline__ void cgs_update_body(size_t n, int nv, const double *const *__restrict__ Q,
+// w -= sum_v red[kGsB + v] Q_v; block partials of ||w||^2.  Small boxes are bound
+// by latency: the loads of four vectors go out at once.
+__device__ __forceinline__ void cgs_update_few(size_t n, int nv, const double *const *__restrict__ Q,
                                                 const double *__restrict__ red, double *__restrict__ w,
                                                 double *partial) {
+  constexpr int VU = 4;
   pdl_trigger();
   pdl_wait();
   const size_t base = (size_t)blockIdx.x * blockDim.x * kGsTile + threadIdx.x;
@@ -919,13 +919,48 @@ __device__ __forceinline__ void cgs_update_body(size_t n, int nv, const double *
   ss = block_sum(ss);
   if (threadIdx.x == 0) partial[blockIdx.x] = ss;
 }
-__global__ void __launch_bounds__(256) k_cgs_update(size_t n, int nv, const double *const *Q, const double *red,
-                                                    double *w, double *partial) {
-  cgs_update_body<1>(n, nv, Q, red, w, partial);
+// Large boxes are bound by the FP64 pipe (nv + 1 operations a cell): a vector at a
+// time, offsets in the instructions and no test per load where a block has no end
+// in it, so that four blocks of the 2304 of 192x128x192 fit an SM (three left the
+// sixth wave of five nearly empty): 81 -> 66 us for six vectors.
+template <bool FULL>
+__device__ __forceinline__ void cgs_update_tile(uint32_t n, uint32_t base, int nv,
+                                                const double *const *__restrict__ Q,
+                                                const double *__restrict__ red, double *__restrict__ w,
+                                                double aw[kGsTile]) {
+  auto in = [&](int t) { return FULL || base + t * 256 < n; };
+#pragma unroll
+  for (int t = 0; t < kGsTile; t++) aw[t] = in(t) ? w[base + t * 256] : 0.;
+  for (int v = 0; v < nv; v++) {
+    const double *p = Q[v] + base, cb = -red[kGsB + v];
+    double q[kGsTile];
+#pragma unroll
+    for (int t = 0; t < kGsTile; t++) q[t] = in(t) ? __ldcs(p + t * 256) : 0.;
+#pragma unroll
+    for (int t = 0; t < kGsTile; t++) aw[t] = fma(cb, q[t], aw[t]);
+  }
+#pragma unroll
+  for (int t = 0; t < kGsTile; t++)
+    if (in(t)) w[base + t * 256] = aw[t];
+}
+__global__ void __launch_bounds__(256, 4) k_cgs_update(size_t n, int nv, const double *const *Q, const double *red,
+                                                       double *w, double *partial) {
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t n32 = (uint32_t)n, first = blockIdx.x * (256 * kGsTile), base = first + threadIdx.x;
+  double aw[kGsTile];
+  if (first + 256 * kGsTile <= n32) cgs_update_tile<true>(n32, base, nv, Q, red, w, aw);
+  else cgs_update_tile<false>(n32, base, nv, Q, red, w, aw);
+  double ss = 0.;
+#pragma unroll
+  for (int t = 0; t < kGsTile; t++)
+    if (base + t * 256 < n32) ss = fma(aw[t], aw[t], ss);
+  ss = block_sum(ss);
+  if (threadIdx.x == 0) partial[blockIdx.x] = ss;
 }
 __global__ void __launch_bounds__(256, 1) k_cgs_update_small(size_t n, int nv, const double *const *Q,
                                                              const double *red, double *w, double *partial) {
-  cgs_update_body<4>(n, nv, Q, red, w, partial);
+  cgs_update_few(n, nv, Q, red, w, partial);
 }
 
 #define GS_DOTS(NV)                                                                                            \
