@@ -1606,9 +1606,10 @@ int run_vcycle(vfs_poisson *h, const vfs_solve_opts &o) {
   // A V-cycle with at most kDirectLevels levels above its tail is a dozen
   // launches at most: issued one by one they start with the chain (a graph
   // starts 10-14 us after its predecessor ends, and its launch takes as long as
-  // theirs): 24x16x24 1016 -> 985 us a solve, 64^3 1704 -> 1671, FP64 72x40x56
-  // 5866 -> 5812 (two levels above the tail: 6050).  Live kernel timing runs
-  // without a graph, too.
+  // theirs): 24x16x24 1016 -> 985 us a solve.  With two levels and more the host
+  // falls behind the short kernels, even a step ahead: 64^3 1503 us with the graph
+  // and 1528 without, FP64 72x40x56 5440 and 5625, 128x96x128 4512 and 4588.  Live
+  // kernel timing runs without a graph, too.
   TailArgs ta;
   size_t tsm;
   int above = 0;
