@@ -18,8 +18,8 @@
 //     The same kernel computes data gradients with flipped, transposed
 //     weights and an FP32 epilogue.
 //   * k_wgrad: weight gradients, A = input tile transposed (ldmatrix.trans),
-//     B = pre-activation gradient tile; a warp owns the three taps of a
-//     (dz, dy), a CTA loops over voxel tiles and stores its sums.
+//     B = pre-activation gradient tile; a warp owns one tap of a dz
+//     plane, a CTA loops over voxel tiles and stores its sums.
 // Every sum over voxels (weights, biases, head, loss) is a set of partials per
 // CTA that one kernel adds in a fixed order (k_grad_reduce): a gradient of the
 // mean squared error is the same bits every time.  ReLU's backward pass has no kernel of its own: what
@@ -59,6 +59,7 @@ constexpr int ROWB = 48;                                     // 16 ch + pad, byt
 constexpr int CONV_SMEM = HVOX * ROWB;                       // 51840
 constexpr int CONV_SMALL = 2 * HX * 6 * 4 * ROWB;            // two stages of the 16x4x2 tile
 constexpr int CONV_THREADS = 256;                            // 8 warps x 4 rows
+constexpr int WGRAD_XT = HX * HY * TZ * ROWB;                // input tile of a weight gradient's dz plane
 
 struct Src {
   const bf16 *p;  // channels-last tensor
@@ -257,32 +258,35 @@ __global__ void __launch_bounds__(CONV_THREADS, CT == 16 ? 4 : 2) k_conv(ConvGeo
   }
 }
 
-// Partial weight gradients: part[CTA][tap][ci][co] = sum over the CTA's voxels
-// of X[v + off(tap)][ci] * Gp[v][co] for input channel group blockIdx.y.  Warp
-// w: dz = w / 3 - 1, dy = w % 3 - 1 and the three dx, which share the
-// gradient's fragments (one tap a warp, a CTA a dz plane and atomics: 28 us for
-// 16 x 16 channels of 64^3 voxels, now 23.5).
+// Partial weight gradients: part[chunk][tap][ci][co] = sum over the chunk's
+// voxel tiles of X[v + off(tap)][ci] * Gp[v][co] for input channel group
+// blockIdx.y and the taps of plane dz = blockIdx.z - 1 (warp w: dy = w / 3 - 1,
+// dx = w % 3 - 1), whose input tile needs no halo along z.  A chunk's products
+// are one chain of FP32 accumulations in the tensor core, tile by tile
+// (blockIdx.x, blockIdx.x + chunks, ...; wgrad_chunks): which tiles share a chain
+// decides the gradient's last bits, and with them BF16 roundings of the next step.
+// 16 x 16 channels of 64^3 voxels: 28.5 us (30.4 with the halo along z, and bounds
+// and addresses formed for each voxel).  All 27 taps a CTA over 256 chunks takes 19,
+// but its chains put the gradient of 48 x 16 channels 6e-6 off.
 template <int COUT>
-__global__ void __launch_bounds__(288) k_wgrad(ConvGeom G, const bf16 *__restrict__ gpre, float *part) {
+__global__ void __launch_bounds__(288, 2) k_wgrad(ConvGeom G, const bf16 *__restrict__ gpre, float *part) {
   extern __shared__ __align__(16) unsigned char smem[];
   pdl_trigger();
   pdl_wait();
   unsigned char *xt = smem;
-  unsigned char *gt = smem + CONV_SMEM;
+  unsigned char *gt = smem + WGRAD_XT;
   constexpr int GROW = COUT * 2 + 16;  // bytes per voxel row of the gradient tile
   constexpr int NT = COUT / 8;
-  const int g = blockIdx.y;
+  const int g = blockIdx.y, dzi = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_x = (G.nx + TX - 1) / TX, tiles_y = (G.ny + TY - 1) / TY, tiles_z = (G.nz + TZ - 1) / TZ;
   const int ntiles = tiles_x * tiles_y * tiles_z;
-  float acc[3][NT][4];
+  float acc[NT][4];
 #pragma unroll
-  for (int d = 0; d < 3; d++)
-#pragma unroll
-    for (int n = 0; n < NT; n++) acc[d][n][0] = acc[d][n][1] = acc[d][n][2] = acc[d][n][3] = 0.f;
+  for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
   // A = X^T: rows ci, columns voxels; matrix i = lane / 8 holds (ci half
   // i & 1, voxel half i >> 1)
-  const uint32_t xa = smem_u32(xt) + (((warp / 3) * HY + warp % 3) * HX + ((lane >> 4) << 3) + (lane & 7)) * ROWB +
+  const uint32_t xa = smem_u32(xt) + ((warp / 3) * HX + warp % 3 + ((lane >> 4) << 3) + (lane & 7)) * ROWB +
                       ((lane >> 3) & 1) * 16;
   // B = gradient rows (voxels) x 8 output channels; x4.trans covers (voxel
   // half i & 1, n-tile n + (i >> 1))
@@ -300,37 +304,32 @@ __global__ void __launch_bounds__(288) k_wgrad(ConvGeom G, const bf16 *__restric
       else
         cp_async16(smem_u32(dst), gpre + (((size_t)z * G.ny + y) * G.nx + x) * COUT + c * 8);
     }
-    load_rows<HY, HZ, 9>(G, g, x0, y0, z0, xt);
+    load_rows<HY, TZ, 9>(G, g, x0, y0, z0 + dzi, xt);
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
-#pragma unroll 2
+#pragma unroll 4
     for (int r = 0; r < TY * TZ; r++) {
       const uint32_t xr = xa + ((r / TY) * HY + r % TY) * HX * ROWB, gr = ga + r * TX * GROW;
-      uint32_t b[NT / 2][4], a[3][4];
+      uint32_t b[NT / 2][4], a[4];
+      ldsm_x4_t(a, xr);
 #pragma unroll
       for (int n = 0; n < NT / 2; n++) ldsm_x4_t(b[n], gr + n * 32);
 #pragma unroll
-      for (int d = 0; d < 3; d++) ldsm_x4_t(a[d], xr + d * ROWB);
-#pragma unroll
-      for (int d = 0; d < 3; d++)
-#pragma unroll
-        for (int n = 0; n < NT / 2; n++) {
-          mma_bf16(acc[d][2 * n], a[d], b[n][0], b[n][1]);
-          mma_bf16(acc[d][2 * n + 1], a[d], b[n][2], b[n][3]);
-        }
+      for (int n = 0; n < NT / 2; n++) {
+        mma_bf16(acc[2 * n], a, b[n][0], b[n][1]);
+        mma_bf16(acc[2 * n + 1], a, b[n][2], b[n][3]);
+      }
     }
   }
   const int cin = G.groups * 16;
-  float *base = part + (size_t)blockIdx.x * 27 * cin * COUT;
+  float *base = part + ((size_t)blockIdx.x * 27 + dzi * 9 + warp) * cin * COUT;
 #pragma unroll
-  for (int d = 0; d < 3; d++)
-#pragma unroll
-    for (int n = 0; n < NT; n++) {
-      const int ci = g * 16 + (lane >> 2), co = n * 8 + (lane & 3) * 2;
-      float *w = base + ((size_t)(warp * 3 + d) * cin + ci) * COUT + co;
-      *reinterpret_cast<float2 *>(w) = make_float2(acc[d][n][0], acc[d][n][1]);
-      *reinterpret_cast<float2 *>(w + 8 * COUT) = make_float2(acc[d][n][2], acc[d][n][3]);
-    }
+  for (int n = 0; n < NT; n++) {
+    const int ci = g * 16 + (lane >> 2), co = n * 8 + (lane & 3) * 2;
+    float *w = base + (size_t)ci * COUT + co;
+    *reinterpret_cast<float2 *>(w) = make_float2(acc[n][0], acc[n][1]);
+    *reinterpret_cast<float2 *>(w + 8 * COUT) = make_float2(acc[n][2], acc[n][3]);
+  }
 }
 
 // The partials of one set of sums: parts rows of `cols` values, `stride` apart.
@@ -347,9 +346,8 @@ struct Sums {
   Sum w[kWeightSets], s[kSmallSets];  // weights (a block 32 values); biases and head (a block a set, cols divides 256)
   int first[kWeightSets + 1];         // blocks of the weight sets
 };
-// (a block's 8 warps share the partials of its values: with a thread a value
-// up to 304 loads stood in a row, 143 us a step, now 41:
-// 65 MB)
+// (a block's 8 warps share the partials of its values: a thread a value has up to 304
+// loads in a row.  64^3 voxels: 36 MB of partials, 28 us)
 __global__ void __launch_bounds__(256) k_grad_reduce(const __grid_constant__ Sums S) {
   pdl_trigger();
   pdl_wait();
@@ -869,12 +867,11 @@ struct ConvGrid {
   }
 };
 
-// CTAs that share a layer's voxel tiles in the weight gradient: two a SM, no
-// more than share them evenly.
+// Chunks of a layer's voxel tiles in the weight gradient: with the three dz
+// planes and the channel groups two CTAs a SM.
 int wgrad_chunks(const Conv &c, int nx, int ny, int nz) {
-  const int ntiles = ((nx + TX - 1) / TX) * ((ny + TY - 1) / TY) * ((nz + TZ - 1) / TZ), groups = c.cin / 16;
-  const int rounds = (ntiles + 304 / groups - 1) / (304 / groups);
-  return (ntiles + rounds - 1) / rounds;
+  const int ntiles = ((nx + TX - 1) / TX) * ((ny + TY - 1) / TY) * ((nz + TZ - 1) / TZ);
+  return std::max(1, std::min(ntiles, 304 / (c.cin / 16 * 3)));
 }
 
 // Rows of the bias partials of layer li: the CTAs of what forms its gradient
@@ -933,7 +930,7 @@ bool smem_attr(K kernel, int bytes) {
 int configure_kernels() {
   std::lock_guard<std::mutex> lk(cfg_mu);
   if (kernels_configured) return VFS_OK;
-  const int wg = CONV_SMEM + TX * TY * TZ * 16;  // + gradient tile rows of (2 COUT + 16) bytes
+  const int wg = WGRAD_XT + TX * TY * TZ * 16;  // + gradient tile rows of (2 COUT + 16) bytes
   bool ok = smem_attr(k_conv<16, kForward, TY, TZ, 1>, CONV_SMEM) && smem_attr(k_conv<32, kForward, TY, TZ, 1>, CONV_SMEM) &&
             smem_attr(k_conv<16, kData, TY, TZ, 1>, CONV_SMEM) && smem_attr(k_conv<32, kData, TY, TZ, 1>, CONV_SMEM) &&
             smem_attr(k_conv<16, kMasked, TY, TZ, 1>, CONV_SMEM) && smem_attr(k_conv<32, kMasked, TY, TZ, 1>, CONV_SMEM) &&
@@ -1011,8 +1008,8 @@ void conv_dgrad_relu(vfs_unet *u, int li, int nx, int ny, int nz, const bf16 *gp
 void conv_wgrad(vfs_unet *u, int li, int nx, int ny, int nz, const bf16 *s0, const bf16 *s1, const bf16 *gp) {
   const Conv &c = u->conv[li];
   ConvGeom G = geom(c, nx, ny, nz, s0, s1);
-  const dim3 grid(u->sums.w[li].parts, G.groups);
-  const int smem = CONV_SMEM + TX * TY * TZ * (c.cout * 2 + 16);
+  const dim3 grid(u->sums.w[li].parts, G.groups, 3);
+  const int smem = WGRAD_XT + TX * TY * TZ * (c.cout * 2 + 16);
   launch(u, c.cout == 16 ? k_wgrad<16> : c.cout == 32 ? k_wgrad<32> : k_wgrad<64>, grid, 288, smem, G, gp, u->wpart[li]);
 }
 
