@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "rules.h"
 #include "vfs_poisson.h"
 
 using namespace vfs;
@@ -639,6 +640,18 @@ bool is_device_ptr(const void *p) {
   }
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
+// kernels may work on the caller's array p itself
+bool in_place(const vfs_poisson *h, const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const MemoryType t = a.type == cudaMemoryTypeDevice    ? MemoryType::device
+                       : a.type == cudaMemoryTypeManaged ? MemoryType::managed
+                                                         : MemoryType::host;
+  return in_place(t, a.device, h->device, (uintptr_t)p);
+}
 
 // copy a caller array (host or device) into a device buffer
 int upload(vfs_poisson *h, double *dst, const double *src, size_t count) {
@@ -646,19 +659,19 @@ int upload(vfs_poisson *h, double *dst, const double *src, size_t count) {
                            is_device_ptr(src) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, h->stream));
   return VFS_OK;
 }
-// device memory is read where it lies; host memory is staged
+// an array that is read: where it lies, or staged
 int device_view(vfs_poisson *h, const double *src, double *stage, size_t count, const double **out) {
-  if (is_device_ptr(src)) {
+  if (in_place(h, src)) {
     *out = src;
     return VFS_OK;
   }
   *out = stage;
   return upload(h, stage, src, count);
 }
-// an array that is read and written: device memory where it lies, host memory
-// through *stage (allocated on first use; the caller downloads it)
+// an array that is read and written: where it lies, or through *stage
+// (allocated on first use; the caller downloads it)
 int device_inout(vfs_poisson *h, double *a, double **stage, size_t count, double **out) {
-  if (is_device_ptr(a)) {
+  if (in_place(h, a)) {
     *out = a;
     return VFS_OK;
   }
@@ -2644,7 +2657,7 @@ int vfs_poisson_set_nvert(vfs_poisson *h, const double *nvert) {
   // count over the fluid, which every right-hand side and mean removal uses),
   // aj at the box cells, the cells near a body and the row scale
   if (incremental) {
-    const bool dev = is_device_ptr(nvert);
+    const bool dev = in_place(h, nvert);
     if (!dev) TRY(upload(h, h->nvert, nvert, N));
     TRY(list_rows(h, h->g, h->box, dev ? nvert : h->nvert, h->nvert, h->nvert_prev, &h->L[0].colflag));
     LAUNCH(h, k_assemble_fine_rows, kRedBlocks, 256, h->g, h->box, h->nvert, h->met, h->A0, h->rowtype0,
@@ -2771,7 +2784,7 @@ int vfs_poisson_volume_flux(vfs_poisson *h, double *ucont, int flg, double flux_
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before volume_flux");
   if (flg < 0 || flg > 3) return fail(VFS_EINVAL, "flg must be 0..3");
   const size_t N = h->g.n();
-  const bool dev = is_device_ptr(ucont);
+  const bool dev = in_place(h, ucont);
   double *u = dev ? ucont : h->ucont;
   if (!dev) TRY(upload(h, u, ucont, 3 * N));
   LAUNCH(h, k_vflux_sum, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, h->met, u, flg, h->partial);
@@ -2790,7 +2803,7 @@ int vfs_poisson_volume_flux0(vfs_poisson *h, double *ucont, int immersed, double
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before volume_flux0");
   if (immersed == 1) return fail(VFS_EINVAL, "immersed 1 takes the other VolumeFlux (vfs_poisson_volume_flux)");
   const size_t N = h->g.n();
-  const bool dev = is_device_ptr(ucont);
+  const bool dev = in_place(h, ucont);
   double *u = dev ? ucont : h->ucont;
   if (!dev) TRY(upload(h, u, ucont, 3 * N));
   LAUNCH(h, k_vflux0_sum, kRedBlocks, 256, h->g, h->box, h->nvert, h->near, h->met, u, h->partial);
@@ -2909,17 +2922,17 @@ int vfs_poisson_solve(vfs_poisson *h, double *phi, const vfs_solve_opts *opts, v
     CUDA_TRY(cudaMemsetAsync(h->x, 0, n * 8, h->stream));  // (no step will write x)
   }
   // phi to a device array in the pass that forms the handle's own copy
-  const bool host_out = phi && !is_device_ptr(phi);
-  double *phi_out = host_out ? nullptr : phi;
+  const bool staged = phi && !in_place(h, phi);
+  double *phi_out = staged ? nullptr : phi;
   const auto tf0 = std::chrono::steady_clock::now();
   TRY(fgmres(h, o, &st, phi_out));
   const auto tf1 = std::chrono::steady_clock::now();
   if (h->phase) cudaEventRecord(h->phev[0], h->stream);
   if (!h->phi_queued) TRY(queue_phi(h, phi_out));
-  // phi to a host array on a side stream, while the solution enters the
+  // phi to an array elsewhere on a side stream, while the solution enters the
   // history on the handle's stream (it reads x, b and the residual, not
   // phi); the handle's stream waits for the copy before the call returns
-  if (host_out) {
+  if (staged) {
     if (!h->dl_stream) {
       CUDA_TRY(cudaStreamCreateWithFlags(&h->dl_stream, cudaStreamNonBlocking));
       CUDA_TRY(cudaEventCreateWithFlags(&h->dl_ev[0], cudaEventDisableTiming));
@@ -2927,7 +2940,8 @@ int vfs_poisson_solve(vfs_poisson *h, double *phi, const vfs_solve_opts *opts, v
     }
     CUDA_TRY(cudaEventRecord(h->dl_ev[0], h->stream));
     CUDA_TRY(cudaStreamWaitEvent(h->dl_stream, h->dl_ev[0], 0));
-    CUDA_TRY(cudaMemcpyAsync(phi, h->phi_da, h->g.n() * sizeof(double), cudaMemcpyDeviceToHost, h->dl_stream));
+    CUDA_TRY(cudaMemcpyAsync(phi, h->phi_da, h->g.n() * sizeof(double),
+                             is_device_ptr(phi) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, h->dl_stream));
     if (h->phase) cudaEventRecord(h->phev[2], h->dl_stream);
     CUDA_TRY(cudaEventRecord(h->dl_ev[1], h->dl_stream));
   }
@@ -2935,7 +2949,7 @@ int vfs_poisson_solve(vfs_poisson *h, double *phi, const vfs_solve_opts *opts, v
     TRY(hist_push(h));
   if (h->phase) cudaEventRecord(h->phev[1], h->stream);
   const auto tf2 = std::chrono::steady_clock::now();
-  if (host_out) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->dl_ev[1], 0));
+  if (staged) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->dl_ev[1], 0));
   CUDA_TRY(cudaEventRecord(h->ev1, h->stream));
   TRY(sync(h));
   if (h->phase) {
@@ -2945,7 +2959,7 @@ int vfs_poisson_solve(vfs_poisson *h, double *phi, const vfs_solve_opts *opts, v
     const auto tf3 = std::chrono::steady_clock::now();
     float a = 0.f, c = -1.f;
     cudaEventElapsedTime(&a, h->phev[0], h->phev[1]);
-    if (host_out) cudaEventElapsedTime(&c, h->phev[0], h->phev[2]);
+    if (staged) cudaEventElapsedTime(&c, h->phev[0], h->phev[2]);
     fprintf(stderr, "vfs solve tail ms: host fgmres %.3f tail %.3f wait %.3f; device to push end %.3f, to copy end %.3f\n",
             std::chrono::duration<double, std::milli>(tf1 - tf0).count(),
             std::chrono::duration<double, std::milli>(tf2 - tf1).count(),
@@ -3435,7 +3449,7 @@ int vfs_poisson_update_pressure(vfs_poisson *h, double *p, double *phi) {
   const size_t N = h->g.n();
   // device arrays are updated where they lie; the handle's phi (which
   // Projection reads) receives its copy in the same pass
-  const bool pdev = is_device_ptr(p), fdev = phi && is_device_ptr(phi);
+  const bool pdev = in_place(h, p), fdev = phi && in_place(h, phi);
   double *pd = pdev ? p : h->p_da;
   if (!pdev) TRY(upload(h, pd, p, N));
   if (phi && !fdev) TRY(upload(h, h->phi_da, phi, N));
@@ -3454,7 +3468,7 @@ int vfs_poisson_projection(vfs_poisson *h, double *ucont, double dt, double st, 
   if (!h->have_nvert) return fail(VFS_ESTATE, "set_nvert must come before projection");
   if (!(coeff != 0.)) return fail(VFS_EINVAL, "coeff must be non-zero");
   const size_t N = h->g.n(), n = h->box.n();
-  const bool dev = is_device_ptr(ucont);
+  const bool dev = in_place(h, ucont);
   double *u = dev ? ucont : h->ucont;
   if (!dev) TRY(upload(h, u, ucont, 3 * N));
   ProjScale ps;
@@ -3554,7 +3568,7 @@ int vfs_poisson_get_metric(vfs_poisson *h, int which, double *out) {
 int vfs_poisson_get_rhs(vfs_poisson *h, double *b) {
   if (!h || !b) return fail(VFS_EINVAL, "null argument");
   if (!h->have_rhs) return fail(VFS_ESTATE, "rhs must come first");
-  const bool dev = is_device_ptr(b);
+  const bool dev = in_place(h, b);
   LAUNCH(h, k_box_to_da, lin_grid(h->g.n()), 256, h->g, h->box, h->b, dev ? b : h->stage);
   if (!dev) TRY(download(h, b, h->stage, h->g.n()));
   return sync(h);
@@ -3567,7 +3581,7 @@ int vfs_poisson_apply(vfs_poisson *h, const double *x, double *y) {
   // device arrays are read and written where they lie
   const double *xd = nullptr;
   TRY(device_view(h, x, h->stage, h->g.n(), &xd));
-  const bool ydev = is_device_ptr(y);
+  const bool ydev = in_place(h, y);
   double *tmp = h->L[0].v64[3], *yd = ydev ? y : h->stage;
   const RowGrid g = row_grid(h->box.nx, h->box.ny, h->box.nz);
   LAUNCH(h, k_da_to_box, lin_grid(n), 256, h->g, h->box, xd, h->r);
