@@ -56,3 +56,43 @@ def test_arrays_off_the_element_grid(cuda_lib):
         s.close()
     for k in got[0]:
         np.testing.assert_array_equal(got[0][k], got[1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 300])
+def test_overlapping_arrays(cuda_lib, shift):
+    """Arrays that share memory, wholly or from an element on: every value from the
+    arrays as they were passed, results written in the order of the arguments."""
+    import torch
+    import vfs_poisson as V
+    from vfs_poisson import configs as CF
+    L = V.load()
+    case, rng = build(DIMS, PERIODIC, "plain")
+    n3, n1 = case.ucont.size, case.nvert.size
+    surf = CF.rod_surface((0.5, 0.2, 0.5), (0.0, 1.0, 0.0), 0.5, 0.2, 16, 6)
+    base = rng.normal(size=2 * n3 + n1)
+    calls = {  # offsets of the arrays in one buffer, in the order of the call's downloads
+        "contra2cart": (lambda h, c, u: L.vfs_poisson_contra2cart(h, u, c, 1), (shift, 0), (n3, 0)),
+        "ib_bc": (lambda h, c, u: L.vfs_poisson_ib_bc(h, 1, None, c, u), (shift, 0), (n3, n3)),
+        "ibm_interpolate": (lambda h, c, p, u: L.vfs_poisson_ibm_interpolate(h, 0, None, 1, None, c, p, u),
+                            (shift, 2 * n3, 0), (n3, n1, n3)),
+        "update_pressure": (lambda h, p, f: L.vfs_poisson_update_pressure(h, p, f), (shift, 0), (n1, n1)),
+    }
+    s = V.PoissonSolver(*case.dims, periodic=PERIODIC)
+    try:
+        s.set_grid(case.coor)
+        nv, _, nodes = s.ibm_search_nodes(surf)
+        assert nodes > 0
+        s.set_nvert(nv)
+        for name, (call, off, size) in calls.items():
+            length = {"update_pressure": n1}.get(name, n3)
+            # each array alone, then the writes in order
+            own = [torch.from_numpy(base[o:o + (n1 if o == 2 * n3 else length)].copy()).cuda() for o in off]
+            V._check(call(s.h, *[a.data_ptr() for a in own]))
+            want = base.copy()
+            for o, a, k in zip(off, own, size):
+                want[o:o + k] = a.cpu().numpy()[:k]
+            buf = torch.from_numpy(base.copy()).cuda()
+            V._check(call(s.h, *[buf.data_ptr() + 8 * o for o in off]))
+            np.testing.assert_array_equal(buf.cpu().numpy(), want, err_msg=name)
+    finally:
+        s.close()

@@ -13,6 +13,9 @@ extern "C" {
 int t_in_place(int type, int memory_device, int device, uintptr_t address) {
   return vfs::in_place((vfs::MemoryType)type, memory_device, device, address);
 }
+int t_overlap(size_t a, size_t na, size_t b, size_t nb, size_t c, size_t nc) {
+  return vfs::overlap({{(void *)a, na}, {(void *)b, nb}, {(void *)c, nc}});
+}
 }
 """
 HOST, DEVICE, MANAGED = 0, 1, 2
@@ -29,6 +32,7 @@ def rules(tmp_path_factory):
                     "-o", str(d / "shim.so")], check=True)
     L = C.CDLL(str(d / "shim.so"))
     L.t_in_place.argtypes = [C.c_int, C.c_int, C.c_int, C.c_size_t]
+    L.t_overlap.argtypes = [C.c_size_t] * 6
     return L
 
 
@@ -58,3 +62,11 @@ def test_the_library_asks_the_rule():
         assert "= is_device_ptr(" not in body and "!is_device_ptr(" not in body, entry
     start = src.index("int device_view(")
     assert "is_device_ptr" not in src[start:src.index("int download(", start)]
+
+
+def test_overlapping_arrays(rules):
+    a, n, none = 0x10000, 240, (0, 240)
+    for b, nb, want in ((a, n, 1), (a + n, n, 0), (a - 80, 80, 0), (a + n - 8, 80, 1), (a - 80, 88, 1), (a + 8, 16, 1),
+                        (a - 8, 400, 1), (0, n, 0)):
+        assert rules.t_overlap(a, n, b, nb, *none) == want
+        assert rules.t_overlap(b, nb, *none, a, n) == want

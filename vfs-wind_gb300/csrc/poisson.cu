@@ -668,10 +668,11 @@ int device_view(vfs_poisson *h, const double *src, double *stage, size_t count, 
   *out = stage;
   return upload(h, stage, src, count);
 }
-// an array that is read and written: where it lies, or through *stage
-// (allocated on first use; the caller downloads it)
-int device_inout(vfs_poisson *h, double *a, double **stage, size_t count, double **out) {
-  if (in_place(h, a)) {
+// an array that is read and written: where it lies (unless `shared`: it overlaps
+// another one of the call), or through *stage (allocated on first use; the caller
+// downloads it)
+int device_inout(vfs_poisson *h, double *a, double **stage, size_t count, bool shared, double **out) {
+  if (!shared && in_place(h, a)) {
     *out = a;
     return VFS_OK;
   }
@@ -2827,7 +2828,7 @@ int vfs_poisson_contra2cart(vfs_poisson *h, const double *ucont, double *ucat, i
   const double *u = nullptr;
   double *v = nullptr;
   TRY(device_view(h, ucont, h->ucont, 3 * N, &u));
-  TRY(device_inout(h, ucat, &h->ucat, 3 * N, &v));
+  TRY(device_inout(h, ucat, &h->ucat, 3 * N, overlap({{ucont, 24 * N}, {ucat, 24 * N}}), &v));
   TRY(contra2cart(h, u, v, zero_solid));
   if (v != ucat) TRY(download(h, ucat, v, 3 * N));
   return sync(h);
@@ -2851,9 +2852,11 @@ int vfs_poisson_ibm_interpolate(vfs_poisson *h, int ibi, const double *u_surf, i
     h->ibm_work_len = need;
   }
   double *ud = nullptr, *pd = nullptr, *cd = nullptr, *us = nullptr;
-  TRY(device_inout(h, ucat, &h->ucat, 3 * N, &ud));
-  TRY(device_inout(h, p, &h->p_da, N, &pd));
-  TRY(device_inout(h, ucont, &h->ucont, 3 * N, &cd));
+  const bool shared =
+      overlap({{ucat, 24 * N}, {p, 8 * N}, {ucont, 24 * N}, {u_surf, (size_t)B.n_v * 24}});
+  TRY(device_inout(h, ucat, &h->ucat, 3 * N, shared, &ud));
+  TRY(device_inout(h, p, &h->p_da, N, shared, &pd));
+  TRY(device_inout(h, ucont, &h->ucont, 3 * N, shared, &cd));
   if (u_surf) {
     if (is_device_ptr(u_surf)) {
       us = const_cast<double *>(u_surf);
@@ -2887,8 +2890,9 @@ int vfs_poisson_ib_bc(vfs_poisson *h, int immersed, const int *bctype, double *u
   const Grid &g = h->g;
   const size_t N = g.n();
   double *ud = nullptr, *cd = nullptr;
-  TRY(device_inout(h, ucat, &h->ucat, 3 * N, &ud));
-  TRY(device_inout(h, ucont, &h->ucont, 3 * N, &cd));
+  const bool shared = overlap({{ucat, 24 * N}, {ucont, 24 * N}});
+  TRY(device_inout(h, ucat, &h->ucat, 3 * N, shared, &ud));
+  TRY(device_inout(h, ucont, &h->ucont, 3 * N, shared, &cd));
   int b[6] = {0, 0, 0, 0, 0, 0};
   if (bctype)
     for (int q = 0; q < 6; q++) b[q] = bctype[q];
@@ -3449,7 +3453,8 @@ int vfs_poisson_update_pressure(vfs_poisson *h, double *p, double *phi) {
   const size_t N = h->g.n();
   // device arrays are updated where they lie; the handle's phi (which
   // Projection reads) receives its copy in the same pass
-  const bool pdev = in_place(h, p), fdev = phi && in_place(h, phi);
+  const bool shared = overlap({{p, 8 * N}, {phi, 8 * N}});
+  const bool pdev = !shared && in_place(h, p), fdev = phi && !shared && in_place(h, phi);
   double *pd = pdev ? p : h->p_da;
   if (!pdev) TRY(upload(h, pd, p, N));
   if (phi && !fdev) TRY(upload(h, h->phi_da, phi, N));
