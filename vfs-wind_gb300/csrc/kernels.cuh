@@ -58,6 +58,8 @@ __global__ void k_periodic_cmpnts(Grid g, double *u);
 __global__ void k_contra2cart_coef(Grid g, Box b, MetricPtrs m, double *cc);
 __global__ void k_contra2cart(Grid g, Box b, const double *nvert, const uint8_t *near, const double *cc,
                               const double *u, double *ucat, int zero);
+__global__ void k_contra2cart_metrics(Grid g, Box b, const double *nvert, const uint8_t *near, MetricPtrs m,
+                                      const double *u, double *ucat, int zero);
 __global__ void k_zero_rim(Grid g, const double *nvert, double *ucat);
 __global__ void k_cellfield_restrict(Grid gh, Grid gc, int cx, int cy, int cz, const double *fh, double *fc);
 __global__ void k_assemble(Grid g, Box b, const double *nvert, MetricPtrs m, int scale, int filter, int split, double *A,

@@ -493,9 +493,10 @@ struct vfs_poisson {
   float *prev32 = nullptr;
   double *ucat = nullptr;  // Contra2Cart output staging (3 per DA point, host arrays only)
   // what Contra2Cart takes from the grid (k_contra2cart_coef: 12 planes over
-  // the box), formed by its first call after the grid was set
+  // the box), formed by its first call after the grid was set where they fit
+  // (VFS_CONTRA2CART_PLANES=0 at create: never)
   double *c2c = nullptr;
-  bool c2c_valid = false;
+  bool c2c_valid = false, c2c_off = false;
   // level-set variant of the operator and projection (vfs_poisson_set_levelset)
   double *ls_rho = nullptr, *ls_level = nullptr;
   int ls_on = 0, ls_bc3 = 0, ls_bc4 = 0, ls_bc5 = 0;
@@ -798,12 +799,14 @@ int face_coef(vfs_poisson *h, const Grid &g, MetricPtrs &m) {
 int contra2cart(vfs_poisson *h, const double *u, double *v, int zero_solid) {
   const Grid &g = h->g;
   const size_t n = h->box.n();
-  if (!h->c2c_valid) {
-    if (!h->c2c) TRY(dalloc(h, &h->c2c, 12 * n));
-    LAUNCH(h, k_contra2cart_coef, lin_grid(n), 256, g, h->box, h->met, h->c2c);
+  if (!h->c2c && !h->c2c_off && dalloc(h, &h->c2c, 12 * n) != VFS_OK) h->c2c_off = true;
+  if (h->c2c_off) {
+    LAUNCH(h, k_contra2cart_metrics, lin_grid(n), 256, g, h->box, h->nvert, h->near, h->met, u, v, zero_solid);
+  } else {
+    if (!h->c2c_valid) LAUNCH(h, k_contra2cart_coef, lin_grid(n), 256, g, h->box, h->met, h->c2c);
     h->c2c_valid = true;
+    LAUNCH(h, k_contra2cart, lin_grid(n), 256, g, h->box, h->nvert, h->near, h->c2c, u, v, zero_solid);
   }
-  LAUNCH(h, k_contra2cart, lin_grid(n), 256, g, h->box, h->nvert, h->near, h->c2c, u, v, zero_solid);
   if (const unsigned nb = shell_grid(g)) LAUNCH(h, k_periodic_cmpnts, nb, 256, g, v);
   if (zero_solid)
     LAUNCH(h, k_zero_rim, lin_grid(4 * ((size_t)g.my * g.mz + (size_t)g.mx * g.mz + (size_t)g.mx * g.my)), 256, g,
@@ -2536,6 +2539,8 @@ int vfs_poisson_create(const vfs_grid_desc *gd, vfs_poisson **out) {
     h->pdl = !(pd && pd[0] == '0');
     const char *inc = getenv("VFS_INCREMENTAL");
     h->inc_enable = !(inc && inc[0] == '0');
+    const char *cp = getenv("VFS_CONTRA2CART_PLANES");
+    h->c2c_off = cp && cp[0] == '0';
   }
   tail_limits(h);
   const size_t N = h->g.n(), n = h->box.n();

@@ -1910,27 +1910,34 @@ __global__ void k_periodic_cmpnts(Grid g, double *u) {
 
 // What Contra2Cart takes from the grid alone: the nine minors of the cell
 // metrics, their determinant, its reciprocal (0 where a quotient by it may leave
-// the normal range) and the reciprocal's rest, 12 planes over the box, formed
-// once per grid.
+// the normal range) and the reciprocal's rest.
+struct CellBasis {
+  double q[9], det, y, yl;
+  __device__ __forceinline__ void form(const MetricPtrs &m, size_t t) {
+    const double *c0 = &m.csi[t * 3], *e0 = &m.eta[t * 3], *z0 = &m.zet[t * 3];
+    const double m00 = c0[0], m01 = c0[1], m02 = c0[2], m10 = e0[0], m11 = e0[1], m12 = e0[2], m20 = z0[0],
+                 m21 = z0[1], m22 = z0[2];
+    q[0] = m11 * m22 - m12 * m21; q[1] = m01 * m22 - m02 * m21; q[2] = m01 * m12 - m02 * m11;
+    q[3] = m10 * m22 - m12 * m20; q[4] = m00 * m22 - m02 * m20; q[5] = m00 * m12 - m02 * m10;
+    q[6] = m10 * m21 - m11 * m20; q[7] = m00 * m21 - m01 * m20; q[8] = m00 * m11 - m01 * m10;
+    det = m00 * q[0] - m01 * q[3] + m02 * q[6];
+    const int ex = (__double2hiint(det) >> 20) & 0x7ff;
+    y = ex > 700 && ex < 1300 ? 1.0 / det : 0.0;
+    yl = fma(-det, y, 1.0) * y;
+  }
+};
+// The 12 planes of them over the box, formed once per grid (where they fit).
 __global__ void __launch_bounds__(256) k_contra2cart_coef(Grid g, Box b, MetricPtrs m, double *__restrict__ cc) {
   const size_t n = b.n(), c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   int i, j, k;
   box_ijk(b, c, i, j, k);
-  const size_t t = g.at(i + 1, j + 1, k + 1);
-  const double *c0 = &m.csi[t * 3], *e0 = &m.eta[t * 3], *z0 = &m.zet[t * 3];
-  const double m00 = c0[0], m01 = c0[1], m02 = c0[2], m10 = e0[0], m11 = e0[1], m12 = e0[2], m20 = z0[0],
-               m21 = z0[1], m22 = z0[2];
-  const double q[9] = {m11 * m22 - m12 * m21, m01 * m22 - m02 * m21, m01 * m12 - m02 * m11,
-                       m10 * m22 - m12 * m20, m00 * m22 - m02 * m20, m00 * m12 - m02 * m10,
-                       m10 * m21 - m11 * m20, m00 * m21 - m01 * m20, m00 * m11 - m01 * m10};
-  const double det = m00 * q[0] - m01 * q[3] + m02 * q[6];
-  for (int p = 0; p < 9; p++) cc[p * n + c] = q[p];
-  cc[9 * n + c] = det;
-  const int ex = (__double2hiint(det) >> 20) & 0x7ff;
-  const double y = ex > 700 && ex < 1300 ? 1.0 / det : 0.0;
-  cc[10 * n + c] = y;
-  cc[11 * n + c] = fma(-det, y, 1.0) * y;
+  CellBasis B;
+  B.form(m, g.at(i + 1, j + 1, k + 1));
+  for (int p = 0; p < 9; p++) cc[p * n + c] = B.q[p];
+  cc[9 * n + c] = B.det;
+  cc[10 * n + c] = B.y;
+  cc[11 * n + c] = B.yl;
 }
 
 // a / d from y = RN(1 / d) and its rest yl: Markstein's quotient where a lies well inside the
@@ -1958,11 +1965,13 @@ __device__ __forceinline__ bool solid(double nv) {
 // also clears solid cells, except on the two outermost layers (k_zero_rim
 // follows once the periodic ghosts have been copied).
 // 192x128x192: 0.72 -> 0.315 ms (77 % of the FP64 pipe; 0.34 ms with Markstein's
-// second correction in place of the reciprocal's rest).
-__global__ void __launch_bounds__(256) k_contra2cart(Grid g, Box b, const double *__restrict__ nvert,
-                                                     const uint8_t *__restrict__ near, const double *__restrict__ cc,
-                                                     const double *__restrict__ u, double *__restrict__ ucat,
-                                                     int zero) {
+// second correction in place of the reciprocal's rest).  Without the planes
+// (PLANES false) a cell forms them from its metrics, the same bits: 0.66 ms.
+template <bool PLANES>
+__device__ __forceinline__ void contra2cart_body(const Grid &g, const Box &b, const double *__restrict__ nvert,
+                                                 const uint8_t *__restrict__ near, const double *__restrict__ cc,
+                                                 const MetricPtrs &m, const double *__restrict__ u,
+                                                 double *__restrict__ ucat, int zero) {
   const size_t n = b.n(), c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   int i, j, k;
@@ -1982,15 +1991,30 @@ __global__ void __launch_bounds__(256) k_contra2cart(Grid g, Box b, const double
                tz = k == 0 && g.pz ? t + (size_t)(b.nz - 1) * g.mx * g.my : t - (size_t)g.mx * g.my;
   const double q0 = scale_down(u[tx * 3] + u[t * 3], 1), q1 = scale_down(u[ty * 3 + 1] + u[t * 3 + 1], 1),
                q2 = scale_down(u[tz * 3 + 2] + u[t * 3 + 2], 1);
-#define CC(p) __ldcs(&cc[(p) * n + c])
-  const double det = CC(9), y = CC(10), yl = CC(11);
-  const double d0 = q0 * CC(0) - q1 * CC(1) + q2 * CC(2);
-  const double d1 = -q0 * CC(3) + q1 * CC(4) - q2 * CC(5);
-  const double d2 = q0 * CC(6) - q1 * CC(7) + q2 * CC(8);
-#undef CC
-  ucat[t * 3 + 0] = quotient(d0, det, y, yl);
-  ucat[t * 3 + 1] = quotient(d1, det, y, yl);
-  ucat[t * 3 + 2] = quotient(d2, det, y, yl);
+  CellBasis B;
+  if (PLANES) {
+    B.det = __ldcs(&cc[9 * n + c]);
+    B.y = __ldcs(&cc[10 * n + c]);
+    B.yl = __ldcs(&cc[11 * n + c]);
+#pragma unroll
+    for (int p = 0; p < 9; p++) B.q[p] = __ldcs(&cc[p * n + c]);
+  } else {
+    B.form(m, t);
+  }
+  const double d0 = q0 * B.q[0] - q1 * B.q[1] + q2 * B.q[2];
+  const double d1 = -q0 * B.q[3] + q1 * B.q[4] - q2 * B.q[5];
+  const double d2 = q0 * B.q[6] - q1 * B.q[7] + q2 * B.q[8];
+  ucat[t * 3 + 0] = quotient(d0, B.det, B.y, B.yl);
+  ucat[t * 3 + 1] = quotient(d1, B.det, B.y, B.yl);
+  ucat[t * 3 + 2] = quotient(d2, B.det, B.y, B.yl);
+}
+__global__ void __launch_bounds__(256) k_contra2cart(Grid g, Box b, const double *nvert, const uint8_t *near,
+                                                     const double *cc, const double *u, double *ucat, int zero) {
+  contra2cart_body<true>(g, b, nvert, near, cc, MetricPtrs{}, u, ucat, zero);
+}
+__global__ void __launch_bounds__(256) k_contra2cart_metrics(Grid g, Box b, const double *nvert, const uint8_t *near,
+                                                             MetricPtrs m, const double *u, double *ucat, int zero) {
+  contra2cart_body<false>(g, b, nvert, near, nullptr, m, u, ucat, zero);
 }
 // the solid points among the two outermost layers of every side
 __global__ void k_zero_rim(Grid g, const double *__restrict__ nvert, double *ucat) {
