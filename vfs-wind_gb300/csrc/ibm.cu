@@ -61,7 +61,7 @@ unsigned glibc_rand_first(unsigned seed) {
 struct HashBox {
   double xmin, ymin, zmin, xmax, ymax, zmax, dcx, dcy, dcz;
   // for the FP32 tests: the hash cells' sizes and reciprocals, the rays' end
-  // height over zmin and the sum of the box's extents
+  // height over zmin and the sum of the box's extents (infinite: no test drops)
   float fcx, fcy, fcz, rcx, rcy, rcz, fz, L;
 };
 
@@ -83,11 +83,19 @@ __device__ __forceinline__ int hash_cell(double t, double d, float r) {
 // Nearly all triangles of a column are missed by far, and an FP64 test of
 // some 45 instructions holds a quarter of the SM for 64 cycles each: a test in
 // FP32 on coordinates relative to the box drops the triangles that the FP64
-// test is certain to drop.  With unit roundoff u = 2^-24, coordinates of at
-// most L and one-norms D, E1, E2 and T of the ray, the edges and the vertex
-// offset, inputs are off by at most 3 u L, and the triple products by at most
-// 24 u times the product of their norms (with L added to T): the margins are
-// 64 u.  A triangle whose det might be 0 within its margin is kept.  tf: v0,
+// test is certain to drop.  With u = 2^-24, L the sum of the box's extents and
+// one-norms D, E1, E2 of the ray and the edges: FP32 has the ray d' = d + x with
+// |x| <= 4 u L (L may be far more than D near a body's top) and t = p - v0 to
+// 2 u L.  For a triangle that the ray meets, t = a e1 + w e2 - s d with a, w >= 0,
+// a + w <= 1 and 0 < s <= 1 (the ray ends above the body), so that
+//   t.(d' x e2) = a det' - s d'.(x x e2)     t.(d' x e2) and d'.(t x e1) within
+//   d'.(t x e1) = w det' + s d'.(x x e1)     4 u L D E2 and 4 u L D E1 of a, w
+//   e2.(t x e1) = s det                      times det', whatever its sign is
+// and where det' has not the sign of det, |det| <= |x.(e2 x e1)| <= 4 u L E1 E2.  With
+// the error of t and the roundings (24 u times the norms) that stays below the
+// margins, 64 u times the norms with L added to that of t.  A triangle whose det'
+// is 0 within its margin is kept, and every one where the box is so large
+// (L > 10^12) that FP32 products might overflow: L is infinite then.  tf: v0,
 // e1, e2, |e1|, |e2| per triangle.  A tower over 840 k cells: 674 -> 380 us, a
 // rod over 48 k cells: 75 -> 58 us; with eight triangles' tests at a time, whose
 // loads fly together, 210 and 30 us (one at a time is a chain of two loads each;
@@ -764,7 +772,8 @@ int ibm_search_impl(vfs_poisson *h, int ibi, int n_v, const double *xyz, int n_e
   H.fcx = (float)H.dcx; H.fcy = (float)H.dcy; H.fcz = (float)H.dcz;
   H.rcx = (float)(1. / H.dcx); H.rcy = (float)(1. / H.dcy); H.rcz = (float)(1. / H.dcz);
   H.fz = (float)(H.zmax + 0.2 - H.zmin);
-  H.L = (float)((H.xmax - H.xmin) + (H.ymax - H.ymin) + (H.zmax + 0.2 - H.zmin));
+  const double extents = (H.xmax - H.xmin) + (H.ymax - H.ymin) + (H.zmax + 0.2 - H.zmin);
+  H.L = extents <= 1e12 ? (float)extents : INFINITY;
   // everything the kernels read of the body in one buffer and one copy:
   // column starts, column entries (triangle and its top hash cell, sorted by
   // the latter, descending), vertices, normals, ray offsets, FP32 triangles
