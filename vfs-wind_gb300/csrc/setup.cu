@@ -860,7 +860,8 @@ __global__ void k_reduce_rows(const double *partial, int nb, int nrow, double *o
 //                       (three operations in all; 2^-54 holds for 1.5 and 3);
 //   RN(a y + RN(a yl))  with yl = RN(delta y), the reciprocal's rest (1 / d to
 //                       about 2^-105): the quotient to just over half an ulp (four).
-// The remainder must not leave the normal range; the callers see to it.
+// The remainder must not leave the normal range: the callers look at the numerator's
+// exponent (k_rhs_nullspace at that of its factors, once for all cells).
 __device__ __forceinline__ double markstein3(double a, double d, double y) {
   const double q = a * y;
   return fma(fma(-q, d, a), y, q);
@@ -871,16 +872,21 @@ __device__ __forceinline__ double markstein4(double a, double d, double y, doubl
 }
 
 // 256x192x256: 0.135 ms (0.196 with five operations and loads behind the byte's;
-// the five operations left are 0.11 ms of the FP64 pipe).
+// the five operations left are 0.11 ms of the FP64 pipe).  Sums within 2^+-300
+// keep numerator, quotient and remainder in the normal range for every aj down to
+// 2^-400 (below, a quotient may be off in its last bit); other ones, infinities
+// and NaN take the division.  A zero sum leaves rhs as it is (its quotients are -0).
 __global__ void __launch_bounds__(256, 8) k_rhs_nullspace(Box b, const uint8_t *__restrict__ fluid,
                                                           const double *__restrict__ aj_box, const double *sums,
                                                           const double *fsum, double *__restrict__ rhs) {
   pdl_trigger();
   pdl_wait();
   const double sum = sums[0], sum_aj = fsum[0], y = 1.0 / sum_aj, delta = fma(-sum_aj, y, 1.0), yl = delta * y;
-  const bool fast = isfinite(y), three = fabs(delta) <= 0x1p-54;
-  const size_t n = b.n();
+  const int es = (__double2hiint(sum) >> 20) & 0x7ff, ea = (__double2hiint(sum_aj) >> 20) & 0x7ff;
+  const bool in = ea > 723 && ea < 1323, fast = in && es > 723 && es < 1323, three = fabs(delta) <= 0x1p-54;
+  const size_t n = in && sum == 0. ? 0 : b.n();
   auto shift = [&](auto quotient_of) {
+#pragma unroll 4
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
       const bool f = fluid[c];
       const double aj = aj_box[c], r = rhs[c];
