@@ -16,6 +16,7 @@ int t_in_place(int type, int memory_device, int device, uintptr_t address) {
 int t_overlap(size_t a, size_t na, size_t b, size_t nb, size_t c, size_t nc) {
   return vfs::overlap({{(void *)a, na}, {(void *)b, nb}, {(void *)c, nc}});
 }
+int t_line_columns(int P, int fp64, int cap, int max_threads) { return vfs::line_columns(P, fp64, cap, max_threads); }
 }
 """
 HOST, DEVICE, MANAGED = 0, 1, 2
@@ -70,3 +71,24 @@ def test_overlapping_arrays(rules):
                         (a - 8, 400, 1), (0, n, 0)):
         assert rules.t_overlap(a, n, b, nb, *none) == want
         assert rules.t_overlap(b, nb, *none, a, n) == want
+
+
+def test_line_columns(rules):
+    """FP64 blocks stay within the limit without giving up the lanes that four columns
+    use; FP32 halves sixteen; a cap holds."""
+    limit = 384
+
+    def used(P, c):
+        return P * c / ((P * c + 31) // 32 * 32)
+
+    for P in range(1, limit + 1):
+        c = rules.t_line_columns(P, 1, 0, limit)
+        four = next(t for t in (4, 2, 1) if t * P <= limit or t == 1)
+        assert 1 <= c <= 8 and c * P <= limit
+        assert used(P, c) >= used(P, four) and c >= four
+        assert rules.t_line_columns(P, 0, 0, limit) == next(t for t in (16, 8, 4, 2, 1) if t * P <= limit or t == 1)
+        for cap in (1, 2, 3, 4, 6):
+            assert rules.t_line_columns(P, 1, cap, limit) <= cap
+            assert rules.t_line_columns(P, 0, cap, limit) <= cap
+    assert rules.t_line_columns(5, 1, 0, limit) == 6
+    assert rules.t_line_columns(77, 1, 0, limit) == 4

@@ -1358,24 +1358,10 @@ void prof_end(vfs_poisson *h, int li) {
 
 // Columns per block of the line kernels for lines of P chunks.  The
 // kernels are compiled for at most kLineMaxThreads threads per block (a
-// whole chunk stays in registers): 16 columns in FP32 and 4 in FP64, where
-// more, smaller blocks per SM measured faster (warm FP64 solve 31.5 -> 30.3
-// ms on the 256x192x256 towers grid; FP32 unchanged), halved while the block
-// would exceed the limit (8 columns for j-lines of 193..384 cells in FP32).
-// Every column is solved independently, so the width changes no result bit.
-// VFS_LINE_COLUMNS caps the width (read at create).
+// whole chunk stays in registers).  Every column is solved independently, so
+// the width changes no result bit.  VFS_LINE_COLUMNS caps it (read at create).
 int line_columns(const vfs_poisson *h, int P, bool fp64) {
-  int ti = fp64 ? 4 : 16;
-  if (fp64) {
-    // four to eight columns, whichever leave the fewest idle lanes: four columns of
-    // five chunks fill 20 of a warp's 32, six fill 30 (72x40x56 solve 5446 -> 5395 us)
-    auto idle = [&](int c) { return (double)((c * P + 31) / 32 * 32) / (c * P); };
-    for (int c = 5; c <= 8; c++)
-      if (idle(c) < idle(ti)) ti = c;
-  }
-  if (h->line_cols_cap > 0 && ti > h->line_cols_cap) ti = h->line_cols_cap;
-  while (ti > 1 && ti * P > kLineMaxThreads) ti >>= 1;
-  return ti;
+  return vfs::line_columns(P, fp64, h->line_cols_cap, kLineMaxThreads);
 }
 
 // One smoothing sweep on level l.  smoother 0: fused j-line Jacobi kernel;

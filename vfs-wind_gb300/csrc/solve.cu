@@ -1402,7 +1402,7 @@ void launch_hist_push(cudaStream_t st, int blocks, size_t n, const double *x, co
   }                                                                                                        \
   __global__ void k_cast_planes_##S(const double *src, T *dst, size_t n) { cast_body<T>(src, dst, n); }
 // the line kernel keeps a whole chunk in registers: at most 384 threads per
-// block (16 columns of up to 24 chunks in FP32, 4 columns in FP64) so that
+// block (16 columns of up to 24 chunks in FP32, 4 to 8 columns in FP64) so that
 // neither precision spills
 TYPED(float, f32, kLineMaxThreads, 1)
 TYPED(double, f64, kLineMaxThreads, 1)
