@@ -15,7 +15,7 @@ from test_gpu_unet import _data, _net, _rel
 
 pytestmark = pytest.mark.gpu
 
-GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "unet_wgrad_64.npz")
+GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "unet", "wgrad_64.npz")
 # The recorded gradient's 33 chains were added by atomics, in any order: 33 additions
 # of relative error 2^-24 each, at random sqrt(33) 2^-24 = 3.4e-7; two such orders
 # differ by at most twice that.  Chains over other tiles are 5.7e-6 off.
