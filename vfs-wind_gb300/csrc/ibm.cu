@@ -1059,8 +1059,9 @@ extern "C" int vfs_poisson_ibm_nodes(vfs_poisson *h, int ibi, vfs_ibm_node *node
 namespace vfs {
 
 // noslip velocity and interpolated pressure at every IB node of one body
-// (ibm.c:3405-3560, wallfunction.c:140-156); lucat / lp are the inputs as
-// read (the reference's local copies), ucat / p are written at the nodes.
+// (ibm.c:3405-3560, wallfunction.c:140-156), formed from lucat / lp, the arrays as
+// they are (the reference's local copies), into val, four values a node: ucat and
+// p are those arrays, and k_ibm_scatter writes them once every node has been read.
 __global__ void k_ibm_gather(Grid g, const vfs_ibm_node *nodes, int n_nodes, const int *tri, const double *u_surf,
                              const double *nvert, const double *lucat, const double *lp, double *val) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;

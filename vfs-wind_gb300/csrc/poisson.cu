@@ -740,13 +740,14 @@ dim3 guess_grid(const Box &b) { return dim3((b.nx + 127) / 128, (b.ny + kGuessRo
     (h)->launches++;                                               \
   } while (0)
 
-// A kernel of the V-cycle.  When the previous operation on the stream was
-// one too, the launch carries programmatic stream serialization: its blocks
-// may start as the previous kernel's last blocks run, load the level's
-// operator planes and wait (griddepcontrol.wait) for that kernel's results.
-// Only kernels that wait before reading anything the V-cycle writes go
-// through here.  A memset or an event in between (vmemset, the profiling
-// events) makes the next launch an ordinary one.
+// A kernel of a chain (the V-cycle, the Krylov step, the stages around the solve).
+// When the previous operation on the stream was one too, the launch carries
+// programmatic stream serialization: its blocks may start as the previous kernel's
+// last blocks run, load what no kernel of the chain writes and wait
+// (griddepcontrol.wait) for that kernel's results.  Only kernels that wait before
+// they read or write anything the chain writes go through here.  A memset or an
+// event in between (vmemset, the profiling events) makes the next launch an
+// ordinary one, and so does chain_start.
 template <typename... P, typename... A>
 void launch_v(vfs_poisson *h, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
   cudaLaunchAttribute at[1];
@@ -1467,6 +1468,11 @@ void tail_limits(vfs_poisson *h) {
 // kTailDofs rows is better spread over the whole chip.  Solves without and
 // with the tail: 24x16x24 1250 and 925 us, 64^3 1882 and 1629, 128x96x128
 // 5525 and 5230, FP64 72x40x56 6620 and 5795.
+// In FP64 a phase is bound by the pipes of the cluster's 16 SMs and the line is
+// flat: solves with at most 16, 12 and 9 warps a CTA, 60x16x16 (15 warps) 2244,
+// 2196 and 2199 us, 28x32x16 (14) 1384, 1366 and 1370, 24x16x24 (12) 1424, 1426
+// and 1375, 40x24x32 (10) 1666, 1666 and 1733; without a tail 3272, 1907, 2108 and
+// 2217.
 template <typename T>
 bool tail_plan(vfs_poisson *h, int li, int nu1, int smoother, TailArgs *a, size_t *smem) {
   constexpr int p = std::is_same<T, double>::value;

@@ -1084,7 +1084,7 @@ __global__ void __launch_bounds__(256) k_box_to_da(Grid g, Box b, const double *
 }
 
 // Periodic ghost points, one thread per point of the two boundary layers of
-// each periodic axis (grid from shell_points on the host: no pass over the
+// each periodic axis (grid from shell_grid on the host: no pass over the
 // whole array).  A point on the layers of two axes is visited twice with the
 // same source, whose periodic coordinates all lie inside, so it is never a
 // target.
