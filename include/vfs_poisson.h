@@ -8,12 +8,12 @@
  * rank: scalars double[mz][my][mx] (i fastest), Cmpnts vectors
  * double[mz][my][mx][3], with index 0 and m-1 the boundary layer
  * (Source/init.c:157-161).  Every array pointer may be host memory or device
- * memory of the handle's GPU; the library detects which.  Per-step calls work on
- * device arrays where they lie; host arrays, another GPU's, arrays off the element
- * grid and arrays of one call that overlap are copied through the handle's stream
- * (slower, the same results; results are then written in the order of the
- * arguments).  Calls are synchronous on return and a handle is not thread-safe.  The handle's private stream is a blocking
- * stream, so device inputs written on the legacy default stream are ready
+ * memory of the handle's GPU; the library detects which.  Most per-step calls work
+ * on device arrays where they lie; host arrays, another GPU's, arrays off the
+ * element grid and arrays of one call that overlap are copied through the handle's
+ * stream (slower, the same results; results are then written in the order of the
+ * arguments).  Calls are synchronous on return and a handle is not thread-safe.
+ * The handle's private stream is a blocking stream, so device inputs written on the legacy default stream are ready
  * when a call starts; inputs written on another stream must be complete (or
  * that stream passed to vfs_poisson_set_stream).
  *

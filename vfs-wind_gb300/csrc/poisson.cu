@@ -1468,11 +1468,11 @@ void tail_limits(vfs_poisson *h) {
 // kTailDofs rows is better spread over the whole chip.  Solves without and
 // with the tail: 24x16x24 1250 and 925 us, 64^3 1882 and 1629, 128x96x128
 // 5525 and 5230, FP64 72x40x56 6620 and 5795.
-// In FP64 a phase is bound by the pipes of the cluster's 16 SMs and the line is
-// flat: solves with at most 16, 12 and 9 warps a CTA, 60x16x16 (15 warps) 2244,
-// 2196 and 2199 us, 28x32x16 (14) 1384, 1366 and 1370, 24x16x24 (12) 1424, 1426
-// and 1375, 40x24x32 (10) 1666, 1666 and 1733; without a tail 3272, 1907, 2108 and
-// 2217.
+// In FP64 a phase is bound by the pipes of the cluster's 16 SMs, and where the line
+// lies matters little: solves with at most 16, 12 and 9 warps a CTA and without a
+// tail, 60x16x16 (15 warps) 2240, 2186, 2185 and 2838 us, 28x32x16 (14) 1385, 1371,
+// 1371 and 1523, 24x16x24 (12) 1428, 1428, 1379 and 1809, 40x24x32 (10) 1665, 1668,
+// 1688 and 1887.
 template <typename T>
 bool tail_plan(vfs_poisson *h, int li, int nu1, int smoother, TailArgs *a, size_t *smem) {
   constexpr int p = std::is_same<T, double>::value;
